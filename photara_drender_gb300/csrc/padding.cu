@@ -8,13 +8,16 @@
 //
 // * a texel's forward-sweep value depends only on the forward values of (x-1,y), (x,y-1), (x-1,y-1) and
 //   (x+1,y-1); the reverse sweep mirrors this. A warp therefore sweeps 32 rows at once on a skewed
-//   wavefront: lane r handles row 32*band + r and reaches column i at step i + 2r, so the three upper
+//   wavefront: lane r handles row r of its rows and reaches column i at step i + 2r, so the three upper
 //   neighbours are the values lane r-1 produced one, two and three steps earlier (one shuffle a step)
 //   and the left neighbour is the lane's own previous value. Each relaxation then runs in the
 //   reference's order with its strict comparison and clamp, so every texel takes the same value.
-// * bands are warps ordered by a ticket; a band's first row reads the row above from the previous
-//   band's boundary buffer. Entries start as a marker that no offset can equal (|offset| <= 16384), so
-//   a value is ready exactly when it differs from the marker: no fences. Every wait is bounded.
+// * atlases up to 4384 texels a side: 64 x 32 tiles, swept in parallel and repeated until every tile was
+//   swept with the values its neighbours end with (pad_tiles_kernel).
+// * larger atlases (pad_sweep_kernel): bands are warps ordered by a ticket; a band's first row reads the row
+//   above from the previous band's boundary buffer. Entries start as a marker that no offset can equal
+//   (|offset| <= 16384), so a value is ready exactly when it differs from the marker: no fences. Every wait
+//   is bounded.
 // * the fill is per texel. A source texel is never written, so copies from it are race-free; the only
 //   other case (an offset inherited from a texel with no source that lands inside the atlas, possible
 //   only when both sides exceed 12000) is resolved in the reference's raster order from a snapshot.
@@ -160,14 +163,10 @@ __device__ __forceinline__ uint32_t final_index(uint32_t x, uint32_t y, uint32_t
 
 // One 8SSEDT sweep (texture_padding.cpp:80-94): the forward sweep writes `out` from the source bits, the
 // reverse sweep (kBack) reads the forward field `in` and writes the final field `out`. control: [0]
-// forward ticket, [1] reverse ticket, [2] failure flag.
-//
-// kExact keeps the reference's relaxations one by one, with their clamp of offsets to +-16384. Without
-// it (atlas sides <= 4384) no offset component can exceed +-16383 (a real source is closer than the atlas
-// side, an offset inherited from a texel without source is at most 12000 + side - 1), so no candidate is
-// ever clamped, and the sequential relaxations equal "the first of [own, left, up, up-left, up-right] with
-// the smallest squared length": everything but the left neighbour is reduced off the step's critical path.
-template <bool kBack, bool kExact>
+// forward ticket, [1] reverse ticket, [2] failure flag. The relaxations run one by one, with the
+// reference's clamp of offsets to +-16384. For atlases above kTileMaxSide, and where the device cannot
+// hold pad_tiles_kernel's grid at once.
+template <bool kBack>
 __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restrict__ src_bits, uint32_t words_per_row,
                                                        const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                        uint32_t* __restrict__ boundary, uint32_t* control,
@@ -286,34 +285,13 @@ __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restric
             const int32_t rcx = rx, rcy = ry - dy;                     // up
             const int32_t pcx = prx - dx, pcy = pry - dy;              // up-left
             const int32_t ncx = nrx + dx, ncy = nry - dy;              // up-right
-            int32_t hx, hy;
-            if (kExact) {
-                hx = ix;
-                hy = iy;
-                int32_t hk = ix * ix + iy * iy;
-                if (left) relax(hx, hy, hk, lcx, lcy);
-                if (up) {
-                    relax(hx, hy, hk, rcx, rcy);
-                    if (left) relax(hx, hy, hk, pcx, pcy);
-                    if (right) relax(hx, hy, hk, ncx, ncy);
-                }
-            } else {
-                constexpr int32_t kInf = 0x7FFFFFFF;
-                const int32_t ki = ix * ix + iy * iy;
-                const int32_t kr = up ? rcx * rcx + rcy * rcy : kInf;
-                const int32_t kp = up && left ? pcx * pcx + pcy * pcy : kInf;
-                const int32_t kn = up && right ? ncx * ncx + ncy * ncy : kInf;
-                // first minimum of the up candidates, then of [own, that]: own wins ties
-                int32_t ax = rcx, ay = rcy, ka = kr;
-                if (kp < ka) { ax = pcx; ay = pcy; ka = kp; }
-                if (kn < ka) { ax = ncx; ay = ncy; ka = kn; }
-                const bool own = ki <= ka;
-                const int32_t bx = own ? ix : ax, by = own ? iy : ay;
-                // the left candidate comes after own (must be strictly shorter) and before the up ones
-                const int32_t thr = own ? ki : ka + 1;
-                const int32_t kl = left ? lcx * lcx + lcy * lcy : kInf;
-                hx = kl < thr ? lcx : bx;
-                hy = kl < thr ? lcy : by;
+            int32_t hx = ix, hy = iy;
+            int32_t hk = ix * ix + iy * iy;
+            if (left) relax(hx, hy, hk, lcx, lcy);
+            if (up) {
+                relax(hx, hy, hk, rcx, rcy);
+                if (left) relax(hx, hy, hk, pcx, pcy);
+                if (right) relax(hx, hy, hk, ncx, ncy);
             }
             mx = active ? hx : mx;
             my = active ? hy : my;
@@ -328,14 +306,303 @@ __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restric
     }
 }
 
+// ---- tiled sweeps ---------------------------------------------------------------------------------
+//
+// The sweeps of atlases up to kTileMaxSide on a side. Two facts make them parallel:
+//
+// 1. A field is the sweep's result exactly when every texel's value is the relaxation of its own start
+//    value by its four earlier neighbours' values (induction in raster order). So tiles may be swept in any
+//    order, with whatever their neighbours hold, and swept again, as long as in the end every texel
+//    satisfies its relaxation. Sweeping a tile satisfies all texels inside it; afterwards only the texels on
+//    its first row, first and last column look at other tiles, and a tile whose neighbours changed checks
+//    just those (tile_settled) before it is swept again. A nearest source is mostly close, so most tiles
+//    are final after one or two sweeps; the loop ends after a pass in which none changed. A value crosses at
+//    most two tile borders per row and one per 64 columns on its way, which bounds the passes.
+// 2. With sides <= 4384 a real offset (squared length <= 2 * 4384^2) is always shorter than one inherited from
+//    a texel without source (components >= 12000 - 4384), no candidate reaches the +-16384 clamp, and the
+//    sequential relaxations equal "the first of [own, left, up, up-left, up-right] with the smallest squared
+//    length". Offsets without a source are therefore all kept as kNoSource: which of them a texel holds is
+//    never looked at once the atlas has a source (and nothing is filled when it has none), and empty areas
+//    are settled at once. A neighbour outside the atlas acts as one without a source.
+//
+// The field holds source positions (x | y << 16) instead of offsets: a value then travels unchanged, and a
+// candidate's squared length is (sx - x)^2 + (sy - y)^2 with the second term fixed along a row.
+//
+// What bounds it: the latency of a tile's wavefront (64 + 3 * 31 steps of about 50 instructions, 10 us) times
+// the passes: a hole of 300 texels takes about 25 passes a sweep, gutters and small holes 5 to 8. One
+// warp-wide wavefront per 32 rows of the whole atlas, each band waiting for the one above, was a chain of
+// W + 2H dependent steps whatever the atlas held. Whole padding call, 4096 x 4096 with 300-texel holes:
+// 6.91 -> 1.93 ms; 1400 x 1000, 8-texel gutters: 1.91 -> 0.42 ms. Tiles of 64 columns: 32 would save a third
+// of a pass and need up to twice the passes. Above kTileMaxSide fact 2 does not hold: pad_sweep_kernel.
+constexpr int32_t kTileMaxSide = 4384;
+constexpr int kPadTileW = 64;
+constexpr int kPadPitch = kPadTileW + 1;  // (row r, column t - 2r): odd pitch - 2, no bank conflicts
+constexpr int kPadRows = 8;               // rows of a tile loaded together: 16 loads of a lane in flight
+constexpr int kPadWarps = 4;              // 34 KB of shared memory: six CTAs per SM
+constexpr uint32_t kPadMaxPasses = 1u << 16;
+constexpr uint32_t kNoSource = 0x75307530u;  // (30000, 30000): farther from any texel than a real source
+static_assert(kPadTileW == 64, "a lane moves two columns of a tile row");
+
+struct TileSweeps {
+    const uint32_t* src_bits;
+    uint32_t* forward;   // [H][W] source positions after the forward sweep
+    uint32_t* field;     // [H][W] after the reverse sweep
+    uint8_t* changed;    // [2][tiles]: tile changed in the pass before / in this pass
+    uint32_t* control;   // [2] failure flag, [8] barrier arrivals, [12..15] "a tile changed" per pass & 3
+    uint32_t* status;
+    uint32_t words_per_row;
+    int32_t W, H, tiles_x, tiles;
+};
+
+// All CTAs of the (cooperative) grid meet; false when the wait gave up or another CTA failed.
+__device__ bool pad_grid_barrier(uint32_t* control, uint32_t& phase) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(control + 8, 1u);
+        const uint32_t target = ++phase * gridDim.x;
+        const long long start = clock64();
+        int good = 1;
+        while (ld_relaxed(control + 8) < target) {
+            if (ld_relaxed(control + 2) != 0 || clock64() - start > kWaitCycles) {
+                atomicExch(control + 2, 1u);
+                good = 0;
+                break;
+            }
+        }
+        __threadfence();
+        ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// A source position as the texels of row y see it.
+struct Source {
+    uint32_t v;   // x | y << 16
+    int32_t sx, row;  // its column, its squared distance along y
+    __device__ __forceinline__ Source(uint32_t value, int32_t y) : v(value), sx((int32_t)(value & 0xFFFFu)) {
+        const int32_t d = (int32_t)(value >> 16) - y;
+        row = d * d;
+    }
+    __device__ __forceinline__ int32_t length(int32_t x) const { return (sx - x) * (sx - x) + row; }
+};
+
+// The relaxation of a texel, the first shortest of own, left, up, up-left and up-right, without the left
+// neighbour, the only one on the wavefront's critical path: `v` is the first shortest of the others, and the
+// left neighbour's value wins below the squared length `limit` (it comes after own, where strictly shorter
+// wins, and before the row above, where as short does).
+__device__ __forceinline__ void relaxed_upper(const Source& own, const Source& u, const Source& ul, const Source& ur,
+                                              int32_t x, uint32_t& v, int32_t& limit) {
+    const int32_t k0 = own.length(x), k1 = ul.length(x), k2 = ur.length(x);
+    int32_t k = u.length(x);
+    uint32_t a = u.v;
+    if (k1 < k) { a = ul.v; k = k1; }
+    if (k2 < k) { a = ur.v; k = k2; }
+    const bool mine = k0 <= k;  // own wins ties against the row above
+    v = mine ? own.v : a;
+    limit = mine ? k0 : k + 1;
+}
+
+// Texels in sweep order: (X, Y) counts from the corner the sweep starts at.
+template <bool kBack>
+struct SweepSpace {
+    const TileSweeps& s;
+    uint32_t* out;
+    __device__ __forceinline__ explicit SweepSpace(const TileSweeps& t) : s(t), out(kBack ? t.field : t.forward) {}
+    __device__ __forceinline__ int32_t x(int32_t X) const { return kBack ? s.W - 1 - X : X; }
+    __device__ __forceinline__ int32_t y(int32_t Y) const { return kBack ? s.H - 1 - Y : Y; }
+    __device__ __forceinline__ uint32_t at(int32_t X, int32_t Y) const { return (uint32_t)(y(Y) * s.W + x(X)); }
+    // another tile may be rewriting the value: read it from L2, old or new (see above)
+    __device__ __forceinline__ uint32_t value(int32_t X, int32_t Y) const {
+        return X < 0 || Y < 0 || X >= s.W || Y >= s.H ? kNoSource : __ldcg(out + at(X, Y));
+    }
+    __device__ __forceinline__ uint32_t start(int32_t X, int32_t Y) const {
+        if (kBack) return __ldcg(s.forward + at(X, Y));
+        const bool source = (s.src_bits[(uint32_t)Y * s.words_per_row + (X >> 5)] >> (X & 31)) & 1u;
+        return source ? (uint32_t)X | (uint32_t)Y << 16 : kNoSource;
+    }
+    __device__ __forceinline__ bool settled(int32_t X, int32_t Y) const {
+        const int32_t px = x(X), py = y(Y);
+        uint32_t v;
+        int32_t limit;
+        const Source left(value(X - 1, Y), py);
+        relaxed_upper(Source(start(X, Y), py), Source(value(X, Y - 1), py), Source(value(X - 1, Y - 1), py),
+                      Source(value(X + 1, Y - 1), py), px, v, limit);
+        return value(X, Y) == (left.length(px) < limit ? left.v : v);
+    }
+};
+
+// Whether the texels of a swept tile that look at other tiles still satisfy their relaxation.
+template <bool kBack>
+__device__ __forceinline__ bool tile_settled(const SweepSpace<kBack>& sp, int32_t X0, int32_t Y0, int32_t tw,
+                                             int32_t rows) {
+    // the first row (two texels a lane), the first and the last column: all loads in flight together
+    const int32_t lane = threadIdx.x & 31, r = min(lane, rows - 1);
+    const bool a = sp.settled(X0 + min(lane, tw - 1), Y0), b = sp.settled(X0 + min(lane + 32, tw - 1), Y0);
+    const bool c = sp.settled(X0, Y0 + r), e = sp.settled(X0 + tw - 1, Y0 + r);
+    return __all_sync(0xFFFFFFFFu, a & b & c & e);
+}
+
+// Sweeps one tile from its start values and what its neighbours hold; whether a value that other tiles look
+// at (its last row, first and last column) changed. Lane r reaches column i at step i + 3r: two steps would
+// do for the row above, the third lets a texel's upper candidates be reduced a step ahead of its turn.
+template <bool kBack>
+__device__ __forceinline__ bool sweep_tile(const SweepSpace<kBack>& sp, int32_t X0, int32_t Y0, int32_t tw,
+                                           int32_t rows, bool first, uint32_t* buf, uint32_t* top) {
+    const TileSweeps& s = sp.s;
+    const int32_t lane = threadIdx.x & 31, Y = Y0 + lane;
+    const bool row_ok = lane < rows, in0 = lane < tw, in1 = lane + 32 < tw;
+    uint32_t* line = buf + lane * kPadPitch;
+    __syncwarp();
+    // the row above (columns X0 - 1 .. X0 + tw), and this row's neighbours left and right of the tile
+    for (int32_t j = lane; j < tw + 2; j += 32) top[j] = first ? kNoSource : sp.value(X0 - 1 + j, Y0 - 1);
+    const uint32_t left = first || !row_ok ? kNoSource : sp.value(X0 - 1, Y);
+    const uint32_t right = first || !row_ok ? kNoSource : sp.value(X0 + tw, Y);
+    // what the tile held on its last row, first and last column
+    uint32_t old[4] = {kNoSource, kNoSource, kNoSource, kNoSource};
+    if (!first) {
+        old[0] = sp.value(X0 + lane, Y0 + rows - 1);
+        old[1] = sp.value(X0 + lane + 32, Y0 + rows - 1);
+        old[2] = sp.value(X0, Y);
+        old[3] = sp.value(X0 + tw - 1, Y);
+    }
+    uint32_t w0 = 0, w1 = 0;  // forward: this row's source bits
+    if (kBack) {
+        for (int32_t r0 = 0; r0 < rows; r0 += kPadRows) {
+            uint32_t v[kPadRows][2];
+#pragma unroll
+            for (int32_t k = 0; k < kPadRows; ++k) {
+                if (in0 && r0 + k < rows) v[k][0] = __ldcg(s.forward + sp.at(X0 + lane, Y0 + r0 + k));
+                if (in1 && r0 + k < rows) v[k][1] = __ldcg(s.forward + sp.at(X0 + lane + 32, Y0 + r0 + k));
+            }
+#pragma unroll
+            for (int32_t k = 0; k < kPadRows; ++k) {
+                if (in0 && r0 + k < rows) buf[(r0 + k) * kPadPitch + lane] = v[k][0];
+                if (in1 && r0 + k < rows) buf[(r0 + k) * kPadPitch + lane + 32] = v[k][1];
+            }
+        }
+    } else if (row_ok) {
+        const uint32_t* w = s.src_bits + (size_t)Y * s.words_per_row + (X0 >> 5);
+        w0 = w[0];
+        w1 = tw > 32 ? w[1] : 0u;
+    }
+    __syncwarp();
+    const int32_t py = sp.y(Y), px0 = sp.x(X0);
+    constexpr int32_t dx = kBack ? -1 : 1;
+    // this row's start value at column i, clamped to the tile (nobody uses one outside it)
+    auto own_at = [&](int32_t i) -> uint32_t {
+        const int32_t c = min(max(i, 0), tw - 1);
+        if (kBack) return line[c];
+        const bool source = ((c < 32 ? w0 : w1) >> (c & 31)) & 1u;
+        return source ? (uint32_t)(px0 + c) | (uint32_t)py << 16 : kNoSource;
+    };
+    // Step t: column i = t - 3 * lane takes its value from `upper` and the left neighbour (cur); then `upper` is
+    // made for column i + 1 from the row above at i, i + 1 and i + 2 (ul, u, ur after the shift), the last
+    // produced by lane - 1 in step t - 1. Columns -1 and tw of a lane hold its neighbours outside the tile. Start
+    // values and lane 0's row above are loaded a step ahead of their use.
+    Source cur(left, py), ul(kNoSource, py), u(lane == 0 ? top[0] : kNoSource, py), ur(lane == 0 ? top[1] : kNoSource, py);
+    uint32_t next_own = own_at(-3 * lane), next_top = top[min(2, tw + 1)];
+    uint32_t upper = kNoSource;
+    int32_t limit = 0;
+    const int32_t steps = tw + 3 * (rows - 1);
+    int32_t i = -1 - 3 * lane, x = px0 + dx * i;
+#pragma unroll 3
+    for (int32_t t = -1; t < steps; ++t) {
+        const uint32_t from_above = __shfl_up_sync(0xFFFFFFFFu, cur.v, 1);
+        const uint32_t from_top = next_top, own = next_own;
+        next_top = top[min(t + 4, tw + 1)];
+        uint32_t v = cur.length(x) < limit ? cur.v : upper;
+        v = i < tw ? v : right;
+        if (i >= 0) cur = Source(v, py);
+        if (row_ok && (uint32_t)i < (uint32_t)tw) line[i] = v;
+        ul = u;
+        u = ur;
+        ur = Source(lane == 0 ? from_top : from_above, py);
+        ++i;
+        x += dx;
+        next_own = own_at(i + 1);
+        relaxed_upper(Source(own, py), u, ul, ur, x, upper, limit);
+    }
+    __syncwarp();
+    bool changed = first;
+    if (!first) {
+        const uint32_t* last = buf + (rows - 1) * kPadPitch;
+        changed = (in0 && last[lane] != old[0]) || (in1 && last[lane + 32] != old[1]) ||
+                  (row_ok && (line[0] != old[2] || line[tw - 1] != old[3]));
+    }
+    for (int32_t r0 = 0; r0 < rows; r0 += kPadRows)
+#pragma unroll
+        for (int32_t k = 0; k < kPadRows; ++k) {
+            if (r0 + k >= rows) break;
+            uint32_t* o = sp.out + sp.at(X0 + lane, Y0 + r0 + k);
+            if (in0) __stcg(o, buf[(r0 + k) * kPadPitch + lane]);
+            if (in1) __stcg(kBack ? o - 32 : o + 32, buf[(r0 + k) * kPadPitch + lane + 32]);
+        }
+    return __any_sync(0xFFFFFFFFu, changed);
+}
+
+template <bool kBack>
+__device__ bool sweep_tiles(const TileSweeps& s, uint32_t& phase, uint32_t* buf, uint32_t* top) {
+    const SweepSpace<kBack> sp(s);
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t warp = blockIdx.x * kPadWarps + (threadIdx.x >> 5), warps = gridDim.x * kPadWarps;
+    const int32_t tiles_y = s.tiles / s.tiles_x;
+    for (uint32_t pass = 0; pass < kPadMaxPasses; ++pass) {
+        const uint8_t* before = s.changed + (size_t)((pass & 1u) ^ 1u) * s.tiles;
+        uint8_t* now = s.changed + (size_t)(pass & 1u) * s.tiles;
+        uint32_t* any = s.control + 12 + (pass & 3u);
+        // the slot of pass + 2 was last read two barriers ago
+        if (blockIdx.x == 0 && threadIdx.x == 0) s.control[12 + ((pass + 2u) & 3u)] = 0u;
+        for (int32_t tile = warp; tile < s.tiles; tile += warps) {
+            const int32_t ty = tile / s.tiles_x, tx = tile - ty * s.tiles_x;
+            const int32_t X0 = tx * kPadTileW, Y0 = ty * 32;
+            const int32_t tw = min(kPadTileW, s.W - X0), rows = min(32, s.H - Y0);
+            bool todo = pass == 0;
+            if (pass > 0) {  // a neighbour this tile looks at changed: left, right, and the three above
+                const int32_t nx = tx + (lane == 0 || lane == 2 ? -1 : lane == 3 ? 0 : 1), ny = ty - (lane >= 2 ? 1 : 0);
+                const bool dirty = lane < 5 && nx >= 0 && nx < s.tiles_x && ny >= 0 && ny < tiles_y &&
+                                   __ldcg(before + ny * s.tiles_x + nx) != 0;
+                todo = __any_sync(0xFFFFFFFFu, dirty) && !tile_settled(sp, X0, Y0, tw, rows);
+            }
+            const bool changed = todo && sweep_tile(sp, X0, Y0, tw, rows, pass == 0, buf, top);
+            if (lane == 0) {
+                __stcg(now + tile, (uint8_t)changed);
+                if (changed) atomicOr(any, 1u);
+            }
+        }
+        if (!pad_grid_barrier(s.control, phase)) return false;
+        if (ld_relaxed(any) == 0) return true;
+    }
+    return false;
+}
+
+__global__ void __launch_bounds__(32 * kPadWarps, 6) pad_tiles_kernel(TileSweeps s) {
+    __shared__ uint32_t buf[kPadWarps][32 * kPadPitch];
+    __shared__ uint32_t top[kPadWarps][kPadTileW + 2];
+    const int warp = threadIdx.x >> 5;
+    uint32_t phase = 0;
+    bool ok = sweep_tiles<false>(s, phase, buf[warp], top[warp]);
+    // the reverse sweep starts its passes at slot 0: clear the slots behind a barrier of their own
+    if (ok && blockIdx.x == 0 && threadIdx.x < 4) s.control[12 + threadIdx.x] = 0u;
+    ok = ok && pad_grid_barrier(s.control, phase);
+    ok = ok && sweep_tiles<true>(s, phase, buf[warp], top[warp]);
+    if (!ok && threadIdx.x == 0) {
+        atomicExch(s.control + 2, 1u);
+        atomicOr(s.status + PDR_STATUS_PAD_ERROR, kErrTimeout);
+    }
+}
+
 struct FillParams {
     float* color;
     const float* snapshot;   // original colours; only when both sides exceed 12000
     const float* coverage;
     float* filled;
     const uint32_t* src_bits;
-    const uint32_t* field;  // final offsets, band-major (final_index)
+    const uint32_t* field;  // [H][W] source positions (bands == 0, pad_tiles_kernel) or band-major offsets (final_index)
     uint32_t channels, words_per_row, margin, fill_unobserved, bands;
+    bool color4;            // four channels at a 16-byte aligned base: texels move as float4
     int32_t W, H;
     unsigned long long margin2, limit2;
 };
@@ -348,8 +615,16 @@ __device__ __forceinline__ bool is_source(const FillParams& P, uint32_t x, uint3
 __device__ __forceinline__ int fill_decision(const FillParams& P, uint32_t x, uint32_t y, uint64_t& src,
                                              bool& covered) {
     const uint64_t p = (uint64_t)y * (uint32_t)P.W + x;
-    const uint32_t f = P.field[final_index(x, y, (uint32_t)P.W, P.bands)];
-    const int32_t ox = unpack_x(f), oy = unpack_y(f);
+    int32_t ox, oy;
+    if (P.bands) {
+        const uint32_t f = P.field[final_index(x, y, (uint32_t)P.W, P.bands)];
+        ox = unpack_x(f);
+        oy = unpack_y(f);
+    } else {
+        const uint32_t f = P.field[p];
+        ox = (int32_t)(f & 0xFFFFu) - (int32_t)x;
+        oy = (int32_t)(f >> 16) - (int32_t)y;
+    }
     const int32_t d2 = ox * ox + oy * oy;
     if (d2 >= 2 * kFar * kFar) return 0;
     const int32_t sx = (int32_t)x + ox, sy = (int32_t)y + oy;
@@ -368,10 +643,10 @@ __global__ void __launch_bounds__(kStatThreads) pad_fill_kernel(FillParams P, co
                                                                 unsigned long long* counters) {
     __shared__ unsigned long long red[kStatThreads / 32];
     if (control[2] != 0 || (stats[0] == 0 && stats[4] == 0)) return;
-    const uint64_t n = (uint64_t)(uint32_t)P.W * (uint32_t)P.H;
+    const uint32_t n = (uint32_t)P.W * (uint32_t)P.H;  // at most 2^28
     unsigned long long gutter = 0, unobserved = 0, remaining = 0;
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t y = (uint32_t)(p / (uint32_t)P.W), x = (uint32_t)(p % (uint32_t)P.W);
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+        const uint32_t y = p / (uint32_t)P.W, x = p - y * (uint32_t)P.W;
         if (is_source(P, x, y)) continue;
         uint64_t s = 0;
         bool covered = false;
@@ -399,8 +674,15 @@ __global__ void __launch_bounds__(kStatThreads) pad_fill_kernel(FillParams P, co
             }
             from = is_source(P, sx, sy) ? P.color : P.snapshot;
         }
-        for (uint32_t c = 0; c < P.channels; ++c) P.color[p * P.channels + c] = from[s * P.channels + c];
-        if (P.channels == 4) P.color[p * 4 + 3] = 1.0f;
+        if (P.color4) {
+            float4 q = reinterpret_cast<const float4*>(from)[s];
+            q.w = 1.0f;
+            reinterpret_cast<float4*>(P.color)[p] = q;
+        } else {
+            for (uint32_t c = 0; c < P.channels; ++c)
+                P.color[(uint64_t)p * P.channels + c] = from[s * P.channels + c];
+            if (P.channels == 4) P.color[(uint64_t)p * 4 + 3] = 1.0f;
+        }
         P.filled[p] = 1.0f;
         if (covered) ++unobserved;
         else ++gutter;
@@ -740,22 +1022,49 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
     unsigned long long* st64 = reinterpret_cast<unsigned long long*>(stats);
     cudaError_t e = cudaMemsetAsync(stats, 0, 5 * sizeof(uint64_t), s);
     if (!e) e = cudaMemsetAsync(ws, 0, L.bits, s);  // control + counters
-    if (!e) e = cudaMemsetAsync(boundary, 0x80, 2ull * bands * width * sizeof(uint32_t), s);
     if (e) return set_cuda_error(e, "pdr_pad_texture_atlas");
     const uint64_t words = (uint64_t)wpr * height;
     pad_classify_kernel<<<stat_blocks(words * 32), kStatThreads, 0, s>>>(valid_mask, coverage_mask, filled_mask, bits,
                                                                          wpr, width, height, valid_threshold, st64);
     uint32_t* field2 = reinterpret_cast<uint32_t*>(ws + L.field2);
-    if (width > 4384 || height > 4384) {
-        pad_sweep_kernel<false, true><<<bands, 32, 0, s>>>(bits, wpr, nullptr, field, boundary, control, status,
-                                                           (int32_t)width, (int32_t)height);
-        pad_sweep_kernel<true, true><<<bands, 32, 0, s>>>(bits, wpr, field, field2, boundary + (size_t)bands * width,
-                                                          control, status, (int32_t)width, (int32_t)height);
-    } else {
-        pad_sweep_kernel<false, false><<<bands, 32, 0, s>>>(bits, wpr, nullptr, field, boundary, control, status,
-                                                            (int32_t)width, (int32_t)height);
-        pad_sweep_kernel<true, false><<<bands, 32, 0, s>>>(bits, wpr, field, field2, boundary + (size_t)bands * width,
-                                                           control, status, (int32_t)width, (int32_t)height);
+    bool tiled = width <= (uint32_t)kTileMaxSide && height <= (uint32_t)kTileMaxSide;
+    if (tiled) {
+        TileSweeps T{};
+        T.src_bits = bits;
+        T.forward = field;
+        T.field = field2;
+        T.changed = reinterpret_cast<uint8_t*>(boundary);
+        T.control = control;
+        T.status = status;
+        T.words_per_row = wpr;
+        T.W = (int32_t)width;
+        T.H = (int32_t)height;
+        T.tiles_x = (int32_t)((width + kPadTileW - 1) / kPadTileW);
+        T.tiles = T.tiles_x * (int32_t)bands;
+        // every CTA resident (they meet at barriers): a cooperative launch of at most what the device holds
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pad_tiles_kernel, 32 * kPadWarps, 0);
+        if (e) return set_cuda_error(e, "pdr_pad_texture_atlas");
+        const int32_t want = (T.tiles + kPadWarps - 1) / kPadWarps, most = per_sm * num_sms();
+        void* args[] = {&T};
+        e = most > 0 ? cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(pad_tiles_kernel),
+                                                   dim3((unsigned)(want < most ? want : most)), dim3(32 * kPadWarps), args,
+                                                   0, s)
+                     : cudaErrorCooperativeLaunchTooLarge;
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            tiled = false;
+            cudaGetLastError();
+        } else if (e) {
+            return set_cuda_error(e, "pdr_pad_texture_atlas");
+        }
+    }
+    if (!tiled) {
+        e = cudaMemsetAsync(boundary, 0x80, 2ull * bands * width * sizeof(uint32_t), s);
+        if (e) return set_cuda_error(e, "pdr_pad_texture_atlas");
+        pad_sweep_kernel<false><<<bands, 32, 0, s>>>(bits, wpr, nullptr, field, boundary, control, status,
+                                                     (int32_t)width, (int32_t)height);
+        pad_sweep_kernel<true><<<bands, 32, 0, s>>>(bits, wpr, field, field2, boundary + (size_t)bands * width,
+                                                    control, status, (int32_t)width, (int32_t)height);
     }
     if (snapshot) {
         e = cudaMemcpyAsync(ws + L.snapshot, color, (size_t)width * height * channels * sizeof(float),
@@ -769,8 +1078,9 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
     P.filled = filled_mask;
     P.src_bits = bits;
     P.field = field2;
-    P.bands = bands;
+    P.bands = tiled ? 0u : bands;
     P.channels = channels;
+    P.color4 = channels == 4 && ((uintptr_t)color & 15u) == 0;
     P.words_per_row = wpr;
     P.margin = margin;
     P.fill_unobserved = fill_unobserved != 0;

@@ -186,3 +186,19 @@ def test_pad_texture_atlas_wrapper_and_project():
     ref = api.pad_texture_atlas(plain.color, (plain.valid_mask > 0).astype(np.float32), 3,
                                 coverage_mask=plain.coverage_mask, fill_unobserved=True)[0]
     assert same_bits(padded.color, ref) and same_bits(padded.valid_mask, plain.valid_mask)
+
+
+@pytest.mark.parametrize("h,w", [(31, 63), (32, 64), (33, 65), (1, 129), (64, 1), (200, 333), (700, 900), (33, 4384),
+                                 (4384, 33), (33, 4385)])
+def test_padding_tiles_sparse_sources_across_tiles(h, w):
+    """The tiled sweeps (64 x 32 tiles, sides up to 4384) and the banded ones beyond: one source, then a
+    handful, so that offsets travel through many tiles in every direction."""
+    rng = np.random.default_rng(h * 10007 + w)
+    for sources in (1, 6):
+        valid = np.zeros((h, w), np.float32)
+        valid[rng.integers(0, h, sources), rng.integers(0, w, sources)] = 1
+        color = rng.uniform(size=(h, w, 4)).astype(np.float32)
+        cov = (rng.uniform(size=(h, w)) > 0.5).astype(np.float32)
+        c, f, st = gpu_pad(color, valid, 50, cov, True)
+        oc, of, ost = api.pad_texture_atlas(color, valid, 50, coverage_mask=cov, fill_unobserved=True)
+        assert tuple(st) == ost and same_bits(c, oc) and same_bits(f, of), (h, w, sources)
