@@ -1065,7 +1065,6 @@ def run_gpu(args, world, rank, local):
         pipe.set_tile_config(cfg, int(pipe.check_capacity() * 1.25) + 1024)
     else:
         tune = pipe.autotune(clip, t_attrs, t_uv, tex)
-    r.render_tile_config = pipe.tile_config
     pipe.step(clip, t_attrs, t_uv, tex, g_attr, g_samp, stream)
     entries = pipe.check_capacity()
     for _ in range(args.warmup):

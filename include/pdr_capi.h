@@ -355,6 +355,13 @@ PDR_API pdr_status pdr_render_forward(const pdr_render_args* args, void* stream)
  * between calls (texture or attribute optimisation) bins once and rasterizes many times. */
 PDR_API pdr_status pdr_render_bin(const pdr_render_args* args, void* stream);
 PDR_API pdr_status pdr_render_raster(const pdr_render_args* args, void* stream);
+/* The images of pdr_render_forward, bit for bit, through a visibility buffer instead of tile lists: the tile
+ * members of the arguments and status are not used, nothing can overflow, and the workspace is
+ * pdr_render_direct_workspace_bytes() bytes, 16-byte aligned. Without attributes and uv attributes it is
+ * Rasterizer::forward (src/rasterizer.cpp:373-442) for all views. */
+PDR_API size_t pdr_render_direct_workspace_bytes(uint32_t views, uint32_t triangle_count, uint32_t width,
+                                                 uint32_t height);
+PDR_API pdr_status pdr_render_direct(const pdr_render_args* args, void* stream);
 /* The adjoints of the forward in one pixel pass: texture_backward, interpolate_backward for both
  * attribute sets (raster gradients summed) and rasterize_backward. With a 16-byte aligned workspace of
  * at least pdr_render_backward_workspace_bytes() bytes, the per-vertex gradients of each view are

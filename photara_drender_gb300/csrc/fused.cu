@@ -143,9 +143,9 @@ TileConfig tile_config(const pdr_render_args* a) {
     return {a->tile_width, a->tile_height, a->stage_triangles};
 }
 
-pdr_status check_render_forward(const pdr_render_args* a) {
-    if (!a || !a->clip_positions || !a->indices || !a->viewports || !a->raster || !a->tile_offsets ||
-        !a->tile_triangles || !a->workspace || !a->status)
+// The images and their inputs, whichever way the raster is made.
+pdr_status check_render_images(const pdr_render_args* a) {
+    if (!a || !a->clip_positions || !a->indices || !a->viewports || !a->raster)
         return set_error(PDR_INVALID_ARGUMENT, "render arguments are incomplete");
     if (a->views == 0 || a->vertex_count == 0 || a->triangle_count == 0 || a->width == 0 || a->height == 0)
         return set_error(PDR_INVALID_ARGUMENT, "render dimensions must be positive");
@@ -154,6 +154,14 @@ pdr_status check_render_forward(const pdr_render_args* a) {
     if (a->texture && (!a->uv_attributes || !a->uv || !a->sampled || a->texture_width == 0 || a->texture_height == 0 ||
                        a->address_mode > 2))
         return set_error(PDR_INVALID_ARGUMENT, "texture sampling needs uv attributes and uv/sampled outputs");
+    return PDR_OK;
+}
+
+pdr_status check_render_forward(const pdr_render_args* a) {
+    if (!a || !a->tile_offsets || !a->tile_triangles || !a->workspace || !a->status)
+        return set_error(PDR_INVALID_ARGUMENT, "render arguments are incomplete");
+    const pdr_status st = check_render_images(a);
+    if (st) return st;
     const TileConfig tc = tile_config(a);
     if (!raster_config_supported(tc.w, tc.h, tc.k))
         return set_error(PDR_INVALID_ARGUMENT, "tile shape and stage depth must be 16x16/256, 16x16/128 or 16x8/128");
@@ -199,6 +207,34 @@ pdr_status pdr_render_raster(const pdr_render_args* a, void* stream) {
 pdr_status pdr_render_forward(const pdr_render_args* a, void* stream) {
     const pdr_status st = pdr_render_bin(a, stream);
     return st ? st : pdr_render_raster(a, stream);
+}
+
+size_t pdr_render_direct_workspace_bytes(uint32_t views, uint32_t triangle_count, uint32_t width, uint32_t height) {
+    if (width == 0 || height == 0) return 0;
+    return direct_workspace_bytes(views, triangle_count, width, height);
+}
+
+pdr_status pdr_render_direct(const pdr_render_args* a, void* stream) {
+    pdr_status st = check_render_images(a);
+    if (st) return st;
+    st = check_raster_args(a->clip_positions, a->views, a->vertex_count, a->indices, a->triangle_count, a->width,
+                           a->height, a->viewports);
+    if (st) return st;
+    if (a->cull_mode > 2) return set_error(PDR_INVALID_ARGUMENT, "cull_mode must be 'none', 'back', or 'front'");
+    if (((uintptr_t)a->raster | (uintptr_t)a->barycentric_derivatives | (uintptr_t)a->sample_differences) & 15u)
+        return set_error(PDR_INVALID_ARGUMENT, "raster outputs and sample_differences must be 16-byte aligned");
+    if (!a->workspace || ((uintptr_t)a->workspace & 15u) ||
+        a->workspace_bytes < direct_workspace_bytes(a->views, a->triangle_count, a->width, a->height))
+        return set_error(PDR_INVALID_ARGUMENT, "workspace is smaller than pdr_render_direct_workspace_bytes()");
+    RasterShade shade{a->attributes, a->attribute_count, a->attributes ? a->interpolated : nullptr, a->uv_attributes,
+                      a->uv_attributes ? a->uv : nullptr, a->texture, a->texture_width, a->texture_height,
+                      a->address_mode, a->texture ? a->sampled : nullptr,
+                      a->texture ? a->sample_differences : nullptr};
+    const cudaError_t err = launch_raster_direct(
+        a->clip_positions, a->views, a->vertex_count, a->indices, a->triangle_count, a->width, a->height, a->viewports,
+        a->cull_mode, a->workspace, a->raster, a->barycentric_derivatives,
+        (a->attributes || a->uv_attributes) ? &shade : nullptr, (cudaStream_t)stream);
+    return set_cuda_error(err, "render_direct");
 }
 
 pdr_status pdr_render_backward(const pdr_render_args* a, void* stream) {

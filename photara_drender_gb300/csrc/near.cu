@@ -126,9 +126,10 @@ __global__ void remap_near_kernel(const float4* __restrict__ clip_all, uint32_t 
     const float4 p0 = __ldg(clip + vi.x), p1 = __ldg(clip + vi.y), p2 = __ldg(clip + vi.z);
     const float4 vp = viewports[view];
     const uint32_t x = (uint32_t)(p % W), y = (uint32_t)(p / W);
-    const WinnerBary wb = winner_barycentrics(p0, p1, p2, sample_ndc(x, vp.x, vp.z), sample_ndc(y, vp.y, vp.w));
+    const NdcAxis ax(vp.x, vp.z), ay(vp.y, vp.w);
+    const WinnerBary wb = winner_barycentrics(p0, p1, p2, ax.at(x), ay.at(y));
     raster[pix] = make_float4(wb.b0, wb.b1, wb.depth, (float)(k + 1));
-    if (deriv) deriv[pix] = winner_derivatives(p0, p1, p2, wb, vp);
+    if (deriv) deriv[pix] = winner_derivatives(p0, p1, p2, wb, ax, ay);
 }
 
 bool near_args_ok(const float* clip, uint32_t views, uint32_t V, const uint32_t* idx, uint32_t T) {

@@ -54,6 +54,12 @@ cudaError_t launch_raster_forward(const float* clip, uint32_t views, uint32_t V,
                                   float* raster, float* deriv, cudaStream_t stream,
                                   const RasterShade* shade = nullptr, const uint32_t* status = nullptr,
                                   uint32_t tile_w = 16, uint32_t tile_h = 16, uint32_t chunk = 256);
+// The same outputs through a visibility buffer, without tile bins (visibility.cu); workspace of
+// direct_workspace_bytes().
+size_t direct_workspace_bytes(uint32_t views, uint32_t T, uint32_t W, uint32_t H);
+cudaError_t launch_raster_direct(const float* clip, uint32_t views, uint32_t V, const uint32_t* idx, uint32_t T,
+                                 uint32_t W, uint32_t H, const float* viewports, uint32_t cull, void* workspace,
+                                 float* raster, float* deriv, const RasterShade* shade, cudaStream_t stream);
 // Tile shapes and stage depths the raster kernels are compiled for: 16x16 with 256 or 128 staged
 // triangles, 16x8 with 128 (shapes that divide the reference's 16x16 tile: triangle_tile_rect).
 bool raster_config_supported(uint32_t tile_w, uint32_t tile_h, uint32_t chunk);

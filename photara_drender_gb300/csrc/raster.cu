@@ -602,20 +602,7 @@ cudaError_t launch_raster_forward(const float* clip, uint32_t views, uint32_t V,
                                   const uint32_t* offsets, const uint32_t* list, unsigned long long capacity,
                                   float* raster, float* deriv, cudaStream_t stream, const RasterShade* shade,
                                   const uint32_t* status, uint32_t tile_w, uint32_t tile_h, uint32_t chunk) {
-    ShadeArgs sa{};
-    if (shade) {
-        sa.attrs = shade->attrs;
-        sa.A = shade->attribute_count;
-        sa.attr_out = shade->attr_out;
-        sa.uv_attrs = reinterpret_cast<const float2*>(shade->uv_attrs);
-        sa.uv_out = reinterpret_cast<float2*>(shade->uv_out);
-        sa.tex = reinterpret_cast<const float4*>(shade->texture);
-        sa.tw = shade->texture_width;
-        sa.th = shade->texture_height;
-        sa.mode = shade->address_mode;
-        sa.sampled = reinterpret_cast<float4*>(shade->sampled);
-        sa.sdiff = reinterpret_cast<float4*>(shade->sample_differences);
-    }
+    const ShadeArgs sa = shade ? shade_args(*shade) : ShadeArgs{};
     const float4* c4 = reinterpret_cast<const float4*>(clip);
     const uint3* i3 = reinterpret_cast<const uint3*>(idx);
     const float4* v4 = reinterpret_cast<const float4*>(viewports);

@@ -23,6 +23,7 @@
 
 #include "bin_rect.cuh"
 #include "pdr_common.cuh"
+#include "pdr_internal.h"
 
 namespace pdr {
 
@@ -37,7 +38,23 @@ struct ShadeArgs {
     uint32_t tw, th, mode;
     float4* sampled;        // [H][W][4]
     float4* sdiff;          // [H][W][2]: texel differences along u and v per channel, or nullptr
+    bool sdiff32;           // sdiff is 32-byte aligned
 };
+
+inline ShadeArgs shade_args(const RasterShade& s) {
+    return {s.attrs,
+            s.attribute_count,
+            s.attr_out,
+            reinterpret_cast<const float2*>(s.uv_attrs),
+            reinterpret_cast<float2*>(s.uv_out),
+            reinterpret_cast<const float4*>(s.texture),
+            s.texture_width,
+            s.texture_height,
+            s.address_mode,
+            reinterpret_cast<float4*>(s.sampled),
+            reinterpret_cast<float4*>(s.sample_differences),
+            ((uintptr_t)s.sample_differences & 31u) == 0};
+}
 
 // One view of one mesh as the tile routine sees it.
 struct RasterView {
@@ -73,13 +90,17 @@ constexpr uint32_t kRectLarge = 0xFFFFFFFFu;  // the bound does not apply: every
 // every passing sample lies in the vertex bounding box grown by D. Pixel indices come from inverting
 // sample_ndc with 0.05 pixel (plus 1e-6 of the viewport size) of slack for its rounding.
 // `err` receives 2e-6 L^2, the bound on |fl(e) - e| at any sample of the tile that the row spans use.
-__device__ __forceinline__ uint32_t pixel_rect(float s0x, float s0y, float s1x, float s1y, float s2x, float s2y,
-                                               float area, float4 vp, uint32_t x_org, uint32_t y_org, uint32_t x_end,
-                                               uint32_t y_end, float tsx_lo, float tsx_hi, float tsy_lo,
-                                               float tsy_hi, float& err) {
+enum class Bounds { kNone, kRect, kWhole };
+
+// The rectangle [x0, x1] x [y0, y1] in image pixels; kNone: empty, kWhole: the bound does not apply. pixw and
+// pixh are one pixel in NDC (2 / viewport size).
+__device__ __forceinline__ Bounds pixel_bounds(float s0x, float s0y, float s1x, float s1y, float s2x, float s2y,
+                                               float area, float4 vp, float pixw, float pixh, uint32_t x_org,
+                                               uint32_t y_org, uint32_t x_end, uint32_t y_end, float tsx_lo,
+                                               float tsx_hi, float tsy_lo, float tsy_hi, float& err, uint32_t& x0,
+                                               uint32_t& x1, uint32_t& y0, uint32_t& y1) {
     const float mnx = fminf(s0x, fminf(s1x, s2x)), mxx = fmaxf(s0x, fmaxf(s1x, s2x));
     const float mny = fminf(s0y, fminf(s1y, s2y)), mxy = fmaxf(s0y, fmaxf(s1y, s2y));
-    const float pxw = 2.0f / vp.z, pyw = 2.0f / vp.w;  // one pixel in NDC
     const float ext = fmaxf(mxx - mnx, mxy - mny);
     // |a - s| over vertices and tile samples (tile sample ranges [tsx_lo, tsx_hi] x [tsy_lo, tsy_hi]), 1% up
     const float L = 1.01f * fmaxf(fmaxf(fabsf(mxx - tsx_lo), fabsf(tsx_hi - mnx)),
@@ -89,8 +110,8 @@ __device__ __forceinline__ uint32_t pixel_rect(float s0x, float s0y, float s1x, 
     err = 2e-6f * L * L;
     const float tau = 1e-7f + err;
     const float D = 2.0f * tau * perim / fabsf(area);
-    // NaN-safe: every comparison with a NaN fails and sends the triangle to the warp path
-    if (!(D <= fminf(pxw, pyw)) || !(fabsf(area) >= 1e-4f * ext * ext)) return kRectLarge;
+    // NaN-safe: every comparison with a NaN fails and leaves the bound unused
+    if (!(D <= fminf(pixw, pixh)) || !(fabsf(area) >= 1e-4f * ext * ext)) return Bounds::kWhole;
     const float slx = 0.05f + 1e-6f * (vp.z + fabsf(vp.x)), sly = 0.05f + 1e-6f * (vp.w + fabsf(vp.y));
     // p = (s + 1) * size / 2 + origin - 0.5 inverts sample_ndc
     const float fx0 = ceilf(((mnx - D) + 1.0f) * 0.5f * vp.z + vp.x - 0.5f - slx);
@@ -99,10 +120,24 @@ __device__ __forceinline__ uint32_t pixel_rect(float s0x, float s0y, float s1x, 
     const float fy1 = floorf(((mxy + D) + 1.0f) * 0.5f * vp.w + vp.y - 0.5f + sly);
     const float cx0 = fmaxf(fx0, (float)x_org), cx1 = fminf(fx1, (float)(x_end - 1u));
     const float cy0 = fmaxf(fy0, (float)y_org), cy1 = fminf(fy1, (float)(y_end - 1u));
-    if (!(cx0 <= cx1) || !(cy0 <= cy1)) return kRectNone;
-    const uint32_t x0 = (uint32_t)cx0 - x_org, x1 = (uint32_t)cx1 - x_org;
-    const uint32_t y0 = (uint32_t)cy0 - y_org, y1 = (uint32_t)cy1 - y_org;
-    return x0 | (x1 << 8) | (y0 << 16) | (y1 << 24);
+    if (!(cx0 <= cx1) || !(cy0 <= cy1)) return Bounds::kNone;
+    x0 = (uint32_t)cx0;
+    x1 = (uint32_t)cx1;
+    y0 = (uint32_t)cy0;
+    y1 = (uint32_t)cy1;
+    return Bounds::kRect;
+}
+
+// pixel_bounds packed tile-local (tiles of at most 64 x 64), or kRectNone / kRectLarge.
+__device__ __forceinline__ uint32_t pixel_rect(float s0x, float s0y, float s1x, float s1y, float s2x, float s2y,
+                                               float area, float4 vp, uint32_t x_org, uint32_t y_org, uint32_t x_end,
+                                               uint32_t y_end, float tsx_lo, float tsx_hi, float tsy_lo,
+                                               float tsy_hi, float& err) {
+    uint32_t x0, x1, y0, y1;
+    const Bounds b = pixel_bounds(s0x, s0y, s1x, s1y, s2x, s2y, area, vp, 2.0f / vp.z, 2.0f / vp.w, x_org, y_org,
+                                  x_end, y_end, tsx_lo, tsx_hi, tsy_lo, tsy_hi, err, x0, x1, y0, y1);
+    if (b != Bounds::kRect) return b == Bounds::kNone ? kRectNone : kRectLarge;
+    return (x0 - x_org) | ((x1 - x_org) << 8) | ((y0 - y_org) << 16) | ((y1 - y_org) << 24);
 }
 
 // Row spans of a candidate rectangle [x0, x1] x [y0, y1] (tile-local, at most 8 rows of at most 16
@@ -121,13 +156,10 @@ __device__ __forceinline__ uint32_t pixel_rect(float s0x, float s0y, float s1x, 
 // slack. NaN or infinite terms leave the row unconstrained.
 // span_coefficients computes, once per (tile, triangle), A = (alpha per edge, -1 / beta of edge 0),
 // G = (gamma per edge, -1 / beta of edge 1) and -1 / beta of edge 2 (0 where beta is 0).
-__device__ __forceinline__ void span_coefficients(float4 ea, float4 eb, float err, uint32_t x0, uint32_t x1, uint32_t y0,
-                                                  uint32_t y1, const float* tile_sx, const float* tile_sy, float4& A,
-                                                  float4& G, float& nb2) {
+__device__ __forceinline__ void span_coefficients(float4 ea, float4 eb, float err, uint32_t nx, uint32_t ny, float sxa,
+                                                  float sxb, float sya, float syc, float4& A, float4& G, float& nb2) {
     const float sgn = eb.z;
-    const float sxa = tile_sx[x0], sxb = tile_sx[x1], sya = tile_sy[y0], syc = tile_sy[y1];
     const float vx[3] = {ea.x, ea.z, eb.x}, vy[3] = {ea.y, ea.w, eb.y};
-    const uint32_t nx = x1 - x0;
     float al[3], ga[3], nb[3];
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
@@ -138,7 +170,7 @@ __device__ __forceinline__ void span_coefficients(float4 ea, float4 eb, float er
         const float e01 = cross2(ax - sxa, ay - syc, bx - sxa, by - syc);
         const float mag = fabsf(e00) + fabsf(e10) + fabsf(e01);
         const float beta = nx ? sgn * (e10 - e00) : 0.0f;
-        ga[e] = y1 > y0 ? sgn * (e01 - e00) : 0.0f;
+        ga[e] = ny ? sgn * (e01 - e00) : 0.0f;
         al[e] = sgn * e00 + ((1e-7f + 4.0f * err) + 4e-6f * mag);
         nb[e] = beta != 0.0f ? -1.0f / beta : 0.0f;
     }
@@ -147,14 +179,13 @@ __device__ __forceinline__ void span_coefficients(float4 ea, float4 eb, float er
     nb2 = nb[2];
 }
 
-// The span of row y0 + i of rectangle [x0, x1] x [y0, y1]: (first column) | (width << 8), width 0 when no
-// column of the row can pass.
-__device__ __forceinline__ uint32_t row_span(float4 A, float4 G, float nb2, uint32_t x0, uint32_t x1, uint32_t y0,
-                                             uint32_t y1, uint32_t i, const float* tile_sy, float slx) {
-    const float sya = tile_sy[y0];
-    const float inv_dy = y1 > y0 ? 1.0f / (tile_sy[y1] - sya) : 0.0f;
-    const float v = (tile_sy[y0 + i] - sya) * inv_dy;
-    const float fnx = (float)(x1 - x0);
+// The span of the row at sample sy of a rectangle with nx + 1 columns whose first row is at sample sya and
+// whose rows cover 1 / inv_dy (inv_dy 0: one row): first column (from the rectangle's) and width, 0 when
+// no column of the row can pass.
+__device__ __forceinline__ uint32_t row_span(float4 A, float4 G, float nb2, uint32_t nx, float sy, float sya,
+                                             float inv_dy, float slx, uint32_t& first) {
+    const float v = (sy - sya) * inv_dy;
+    const float fnx = (float)nx;
     const float al[3] = {A.x, A.y, A.z}, ga[3] = {G.x, G.y, G.z}, nb[3] = {A.w, G.w, nb2};
     float lo = 0.0f, hi = 1.0f;
     bool empty = false;
@@ -165,11 +196,12 @@ __device__ __forceinline__ uint32_t row_span(float4 A, float4 G, float nb2, uint
         else if (nb[e] > 0.0f) hi = fminf(hi, a * nb[e]);  // beta < 0: t <= -a / beta
         else if (a < 0.0f) empty = true;                   // beta = 0: the whole row or none of it
     }
+    first = 0u;
     if (empty || !(lo <= hi)) return 0u;
     const float cl = fmaxf(ceilf(lo * fnx - slx), 0.0f), ch = fminf(floorf(hi * fnx + slx), fnx);
     if (!(cl <= ch)) return 0u;
-    const uint32_t c0 = (uint32_t)cl;
-    return (x0 + c0) | (((uint32_t)ch - c0 + 1u) << 8);
+    first = (uint32_t)cl;
+    return (uint32_t)ch - first + 1u;
 }
 
 // Four nibbles from the low nibbles of four bytes (byte j -> bits 4j .. 4j + 3).
@@ -177,6 +209,34 @@ __device__ __forceinline__ uint32_t pack_nibbles(uint32_t v) {
     v = (v | (v >> 4)) & 0x00FF00FFu;
     return (v | (v >> 8)) & 0xFFFFu;
 }
+
+// One axis of a viewport with the reciprocal of its size, for divisions by that size without a division: the
+// quotient a / b by a fixed divisor is q = RN(a y), r = RN(a - q b), RN(q + r y) with y = RN(1 / b), which is
+// correctly rounded (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990, theorem 8.2) unless b's significand is all ones, and while nothing under- or overflows:
+// `exact` and the bounds on a keep both away. Otherwise the division itself.
+struct NdcAxis {
+    float v0, size, rcp;
+    bool exact;
+    __device__ __forceinline__ NdcAxis(float origin, float extent) : v0(origin), size(extent), rcp(1.0f / extent) {
+        exact = extent >= 1e-6f && extent <= 1e9f && fabsf(origin) <= 1e9f &&
+                (__float_as_uint(extent) & 0x7fffffu) != 0x7fffffu;
+    }
+    __device__ __forceinline__ float quotient(float a) const {  // exact, and a zero or of moderate size
+        const float q = a * rcp;
+        return __fmaf_rn(__fmaf_rn(-q, size, a), rcp, q);
+    }
+    // sample_ndc
+    __device__ __forceinline__ float at(uint32_t p) const {
+        if (!exact) return sample_ndc(p, v0, size);
+        return quotient(((float)p - v0 + 0.5f) * 2.0f) - 1.0f;
+    }
+    // a / size
+    __device__ __forceinline__ float divide(float a) const {
+        const float m = fabsf(a);
+        return exact && m >= 1e-25f && m <= 1e25f ? quotient(a) : a / size;
+    }
+};
 
 // The winner's outputs at sample (sx, sy), rasterize_forward.hlsl's arithmetic: clamped barycentrics,
 // 1 / area and clamped depth; and its pixel derivatives [du/dx, du/dy, dv/dx, dv/dy]. Shared with the
@@ -203,7 +263,8 @@ __device__ __forceinline__ WinnerBary winner_barycentrics(float4 p0, float4 p1, 
     return r;
 }
 
-__device__ __forceinline__ float4 winner_derivatives(float4 p0, float4 p1, float4 p2, const WinnerBary& w, float4 vp) {
+__device__ __forceinline__ float4 winner_derivatives(float4 p0, float4 p1, float4 p2, const WinnerBary& w,
+                                                     const NdcAxis& ax, const NdcAxis& ay) {
     const float da0_dx = -p1.w * p2.y + p2.w * p1.y;
     const float da0_dy = -p1.x * p2.w + p1.w * p2.x;
     const float da1_dx = -p2.w * p0.y + p2.y * p0.w;
@@ -212,8 +273,8 @@ __device__ __forceinline__ float4 winner_derivatives(float4 p0, float4 p1, float
     const float da2_dy = -p0.x * p1.w + p0.w * p1.x;
     const float dadx = da0_dx + da1_dx + da2_dx;
     const float dady = da0_dy + da1_dy + da2_dy;
-    return make_float4((da0_dx - w.b0 * dadx) * w.binv * 2.0f / vp.z, (da0_dy - w.b0 * dady) * w.binv * 2.0f / vp.w,
-                       (da1_dx - w.b1 * dadx) * w.binv * 2.0f / vp.z, (da1_dy - w.b1 * dady) * w.binv * 2.0f / vp.w);
+    return make_float4(ax.divide((da0_dx - w.b0 * dadx) * w.binv * 2.0f), ay.divide((da0_dy - w.b0 * dady) * w.binv * 2.0f),
+                       ax.divide((da1_dx - w.b1 * dadx) * w.binv * 2.0f), ay.divide((da1_dy - w.b1 * dady) * w.binv * 2.0f));
 }
 
 // Orders (depth, triangle) pairs as the reference's depth test does: nearest depth first (-0 and
@@ -225,83 +286,108 @@ __device__ __forceinline__ unsigned long long depth_key(float depth, uint32_t t)
     return ((unsigned long long)o << 32) | t;
 }
 
+// 32 bytes with one store (addr 32-byte aligned), streaming.
+__device__ __forceinline__ void store_v8_cs(float4* addr, float4 a, float4 b) {
+    asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(addr), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 // The outputs of pixel (px, py) of a view whose winner is triangle best_tri - 1 (0: no triangle): the
 // winner's barycentrics and depth recomputed with the reference's arithmetic (rasterize_forward.hlsl),
-// its pixel derivatives, and the shading (interpolate_forward.hlsl, texture_forward.hlsl): the tile
-// routine's epilogue.
-template <bool kDeriv, bool kShade>
+// its pixel derivatives, and the shading (interpolate_forward.hlsl, texture_forward.hlsl): the epilogue of the
+// tile routine and the visibility buffer's shading pass. kA >= 0: that many attributes, whose gathers are then
+// issued with the positions' instead of one attribute after the other. Images are written once and read, if at
+// all, after the whole pass: streaming stores leave L2 to the vertices and the texture.
+template <bool kDeriv, bool kShade, int kA = -1>
 __device__ __forceinline__ void shade_pixel(const RasterView& v, uint32_t px, uint32_t py, size_t pix,
                                             uint32_t best_tri) {
     const ShadeArgs& shade = v.shade;
+    const uint32_t A = kA >= 0 ? (uint32_t)kA : (shade.attr_out ? shade.A : 0u);
     if (best_tri == 0u) {
-        v.raster[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (kDeriv) v.deriv[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        __stcs(v.raster + pix, zero);
+        if (kDeriv) __stcs(v.deriv + pix, zero);
         if (kShade) {
-            if (shade.attr_out)
-                for (uint32_t a = 0; a < shade.A; ++a) shade.attr_out[pix * shade.A + a] = 0.0f;
-            if (shade.uv_out) shade.uv_out[pix] = make_float2(0.0f, 0.0f);
-            if (shade.sampled) shade.sampled[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (uint32_t a = 0; a < A; ++a) __stcs(shade.attr_out + pix * A + a, 0.0f);
+            if (shade.uv_out) __stcs(shade.uv_out + pix, make_float2(0.0f, 0.0f));
+            if (shade.sampled) __stcs(shade.sampled + pix, zero);
         }
         return;
     }
     const float4 vp = v.vp;
-    const float sx = sample_ndc(px, vp.x, vp.z);
-    const float sy = sample_ndc(py, vp.y, vp.w);
+    const NdcAxis ax(vp.x, vp.z), ay(vp.y, vp.w);
     const uint3 vi = v.idx[best_tri - 1];
     const float4 p0 = v.clip[vi.x], p1 = v.clip[vi.y], p2 = v.clip[vi.z];
-    const WinnerBary wb = winner_barycentrics(p0, p1, p2, sx, sy);
-    const float bb0 = wb.b0, bb1 = wb.b1;
-    v.raster[pix] = make_float4(bb0, bb1, wb.depth, (float)best_tri);
-    if (kDeriv) v.deriv[pix] = winner_derivatives(p0, p1, p2, wb, vp);
-    if (kShade) {
-        // interpolate_forward.hlsl for the winner (id <= T and indices < V hold here), then
-        // texture_forward.hlsl at the interpolated uv: the same arithmetic as the separate kernels.
-        const float u = bb0, vv = bb1, w = 1.0f - u - vv;
-        if (shade.attr_out) {
-            const float* at = shade.attrs;
-            const uint32_t A = shade.A;
-            for (uint32_t a = 0; a < A; ++a)
-                shade.attr_out[pix * A + a] = u * __ldg(at + (size_t)vi.x * A + a) + vv * __ldg(at + (size_t)vi.y * A + a) +
-                                              w * __ldg(at + (size_t)vi.z * A + a);
+    constexpr int kN = kA > 0 ? kA : 1;
+    float t0[kN], t1[kN], t2[kN];
+    if (kShade && kA > 0) {
+#pragma unroll
+        for (int a = 0; a < kA; ++a) {
+            t0[a] = __ldg(shade.attrs + (size_t)vi.x * kA + a);
+            t1[a] = __ldg(shade.attrs + (size_t)vi.y * kA + a);
+            t2[a] = __ldg(shade.attrs + (size_t)vi.z * kA + a);
         }
-        if (shade.uv_out) {
-            const float2 t0 = __ldg(shade.uv_attrs + vi.x), t1 = __ldg(shade.uv_attrs + vi.y), t2 = __ldg(shade.uv_attrs + vi.z);
-            const float2 uvp = make_float2(u * t0.x + vv * t1.x + w * t2.x, u * t0.y + vv * t1.y + w * t2.y);
-            shade.uv_out[pix] = uvp;
-            if (shade.sampled) {
-                const float tx_ = uvp.x * (float)shade.tw - 0.5f, ty_ = uvp.y * (float)shade.th - 0.5f;
-                const int32_t bx = f2i_sat(floorf(tx_)), by = f2i_sat(floorf(ty_));
-                const float fx = tx_ - floorf(tx_), fy = ty_ - floorf(ty_);
-                const int32_t x0 = address_coordinate(bx, shade.tw, shade.mode), x1 = address_coordinate(add1(bx), shade.tw, shade.mode);
-                const int32_t y0 = address_coordinate(by, shade.th, shade.mode), y1 = address_coordinate(add1(by), shade.th, shade.mode);
-                const float w0 = (1.0f - fx) * (1.0f - fy), w1 = fx * (1.0f - fy), w2 = (1.0f - fx) * fy, w3 = fx * fy;
-                const float4 c0 = __ldg(shade.tex + (size_t)(uint32_t)y0 * shade.tw + (uint32_t)x0);
-                const float4 c1 = __ldg(shade.tex + (size_t)(uint32_t)y0 * shade.tw + (uint32_t)x1);
-                const float4 c2 = __ldg(shade.tex + (size_t)(uint32_t)y1 * shade.tw + (uint32_t)x0);
-                const float4 c3 = __ldg(shade.tex + (size_t)(uint32_t)y1 * shade.tw + (uint32_t)x1);
-                float4 r;
-                r.x = c0.x * w0 + c1.x * w1 + c2.x * w2 + c3.x * w3;
-                r.y = c0.y * w0 + c1.y * w1 + c2.y * w2 + c3.y * w3;
-                r.z = c0.z * w0 + c1.z * w1 + c2.z * w2 + c3.z * w3;
-                r.w = c0.w * w0 + c1.w * w1 + c2.w * w2 + c3.w * w3;
-                shade.sampled[pix] = r;
-                if (shade.sdiff) {
-                    // texture_grad_uv.hlsl's texel differences (c0 = c00, c1 = c10, c2 = c01, c3 = c11),
-                    // kept for the backward so it does not gather the texels again
-                    float4 du, dv;
-                    du.x = (1.0f - fy) * (c1.x - c0.x) + fy * (c3.x - c2.x);
-                    du.y = (1.0f - fy) * (c1.y - c0.y) + fy * (c3.y - c2.y);
-                    du.z = (1.0f - fy) * (c1.z - c0.z) + fy * (c3.z - c2.z);
-                    du.w = (1.0f - fy) * (c1.w - c0.w) + fy * (c3.w - c2.w);
-                    dv.x = (1.0f - fx) * (c2.x - c0.x) + fx * (c3.x - c1.x);
-                    dv.y = (1.0f - fx) * (c2.y - c0.y) + fx * (c3.y - c1.y);
-                    dv.z = (1.0f - fx) * (c2.z - c0.z) + fx * (c3.z - c1.z);
-                    dv.w = (1.0f - fx) * (c2.w - c0.w) + fx * (c3.w - c1.w);
-                    shade.sdiff[pix * 2] = du;
-                    shade.sdiff[pix * 2 + 1] = dv;
-                }
-            }
-        }
+    }
+    float2 c0 = make_float2(0.0f, 0.0f), c1 = c0, c2 = c0;
+    if (kShade && shade.uv_out) {
+        c0 = __ldg(shade.uv_attrs + vi.x);
+        c1 = __ldg(shade.uv_attrs + vi.y);
+        c2 = __ldg(shade.uv_attrs + vi.z);
+    }
+    const WinnerBary wb = winner_barycentrics(p0, p1, p2, ax.at(px), ay.at(py));
+    // interpolate_forward.hlsl for the winner (id <= T and indices < V hold here), then texture_forward.hlsl at
+    // the interpolated uv: the same arithmetic as the separate kernels.
+    const float u = wb.b0, vv = wb.b1, w = 1.0f - u - vv;
+    __stcs(v.raster + pix, make_float4(u, vv, wb.depth, (float)best_tri));
+    if (kDeriv) __stcs(v.deriv + pix, winner_derivatives(p0, p1, p2, wb, ax, ay));
+    if (!kShade) return;
+    if (kA >= 0) {
+#pragma unroll
+        for (int a = 0; a < kA; ++a) __stcs(shade.attr_out + pix * kA + a, u * t0[a] + vv * t1[a] + w * t2[a]);
+    } else {
+        const float* at = shade.attrs;
+        for (uint32_t a = 0; a < A; ++a)
+            __stcs(shade.attr_out + pix * A + a, u * __ldg(at + (size_t)vi.x * A + a) + vv * __ldg(at + (size_t)vi.y * A + a) +
+                                                     w * __ldg(at + (size_t)vi.z * A + a));
+    }
+    if (!shade.uv_out) return;
+    const float2 uvp = make_float2(u * c0.x + vv * c1.x + w * c2.x, u * c0.y + vv * c1.y + w * c2.y);
+    __stcs(shade.uv_out + pix, uvp);
+    if (!shade.sampled) return;
+    const float tx_ = uvp.x * (float)shade.tw - 0.5f, ty_ = uvp.y * (float)shade.th - 0.5f;
+    const int32_t bx = f2i_sat(floorf(tx_)), by = f2i_sat(floorf(ty_));
+    const float fx = tx_ - floorf(tx_), fy = ty_ - floorf(ty_);
+    const int32_t x0 = address_coordinate(bx, shade.tw, shade.mode), x1 = address_coordinate(add1(bx), shade.tw, shade.mode);
+    const int32_t y0 = address_coordinate(by, shade.th, shade.mode), y1 = address_coordinate(add1(by), shade.th, shade.mode);
+    const float w0 = (1.0f - fx) * (1.0f - fy), w1 = fx * (1.0f - fy), w2 = (1.0f - fx) * fy, w3 = fx * fy;
+    const float4 k0 = __ldg(shade.tex + (size_t)(uint32_t)y0 * shade.tw + (uint32_t)x0);
+    const float4 k1 = __ldg(shade.tex + (size_t)(uint32_t)y0 * shade.tw + (uint32_t)x1);
+    const float4 k2 = __ldg(shade.tex + (size_t)(uint32_t)y1 * shade.tw + (uint32_t)x0);
+    const float4 k3 = __ldg(shade.tex + (size_t)(uint32_t)y1 * shade.tw + (uint32_t)x1);
+    float4 r;
+    r.x = k0.x * w0 + k1.x * w1 + k2.x * w2 + k3.x * w3;
+    r.y = k0.y * w0 + k1.y * w1 + k2.y * w2 + k3.y * w3;
+    r.z = k0.z * w0 + k1.z * w1 + k2.z * w2 + k3.z * w3;
+    r.w = k0.w * w0 + k1.w * w1 + k2.w * w2 + k3.w * w3;
+    __stcs(shade.sampled + pix, r);
+    if (!shade.sdiff) return;
+    // texture_grad_uv.hlsl's texel differences (k0 = c00, k1 = c10, k2 = c01, k3 = c11), kept for the backward
+    // so it does not gather the texels again
+    float4 du, dv;
+    du.x = (1.0f - fy) * (k1.x - k0.x) + fy * (k3.x - k2.x);
+    du.y = (1.0f - fy) * (k1.y - k0.y) + fy * (k3.y - k2.y);
+    du.z = (1.0f - fy) * (k1.z - k0.z) + fy * (k3.z - k2.z);
+    du.w = (1.0f - fy) * (k1.w - k0.w) + fy * (k3.w - k2.w);
+    dv.x = (1.0f - fx) * (k2.x - k0.x) + fx * (k3.x - k1.x);
+    dv.y = (1.0f - fx) * (k2.y - k0.y) + fx * (k3.y - k1.y);
+    dv.z = (1.0f - fx) * (k2.z - k0.z) + fx * (k3.z - k1.z);
+    dv.w = (1.0f - fx) * (k2.w - k0.w) + fx * (k3.w - k1.w);
+    if (shade.sdiff32) {
+        store_v8_cs(shade.sdiff + pix * 2, du, dv);
+    } else {
+        __stcs(shade.sdiff + pix * 2, du);
+        __stcs(shade.sdiff + pix * 2 + 1, dv);
     }
 }
 
@@ -402,9 +488,9 @@ __device__ __forceinline__ void raster_tile(const RasterView& v, uint32_t tx, ui
                     y1 = rect >> 24;
                 }
                 if (rect != kRectNone && (x1 - x0 + 1u) * (y1 - y0 + 1u) > kSpanMin) {
-                    span_coefficients(make_float4(s0x, s0y, s1x, s1y), make_float4(s2x, s2y, sgn, 0.0f), err, x0, x1,
-                                      y0, y1, tile_sx, tile_sy, span_a[threadIdx.x], span_g[threadIdx.x],
-                                      span_n[threadIdx.x]);
+                    span_coefficients(make_float4(s0x, s0y, s1x, s1y), make_float4(s2x, s2y, sgn, 0.0f), err, x1 - x0,
+                                      y1 - y0, tile_sx[x0], tile_sx[x1], tile_sy[y0], tile_sy[y1],
+                                      span_a[threadIdx.x], span_g[threadIdx.x], span_n[threadIdx.x]);
                     span_list[atomicAdd(&span_count, 1u)] = (uint8_t)threadIdx.x;
                 }
             }
@@ -423,9 +509,13 @@ __device__ __forceinline__ void raster_tile(const RasterView& v, uint32_t tx, ui
                     y0 = (rc >> 16) & 0xFFu;
                     y1 = rc >> 24;
                 }
-                spans[kk][i] = (uint16_t)(i <= y1 - y0 ? row_span(span_a[kk], span_g[kk], span_n[kk], x0, x1, y0, y1, i,
-                                                                  tile_sy, slx)
-                                                       : 0u);
+                uint32_t first = 0, width = 0;
+                if (i <= y1 - y0) {
+                    const float inv_dy = y1 > y0 ? 1.0f / (tile_sy[y1] - tile_sy[y0]) : 0.0f;
+                    width = row_span(span_a[kk], span_g[kk], span_n[kk], x1 - x0, tile_sy[y0 + i], tile_sy[y0], inv_dy,
+                                     slx, first);
+                }
+                spans[kk][i] = (uint16_t)(width ? (x0 + first) | (width << 8) : 0u);
             }
             __syncthreads();
             if (threadIdx.x == 0) span_count = 0;  // read by every thread above; rewritten after the next barrier

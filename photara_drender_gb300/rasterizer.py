@@ -261,6 +261,26 @@ class Rasterizer:
         return clip
 
     # -- rasterize ----------------------------------------------------------------------------
+    def _raster(self, clip: torch.Tensor, idx: torch.Tensor, width: int, height: int, vps: torch.Tensor, cull: int,
+                raster: torch.Tensor, deriv: Optional[torch.Tensor]) -> None:
+        """Raster (and derivatives) of every view through a visibility buffer: pdr_render_direct without shading.
+        Nothing in it can overflow, so nothing waits."""
+        from .pipeline import RenderArgsC
+
+        ctx = self.context
+        views, V = clip.shape[0], clip.shape[1]
+        T = idx.shape[0]
+        ws = torch.empty(_native.lib().pdr_render_direct_workspace_bytes(views, T, width, height), dtype=torch.uint8,
+                         device=ctx.device)
+        a = RenderArgsC()
+        a.clip_positions, a.views, a.vertex_count = clip.data_ptr(), views, V
+        a.indices, a.triangle_count, a.width, a.height = idx.data_ptr(), T, width, height
+        a.viewports, a.cull_mode, a.raster = vps.data_ptr(), cull, raster.data_ptr()
+        if deriv is not None:
+            a.barycentric_derivatives = deriv.data_ptr()
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        _native.call("pdr_render_direct", C.addressof(a), ctx.stream())
+
     def forward(self, positions, indices, resolution, cull_mode: str = "none",
                 output_barycentric_derivatives: bool = True, viewport=None, *, clip_near_plane: bool = False):
         """Rasterizer::forward (src/rasterizer.cpp:373-442). resolution is (height, width).
@@ -290,15 +310,11 @@ class Rasterizer:
                 cidx = torch.empty((2 * T, 3), dtype=torch.int32, device=ctx.device)
                 _native.call("pdr_clip_near", _ptr(clip), views, V, _ptr(idx), T, _ptr(cpos), _ptr(cidx), None,
                              ctx.stream())
-                offsets, lst, capacity, _ = self._bin(cpos, cidx, w, h, vps)
-                _native.call("pdr_rasterize_forward", _ptr(cpos), views, 4 * T, _ptr(cidx), 2 * T, w, h, _ptr(vps),
-                             cull, _ptr(offsets), _ptr(lst), capacity, _ptr(raster), _ptr(deriv), ctx.stream())
+                self._raster(cpos, cidx, w, h, vps, cull, raster, deriv)
                 _native.call("pdr_remap_near", _ptr(clip), views, V, _ptr(idx), T, w, h, _ptr(vps), _ptr(raster),
                              _ptr(deriv), ctx.stream())
             else:
-                offsets, lst, capacity, _ = self._bin(clip, idx, w, h, vps)
-                _native.call("pdr_rasterize_forward", _ptr(clip), views, V, _ptr(idx), idx.shape[0], w, h, _ptr(vps),
-                             cull, _ptr(offsets), _ptr(lst), capacity, _ptr(raster), _ptr(deriv), ctx.stream())
+                self._raster(clip, idx, w, h, vps, cull, raster, deriv)
             if deriv is None:
                 deriv = torch.empty((views, 0, 0, 4), dtype=torch.float32, device=ctx.device)
             if not batched:

@@ -185,20 +185,14 @@ _MODES = {"none": 0, "back": 1, "front": 2}
 _ADDRESS = {"clamp": 0, "wrap": 1, "mirror": 2}
 
 
-def _apply_status(r: Rasterizer, reports) -> None:
-    """Acts on status blocks of earlier calls that did not wait for their work: grows the tile-list
-    capacity to what the binning needed, raises the errors the device recorded."""
+def _apply_status(reports) -> None:
+    """Raises the errors the device recorded in status blocks of earlier calls that did not wait for them."""
     from . import _native
 
-    for kind, st in reports:
-        if kind == "render_forward":
-            if st[_native.STATUS_TILE_ENTRIES_HI] != 0:
-                raise OverflowError("Tile triangle list exceeds backend limits")
-            total = st[_native.STATUS_TILE_ENTRIES] & 0xFFFFFFFF
-            r._render_capacity = max(getattr(r, "_render_capacity", 0), total + total // 8 + 1024)
-        elif st[_native.STATUS_TEXEL_ERROR] == 1:
+    for _, st in reports:
+        if st[_native.STATUS_TEXEL_ERROR] == 1:
             raise ValueError("uv contains a non-finite value in a covered pixel")
-        elif st[_native.STATUS_TEXEL_ERROR] == 2:
+        if st[_native.STATUS_TEXEL_ERROR] == 2:
             raise IndexError("uv is too large for portable texture addressing")
 
 
@@ -224,26 +218,20 @@ def _cached_viewports(r: Rasterizer, viewport, views: int, w: int, h: int) -> to
 
 def check_deferred_errors(rasterizer: Rasterizer) -> None:
     """Waits for every `render(..., deferred_errors=True)` call made on this rasterizer and raises the
-    first error the device recorded for them (ValueError / IndexError / OverflowError, as the
-    synchronous path raises at once)."""
+    first error the device recorded for them (ValueError / IndexError, as the synchronous path raises at once)."""
     with rasterizer.context.lock:
-        _apply_status(rasterizer, rasterizer.context.poll_status(wait=True, kinds=("render_forward",
-                                                                                   "render_backward")))
+        _apply_status(rasterizer.context.poll_status(wait=True, kinds=("render_backward",)))
 
 
-def _render_forward(r: Rasterizer, clip, idx, h, w, attrs, uv_attrs, tex, vps, cull, mode, deferred=False):
+def _render_forward(r: Rasterizer, clip, idx, h, w, attrs, uv_attrs, tex, vps, cull, mode):
+    """One pdr_render_direct: triangles into a visibility buffer, one shading pass. Nothing waits."""
     from . import _native
     from .pipeline import RenderArgsC
-    from .rasterizer import TILE, _ptr
 
     ctx = r.context
     dev = ctx.device
     views, V = clip.shape[0], clip.shape[1]
     T = idx.shape[0]
-    # tile shape and stage depth of the fused binning and raster (pipeline.TILE_CONFIGS; outputs do not
-    # depend on it): the rasterizer's render_tile_config, e.g. one RenderFwdBwd.autotune picked
-    tw_, th_, stage = getattr(r, "render_tile_config", (TILE, TILE, 256))
-    tiles = ((w + tw_ - 1) // tw_) * ((h + th_ - 1) // th_)
     f = dict(dtype=torch.float32, device=dev)
     out = dict(raster=torch.empty((views, h, w, 4), **f), deriv=torch.empty((views, h, w, 4), **f),
                interp=torch.empty((views, h, w, attrs.shape[1]), **f) if attrs is not None else None,
@@ -251,55 +239,31 @@ def _render_forward(r: Rasterizer, clip, idx, h, w, attrs, uv_attrs, tex, vps, c
                sampled=torch.empty((views, h, w, 4), **f) if tex is not None else None,
                # texel differences of each covered pixel's sample, kept for the backward (32 B per pixel)
                sdiff=torch.empty((views, h, w, 8), **f) if tex is not None else None)
-    offsets = torch.empty(views * tiles + 1, dtype=torch.int32, device=dev)
-    _apply_status(r, ctx.poll_status(kinds=("render_forward", "render_backward")))
-    capacity = max(getattr(r, "_render_capacity", 0), 2 * T * views + 1024)
+    _apply_status(ctx.poll_status(kinds=("render_backward",)))
     L = _native.lib()
-    for _ in range(1 if deferred else 3):
-        lst = torch.empty(capacity, dtype=torch.int32, device=dev)
-        ws_bytes = L.pdr_render_workspace_bytes_tiled(views, T, w, h, capacity, tw_, th_)
-        ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-        ctx.status.zero_()
-        a = RenderArgsC()
-        a.clip_positions, a.views, a.vertex_count = clip.data_ptr(), views, V
-        a.indices, a.triangle_count, a.width, a.height = idx.data_ptr(), T, w, h
-        a.viewports, a.cull_mode = vps.data_ptr(), cull
-        if attrs is not None:
-            a.attributes, a.attribute_count, a.interpolated = attrs.data_ptr(), attrs.shape[1], out["interp"].data_ptr()
-        if uv_attrs is not None:
-            a.uv_attributes, a.uv = uv_attrs.data_ptr(), out["uv"].data_ptr()
-        if tex is not None:
-            a.texture, a.texture_width, a.texture_height = tex.data_ptr(), tex.shape[1], tex.shape[0]
-            a.address_mode, a.sampled = mode, out["sampled"].data_ptr()
-            a.sample_differences = out["sdiff"].data_ptr()
-        a.tile_offsets, a.tile_triangles, a.capacity = offsets.data_ptr(), lst.data_ptr(), capacity
-        a.workspace, a.workspace_bytes, a.status = ws.data_ptr(), ws_bytes, ctx.status.data_ptr()
-        a.raster, a.barycentric_derivatives = out["raster"].data_ptr(), out["deriv"].data_ptr()
-        a.tile_width, a.tile_height, a.stage_triangles = tw_, th_, stage
-        _native.check(L.pdr_render_forward(C.addressof(a), ctx.stream()))
-        if deferred:
-            # No wait: a tile whose list overflowed the capacity is rasterized from all triangles with the
-            # binning rule (same result, slower); the entry count reaches the host later and sizes the
-            # capacity of the next calls.
-            ctx.defer_status("render_forward")
-            return out
-        st = ctx.status.cpu()
-        total = int(st[_native.STATUS_TILE_ENTRIES]) & 0xFFFFFFFF
-        if int(st[_native.STATUS_TILE_ENTRIES_HI]) != 0:
-            raise OverflowError("Tile triangle list exceeds backend limits")
-        if not int(st[_native.STATUS_TILE_OVERFLOW]):
-            r._render_capacity = max(getattr(r, "_render_capacity", 0), total + total // 8 + 1024)
-            return out
-        capacity = total + total // 8 + 1024
-    raise RuntimeError("tile binning did not converge")
+    ws = torch.empty(L.pdr_render_direct_workspace_bytes(views, T, w, h), dtype=torch.uint8, device=dev)
+    a = RenderArgsC()
+    a.clip_positions, a.views, a.vertex_count = clip.data_ptr(), views, V
+    a.indices, a.triangle_count, a.width, a.height = idx.data_ptr(), T, w, h
+    a.viewports, a.cull_mode = vps.data_ptr(), cull
+    if attrs is not None:
+        a.attributes, a.attribute_count, a.interpolated = attrs.data_ptr(), attrs.shape[1], out["interp"].data_ptr()
+    if uv_attrs is not None:
+        a.uv_attributes, a.uv = uv_attrs.data_ptr(), out["uv"].data_ptr()
+    if tex is not None:
+        a.texture, a.texture_width, a.texture_height = tex.data_ptr(), tex.shape[1], tex.shape[0]
+        a.address_mode, a.sampled = mode, out["sampled"].data_ptr()
+        a.sample_differences = out["sdiff"].data_ptr()
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    a.raster, a.barycentric_derivatives = out["raster"].data_ptr(), out["deriv"].data_ptr()
+    _native.check(L.pdr_render_direct(C.addressof(a), ctx.stream()))
+    return out
 
 
 class _RenderFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, positions, vertex_attributes, vertex_uv, texture_values, indices, resolution, rasterizer,
                 viewport, cull_mode, address_mode, deferred_errors):
-        from .rasterizer import _viewports
-
         r = rasterizer
         deferred = bool(deferred_errors) or torch.cuda.is_current_stream_capturing()
         with r.context.lock:
@@ -312,8 +276,7 @@ class _RenderFunction(torch.autograd.Function):
             attrs = vertex_attributes.detach().contiguous() if vertex_attributes is not None else None
             uva = vertex_uv.detach().contiguous() if vertex_uv is not None else None
             tex = texture_values.detach().contiguous() if texture_values is not None else None
-            out = _render_forward(r, clip, idx, h, w, attrs, uva, tex, vps, _MODES[cull_mode], _ADDRESS[address_mode],
-                                  deferred)
+            out = _render_forward(r, clip, idx, h, w, attrs, uva, tex, vps, _MODES[cull_mode], _ADDRESS[address_mode])
         ctx.r, ctx.vps, ctx.batched, ctx.viewport = r, vps, batched, viewport
         ctx.deferred = deferred
         ctx.mode = _ADDRESS[address_mode]
@@ -372,7 +335,7 @@ class _RenderFunction(torch.autograd.Function):
             ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws_bytes
             deferred = ctx.deferred or torch.cuda.is_current_stream_capturing()
-            _apply_status(r, r.context.poll_status(kinds=("render_forward", "render_backward")))
+            _apply_status(r.context.poll_status(kinds=("render_backward",)))
             r.context.status.zero_()
             _native.check(_native.lib().pdr_render_backward(C.addressof(a), r.context.stream()))
             if deferred:
@@ -405,12 +368,11 @@ def render(positions: torch.Tensor, indices: torch.Tensor, resolution: Sequence[
     bit-identical to them, with the same gradients. vertex_attributes [V, A] (A <= 8) and vertex_uv [V, 2]
     are shared by all views; the texture is [H, W, 4] and needs vertex_uv.
 
-    By default each forward and backward waits for its kernels to check the device status (tile-list
-    capacity, non-finite or out-of-range uv) and raises at once, as the separate calls do. With
+    By default the backward waits for its kernels to check the device status (non-finite or out-of-range
+    uv) and raises at once, as the separate calls do; the forward has nothing to wait for. With
     deferred_errors=True (and always inside a CUDA graph capture) neither waits: the host can run ahead
-    of the GPU and the pass can be captured. A tile-list overflow then costs time, not correctness (the
-    tiles concerned rasterize from all triangles with the binning rule), and errors the device records
-    are raised by a later call on the same rasterizer, or by check_deferred_errors(rasterizer)."""
+    of the GPU and the pass can be captured. Errors the device records are then raised by a later call on
+    the same rasterizer, or by check_deferred_errors(rasterizer)."""
     if positions.dtype != torch.float32 or positions.ndim not in (2, 3) or positions.shape[-1] != 4:
         raise ValueError("positions must be a float32 tensor with shape [vertex_count, 4]")
     if indices.ndim != 2 or indices.shape[1] != 3:
