@@ -372,6 +372,10 @@ PDR_API pdr_status pdr_render_backward(const pdr_render_args* args, void* stream
 /* Workspace bytes for pdr_render_backward's per-view vertex-gradient records:
  * views * vertex_count * 4 * ceil((attribute_count + 5) / 4) * sizeof(float); 0 for attribute_count > 8. */
 PDR_API size_t pdr_render_backward_workspace_bytes(uint32_t views, uint32_t vertex_count, uint32_t attribute_count);
+/* With this many workspace bytes pdr_render_backward may also sort the pixel tiles of all views by the part of
+ * the texture they sample (many views of a texture larger than L2). Only the summation order changes. */
+PDR_API size_t pdr_render_backward_ordered_workspace_bytes(uint32_t views, uint32_t vertex_count,
+                                                           uint32_t attribute_count, uint32_t width, uint32_t height);
 
 
 /* ---- calibration --------------------------------------------------------------------------------
@@ -531,6 +535,13 @@ PDR_API pdr_status pdr_render_batch_forward(const pdr_render_mesh* meshes, uint3
                                             const pdr_batch_config* config, uint32_t* tile_offsets,
                                             uint32_t* tile_triangles, uint64_t capacity, void* workspace,
                                             size_t workspace_bytes, uint32_t* status, void* stream);
+/* The images of pdr_render_batch_forward, bit for bit, through a visibility buffer instead of tile lists: nothing
+ * can overflow. The workspace is pdr_render_batch_direct_workspace_bytes() bytes, 16-byte aligned. */
+PDR_API pdr_status pdr_render_batch_direct_workspace_bytes(const pdr_render_mesh* meshes, uint32_t mesh_count,
+                                                           uint32_t attribute_count, size_t* workspace_bytes);
+PDR_API pdr_status pdr_render_batch_direct(const pdr_render_mesh* meshes, uint32_t mesh_count, uint32_t attribute_count,
+                                           uint32_t cull_mode, uint32_t address_mode, void* workspace,
+                                           size_t workspace_bytes, void* stream);
 /* The adjoints of the forward for every mesh (gradient outputs are overwritten). */
 PDR_API pdr_status pdr_render_batch_backward(const pdr_render_mesh* meshes, uint32_t mesh_count,
                                              uint32_t attribute_count, uint32_t address_mode,

@@ -1,9 +1,8 @@
 """Uneven multi-mesh batches in one launch (no counterpart in the reference, which renders one mesh per
-call): many meshes, each with its own views, resolution and texture, run through one binning pass, one
-raster launch with the shading epilogue and one adjoint launch (include/pdr_capi.h
-pdr_render_batch_*). The forward tile shape and the triangles staged per pass (the bin depth) come
-from `MeshBatch.autotune`, which times every compiled configuration on the batch itself; outputs are
-bit-identical for every configuration.
+call): many meshes, each with its own views, resolution and texture, run through one visibility pass, one
+shading launch and one adjoint launch (include/pdr_capi.h pdr_render_batch_direct, pdr_render_batch_backward).
+The tile configurations are those of pdr_render_batch_forward, the tile-list forward with the same outputs;
+nothing of the passes here depends on them.
 """
 from __future__ import annotations
 
@@ -88,7 +87,6 @@ class MeshBatch:
                 if name not in m.outputs:
                     m.outputs[name] = torch.empty(shape + (channels,), **f)
         self.status = torch.zeros(_native.STATUS_WORDS, dtype=torch.int32, device=dev)
-        self.capacity = 0
         self.set_config(config)
 
     # -- native structures -------------------------------------------------------------------------------
@@ -119,39 +117,19 @@ class MeshBatch:
         if tuple(config) not in CONFIGS:
             raise ValueError(f"batch configuration must be one of {CONFIGS}")
         self.config = BatchConfigC(*config)
-        segs, ws = C.c_uint64(), C.c_size_t()
+        segs, ws, direct = C.c_uint64(), C.c_size_t(), C.c_size_t()
         _native.call("pdr_render_batch_sizes", self._table(), len(self.meshes), C.byref(self.config), self.A,
                      C.byref(segs), C.byref(ws))
-        dev = self.r.context.device
+        _native.call("pdr_render_batch_direct_workspace_bytes", self._table(), len(self.meshes), self.A, C.byref(direct))
         self.segments = segs.value
-        self.offsets = torch.empty(self.segments + 1, dtype=torch.int32, device=dev)
-        self.workspace = torch.empty(max(ws.value, 1), dtype=torch.uint8, device=dev)
-        total_tris = sum(m.clip.shape[0] * m.indices.shape[0] for m in self.meshes)
-        self._ensure_capacity(max(self.capacity, 2 * total_tris + 1024))
-
-    def _ensure_capacity(self, capacity: int) -> None:
-        if capacity > self.capacity or not hasattr(self, "list"):
-            self.capacity = int(capacity)
-            self.list = torch.empty(self.capacity, dtype=torch.int32, device=self.r.context.device)
+        self.workspace = torch.empty(max(ws.value, direct.value, 1), dtype=torch.uint8, device=self.r.context.device)
 
     # -- passes --------------------------------------------------------------------------------------------
     def forward(self, stream=None) -> None:
-        """Renders every view of every mesh (re-running with a larger tile list when it overflowed)."""
-        ctx = self.r.context
-        s = stream if stream is not None else ctx.stream()
-        for _ in range(3):
-            self.status.zero_()
-            _native.call("pdr_render_batch_forward", self._table(), len(self.meshes), self.A, self.cull, self.mode,
-                         C.byref(self.config), _ptr(self.offsets), _ptr(self.list), self.capacity,
-                         _ptr(self.workspace), self.workspace.numel(), _ptr(self.status), s)
-            st = self.status.cpu()
-            if int(st[_native.STATUS_TILE_ENTRIES_HI]) != 0:
-                raise OverflowError("Tile triangle list exceeds backend limits")
-            if not int(st[_native.STATUS_TILE_OVERFLOW]):
-                return
-            total = int(st[_native.STATUS_TILE_ENTRIES]) & 0xFFFFFFFF
-            self._ensure_capacity(total + total // 8 + 1024)
-        raise RuntimeError("tile binning did not converge")
+        """Renders every view of every mesh."""
+        s = stream if stream is not None else self.r.context.stream()
+        _native.call("pdr_render_batch_direct", self._table(), len(self.meshes), self.A, self.cull, self.mode,
+                     _ptr(self.workspace), self.workspace.numel(), s)
 
     def allocate_gradients(self) -> None:
         for m in self.meshes:

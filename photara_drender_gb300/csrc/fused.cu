@@ -13,99 +13,113 @@
 // per pixel instead of gathering four texels again.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <numeric>
+
 #include "../../include/pdr_capi.h"
 #include "pdr_common.cuh"
 #include "pdr_internal.h"
 #include "render_bwd_tile.cuh"
+#include "tile_order.cuh"
 
 namespace pdr {
 namespace {
 
-// The adjoint runs 16x8 tiles of 128 threads, 12 CTAs per SM (40 registers, a few spills): 2.42 ms on
-// 64 views against 2.50 ms for 16x16 tiles of 256 threads at 6 CTAs per SM.
-constexpr int kBwdTileH = 8;
-constexpr int kBwdThreads = 16 * kBwdTileH;
-
+// Tiles of all views, in `order` or view by view, over CTAs that stay resident: the tiles' chain of dependent
+// loads (order, raster value, triangle, vertices) is what a pixel waits for, so the first three are loaded ahead of
+// their tile.
 template <int kA, int kTexAgg>
-__global__ void __launch_bounds__(kBwdThreads, 12)
+__global__ void __launch_bounds__(kBwdThreads, backward_ctas(kA))
 render_backward_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* __restrict__ idx, uint32_t T,
-                       uint32_t W, uint32_t H, const float4* __restrict__ viewports, uint32_t tcx,
+                       uint32_t W, uint32_t H, const float4* __restrict__ viewports, FastDiv tcx,
                        const float* __restrict__ attrs, const float2* __restrict__ uv_attrs,
                        const float4* __restrict__ tex, uint32_t tw, uint32_t th, uint32_t mode,
                        const float4* __restrict__ raster, const float2* __restrict__ uv,
                        const float* __restrict__ grad_attr_out, const float4* __restrict__ grad_sampled,
                        float* __restrict__ g_clip_all, float* __restrict__ g_attr, float* __restrict__ g_uv,
                        float* __restrict__ g_tex, const float4* __restrict__ sdiff, uint32_t* __restrict__ status,
-                       float* __restrict__ g_vtx_all) {
-    const uint32_t view = blockIdx.y;
-    const uint32_t tile = blockIdx.x;
+                       float* __restrict__ g_vtx_all, FastDiv tiles, uint32_t total,
+                       const uint32_t* __restrict__ order) {
+    __shared__ BackwardShared<kA> shared;
     const size_t P = (size_t)W * H;
+    const uint32_t step = gridDim.x;
+    auto entry_at = [&](uint32_t at) { return at < total ? (order ? __ldg(order + at) : at) : 0xffffffffu; };
+    // this thread's pixel of a tile
+    auto pixel_of = [&](uint32_t entry, uint32_t& view, uint32_t& px, uint32_t& py) {
+        view = tiles.quotient(entry);
+        const uint32_t tile = entry - view * tiles.divisor, ty = tcx.quotient(tile);
+        px = (tile - ty * tcx.divisor) * kTile + (threadIdx.x & 15u);
+        py = ty * (uint32_t)kBwdTileH + (threadIdx.x >> 4);
+    };
+    auto raster_at = [&](uint32_t entry) {
+        if (entry == 0xffffffffu) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint32_t view, px, py;
+        pixel_of(entry, view, px, py);
+        return px < W && py < H ? __ldcs(raster + view * P + (size_t)py * W + px) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    uint32_t at = blockIdx.x;
+    uint32_t entry = entry_at(at), next_entry = entry_at(at + step);
     BackwardView v;
-    v.clip = clip_all + (size_t)view * V;
+    v.clip = clip_all;
     v.V = V;
-    v.idx = idx;
     v.T = T;
     v.W = W;
     v.H = H;
-    v.vp = viewports[view];
     v.attrs = attrs;
     v.uv_attrs = uv_attrs;
     v.tex = tex;
     v.tw = tw;
     v.th = th;
     v.mode = mode;
-    v.raster = raster + view * P;
-    v.uv = uv ? uv + view * P : nullptr;
-    v.grad_attr_out = grad_attr_out ? grad_attr_out + view * P * kA : nullptr;
-    v.grad_sampled = grad_sampled ? grad_sampled + view * P : nullptr;
-    v.g_clip = g_clip_all + (size_t)view * V * 4;
+    v.uv = uv;
+    v.grad_attr_out = grad_attr_out;
+    v.grad_sampled = grad_sampled;
+    v.g_clip = g_clip_all;
     v.g_attr = g_attr;
     v.g_uv = g_uv;
     v.g_tex = g_tex;
-    v.sdiff = sdiff ? sdiff + view * P * 2 : nullptr;
+    v.sdiff = sdiff;
+    v.sdiff32 = sdiff && ((uintptr_t)sdiff & 31u) == 0;
     v.status = status;
-    v.g_vtx = g_vtx_all ? g_vtx_all + (size_t)view * V * vertex_record_floats(kA) : nullptr;
-    render_backward_tile<kA, kTexAgg, kBwdTileH>(v, tile % tcx, tile / tcx);
+    v.g_vtx = g_vtx_all;
+    PixelHead head;
+    head.r = raster_at(entry);
+    head.vi = head_triangle(head.r, idx, T);
+    for (; at < total; at += step) {
+        const float4 next_r = raster_at(next_entry);
+        const uint32_t far_entry = entry_at(at + 2 * step);
+        uint3 next_vi;
+        uint32_t view, px, py;
+        pixel_of(entry, view, px, py);
+        v.first_vertex = (size_t)view * V;
+        v.vp = viewports[view];
+        render_backward_pixel<kA, kTexAgg>(v, px, py, view * P + (size_t)py * W + px, head, shared,
+                                           [&] { next_vi = head_triangle(next_r, idx, T); });
+        entry = next_entry;
+        next_entry = far_entry;
+        head.r = next_r;
+        head.vi = next_vi;
+    }
 }
 
-// The vertex-gradient records of all views into the outputs: each view's clip gradient (x, y, 0, w), and
-// the uv and attribute gradients summed over the views in view order. One thread per vertex; every
-// output element is written, so none needs clearing first.
+// The bin of every tile of all views: the uv at the probed pixels.
+__global__ void __launch_bounds__(kOrderThreads)
+backward_order_kernel(const float4* __restrict__ raster, const float2* __restrict__ uv, uint32_t W, uint32_t H,
+                      FastDiv tcx, FastDiv tiles, uint32_t total, uint32_t mode, TileOrder o) {
+    const size_t P = (size_t)W * H;
+    order_tile(
+        blockIdx.x * kOrderThreads + threadIdx.x, total, tiles, tcx, W, H, mode, o,
+        [&](uint32_t view, size_t pix) { return __ldg(&raster[view * P + pix].w) != 0.0f ? 1u : 0u; },
+        [&](uint32_t view, size_t pix, uint32_t) { return __ldg(uv + view * P + pix); });
+}
+
+// The vertex-gradient records of all views into the outputs, one thread per vertex.
 template <int kA>
 __global__ void __launch_bounds__(256)
 vertex_grad_finish_kernel(const float* __restrict__ rec_all, uint32_t views, uint32_t V, float* __restrict__ g_clip_all,
                           float* __restrict__ g_attr, float* __restrict__ g_uv) {
-    constexpr uint32_t kR = vertex_record_floats(kA);
-    constexpr uint32_t kNV = 2 + kA + 3;
     const uint32_t vtx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (vtx >= V) return;
-    float acc[2 + kA];
-#pragma unroll
-    for (int j = 0; j < 2 + kA; ++j) acc[j] = 0.0f;
-    for (uint32_t view = 0; view < views; ++view) {
-        const float4* rec = reinterpret_cast<const float4*>(rec_all + ((size_t)view * V + vtx) * kR);
-        float r[kR];
-#pragma unroll
-        for (uint32_t c = 0; c < kR / 4; ++c) {
-            const float4 q = __ldcs(rec + c);
-            r[4 * c] = q.x;
-            r[4 * c + 1] = q.y;
-            r[4 * c + 2] = q.z;
-            r[4 * c + 3] = q.w;
-        }
-#pragma unroll
-        for (int j = 0; j < 2 + kA; ++j) acc[j] += r[j];
-        reinterpret_cast<float4*>(g_clip_all)[(size_t)view * V + vtx] =
-            make_float4(r[kNV - 3], r[kNV - 2], 0.0f, r[kNV - 1]);
-    }
-    if (g_uv) {
-        g_uv[(size_t)vtx * 2] = acc[0];
-        g_uv[(size_t)vtx * 2 + 1] = acc[1];
-    }
-    if (g_attr) {
-#pragma unroll
-        for (int a = 0; a < kA; ++a) g_attr[(size_t)vtx * kA + a] = acc[2 + a];
-    }
+    if (vtx < V) sum_vertex_records<kA>(rec_all, views, V, vtx, g_clip_all, g_attr, g_uv);
 }
 
 }  // namespace
@@ -119,6 +133,14 @@ extern "C" {
 size_t pdr_render_backward_workspace_bytes(uint32_t views, uint32_t vertex_count, uint32_t attribute_count) {
     if (attribute_count > 8) return 0;
     return (size_t)views * vertex_count * vertex_record_floats((int)attribute_count) * sizeof(float);
+}
+
+size_t pdr_render_backward_ordered_workspace_bytes(uint32_t views, uint32_t vertex_count, uint32_t attribute_count,
+                                                   uint32_t width, uint32_t height) {
+    if (attribute_count > 8) return 0;
+    const uint64_t tiles = (uint64_t)((width + kOrderTileW - 1) / kOrderTileW) * ((height + kOrderTileH - 1) / kOrderTileH);
+    return align_up(pdr_render_backward_workspace_bytes(views, vertex_count, attribute_count)) +
+           tile_order_bytes(tiles * views);
 }
 
 size_t pdr_render_workspace_bytes(uint32_t views, uint32_t triangle_count, uint32_t width, uint32_t height,
@@ -272,18 +294,38 @@ pdr_status pdr_render_backward(const pdr_render_args* a, void* stream) {
         err = cudaMemsetAsync(a->grad_texture, 0, (size_t)a->texture_width * a->texture_height * 4 * sizeof(float), s);
     if (err != cudaSuccess) return set_cuda_error(err, "render_backward(memset)");
     const uint32_t tcx = (a->width + kTile - 1) / kTile, tcy = (a->height + kBwdTileH - 1) / kBwdTileH;
-    const dim3 grid(tcx * tcy, a->views);
+    const uint32_t tiles = tcx * tcy, total = tiles * a->views;
+    // Resident CTAs walk the tiles a grid apart. In view order a step that shares a factor with the row's tiles would
+    // keep a CTA in the same columns of every view, covered or empty (64 views at 1024 x 1024: 2.01 ms).
+    uint32_t grid = std::min(total, (uint32_t)num_sms() * backward_ctas((int)A));
+    while (grid < total && std::gcd(grid, tcx) != 1) --grid;
+    const FastDiv tcx_div = fast_div(tcx), tiles_div = fast_div(tiles);
+    // room for a tile order behind the records: the adjoint takes the tiles by what they sample of a large texture
+    const uint32_t* order = nullptr;
+    if (g_vtx && a->grad_texture && a->texture && order_pays((uint64_t)a->texture_width * a->texture_height, a->views, (uint64_t)a->width * a->height) &&
+        a->workspace_bytes >= pdr_render_backward_ordered_workspace_bytes(a->views, a->vertex_count, A, a->width, a->height)) {
+        const TileOrder o = tile_order_at(static_cast<char*>(a->workspace) + align_up(rec_bytes), total);
+        err = cudaMemsetAsync(o.counts, 0, kOrderBins * sizeof(uint32_t), s);
+        if (err != cudaSuccess) return set_cuda_error(err, "render_backward(order)");
+        backward_order_kernel<<<(total + kOrderThreads - 1) / kOrderThreads, kOrderThreads, 0, s>>>(
+            reinterpret_cast<const float4*>(a->raster), reinterpret_cast<const float2*>(a->uv), a->width, a->height,
+            tcx_div, tiles_div, total, a->address_mode, o);
+        err = launch_order_tiles(o, total, s);
+        if (err != cudaSuccess) return set_cuda_error(err, "render_backward(order)");
+        order = o.order;
+    }
     // warp-aggregated texture-gradient taps for magnified textures (see red_add_v4_texel)
     const bool magnified = (uint64_t)a->texture_width * a->texture_height < (uint64_t)a->width * a->height;
 #define PDR_RENDER_BWD_AGG(KA, AGG)                                                                                  \
     render_backward_kernel<KA, AGG><<<grid, kBwdThreads, 0, s>>>(                                                 \
         reinterpret_cast<const float4*>(a->clip_positions), a->vertex_count, reinterpret_cast<const uint3*>(a->indices), \
-        a->triangle_count, a->width, a->height, reinterpret_cast<const float4*>(a->viewports), tcx, a->attributes,   \
+        a->triangle_count, a->width, a->height, reinterpret_cast<const float4*>(a->viewports), tcx_div, a->attributes,   \
         reinterpret_cast<const float2*>(a->uv_attributes), reinterpret_cast<const float4*>(a->texture),            \
         a->texture_width, a->texture_height, a->address_mode, reinterpret_cast<const float4*>(a->raster),           \
         reinterpret_cast<const float2*>(a->uv), a->grad_interpolated, reinterpret_cast<const float4*>(a->grad_sampled), \
         a->grad_clip_positions, a->grad_attributes, a->grad_uv_attributes, a->grad_texture,                     \
-        reinterpret_cast<const float4*>(a->texture ? a->sample_differences : nullptr), a->status, g_vtx)
+        reinterpret_cast<const float4*>(a->texture ? a->sample_differences : nullptr), a->status, g_vtx,     \
+        tiles_div, total, order)
 #define PDR_RENDER_BWD(KA)                  \
     if (magnified) {                        \
         PDR_RENDER_BWD_AGG(KA, 1);          \

@@ -90,7 +90,49 @@ PDR_HD float ldexp_exact(float x, int e) {
 constexpr int kTexelNonFinite = 1;
 constexpr int kTexelRange = 2;
 
+// Quotients of 31-bit numerators by a divisor fixed for a launch (T. Granlund and P. Montgomery, "Division by
+// invariant integers using multiplication", 1994): a high product, an addition and a shift.
+struct FastDiv {
+    uint32_t divisor, multiplier, shift;
+#if defined(__CUDACC__)
+    __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return (__umulhi(multiplier, n) + n) >> shift; }
+#endif
+};
+
+inline FastDiv fast_div(uint32_t d) {  // 1 <= d < 2^31
+    uint32_t s = 0;
+    while ((1ull << s) < d) ++s;
+    return {d, (uint32_t)((((1ull << s) - d) << 32) / d + 1), s};
+}
+
+PDR_HD float fma_rn(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+    return __fmaf_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+
 PDR_HD int exact_texel_coordinate(float u, uint32_t size, int32_t* base, float* fraction) {
+    // Coordinates past the first half texel of textures below 2^24 texels a side, in floats: u * size = hi + lo
+    // exactly (lo from a fused multiply-add). hi >= 0.5 is a multiple of 2^-24, so its fraction +- 0.5 is exact
+    // and the last addition is the one rounding. About 15 instructions against 75 below.
+    const float s = (float)size, hi = u * s;
+    if (size < (1u << 24) && hi >= 0.5f && hi < 4194304.0f) {
+        const float lo = fma_rn(u, s, -hi), whole = floorf(hi), f = hi - whole;
+        int32_t b = (int32_t)whole;
+        float n = f - 0.5f;
+        if (f < 0.5f) {
+            n = f + 0.5f;
+            b -= 1;
+        } else if (n == 0.0f && lo < 0.0f) {  // just below a texel centre
+            n = 1.0f;
+            b -= 1;
+        }
+        *base = b;
+        *fraction = n + lo;
+        return 0;
+    }
     uint32_t bits;
 #if defined(__CUDA_ARCH__)
     bits = __float_as_uint(u);

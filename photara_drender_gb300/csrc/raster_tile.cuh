@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include "bin_rect.cuh"
+#include "ndc_axis.cuh"
 #include "pdr_common.cuh"
 #include "pdr_internal.h"
 
@@ -210,34 +211,6 @@ __device__ __forceinline__ uint32_t pack_nibbles(uint32_t v) {
     return (v | (v >> 8)) & 0xFFFFu;
 }
 
-// One axis of a viewport with the reciprocal of its size, for divisions by that size without a division: the
-// quotient a / b by a fixed divisor is q = RN(a y), r = RN(a - q b), RN(q + r y) with y = RN(1 / b), which is
-// correctly rounded (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990, theorem 8.2) unless b's significand is all ones, and while nothing under- or overflows:
-// `exact` and the bounds on a keep both away. Otherwise the division itself.
-struct NdcAxis {
-    float v0, size, rcp;
-    bool exact;
-    __device__ __forceinline__ NdcAxis(float origin, float extent) : v0(origin), size(extent), rcp(1.0f / extent) {
-        exact = extent >= 1e-6f && extent <= 1e9f && fabsf(origin) <= 1e9f &&
-                (__float_as_uint(extent) & 0x7fffffu) != 0x7fffffu;
-    }
-    __device__ __forceinline__ float quotient(float a) const {  // exact, and a zero or of moderate size
-        const float q = a * rcp;
-        return __fmaf_rn(__fmaf_rn(-q, size, a), rcp, q);
-    }
-    // sample_ndc
-    __device__ __forceinline__ float at(uint32_t p) const {
-        if (!exact) return sample_ndc(p, v0, size);
-        return quotient(((float)p - v0 + 0.5f) * 2.0f) - 1.0f;
-    }
-    // a / size
-    __device__ __forceinline__ float divide(float a) const {
-        const float m = fabsf(a);
-        return exact && m >= 1e-25f && m <= 1e25f ? quotient(a) : a / size;
-    }
-};
-
 // The winner's outputs at sample (sx, sy), rasterize_forward.hlsl's arithmetic: clamped barycentrics,
 // 1 / area and clamped depth; and its pixel derivatives [du/dx, du/dy, dv/dx, dv/dy]. Shared with the
 // near-plane remap, which evaluates them for the original triangle of a clipped one.
@@ -309,7 +282,8 @@ __device__ __forceinline__ void shade_pixel(const RasterView& v, uint32_t px, ui
         __stcs(v.raster + pix, zero);
         if (kDeriv) __stcs(v.deriv + pix, zero);
         if (kShade) {
-            for (uint32_t a = 0; a < A; ++a) __stcs(shade.attr_out + pix * A + a, 0.0f);
+            if constexpr (kA != 0)
+                for (uint32_t a = 0; a < A; ++a) __stcs(shade.attr_out + pix * A + a, 0.0f);
             if (shade.uv_out) __stcs(shade.uv_out + pix, make_float2(0.0f, 0.0f));
             if (shade.sampled) __stcs(shade.sampled + pix, zero);
         }
@@ -321,7 +295,7 @@ __device__ __forceinline__ void shade_pixel(const RasterView& v, uint32_t px, ui
     const float4 p0 = v.clip[vi.x], p1 = v.clip[vi.y], p2 = v.clip[vi.z];
     constexpr int kN = kA > 0 ? kA : 1;
     float t0[kN], t1[kN], t2[kN];
-    if (kShade && kA > 0) {
+    if constexpr (kShade && kA > 0) {
 #pragma unroll
         for (int a = 0; a < kA; ++a) {
             t0[a] = __ldg(shade.attrs + (size_t)vi.x * kA + a);
@@ -342,7 +316,7 @@ __device__ __forceinline__ void shade_pixel(const RasterView& v, uint32_t px, ui
     __stcs(v.raster + pix, make_float4(u, vv, wb.depth, (float)best_tri));
     if (kDeriv) __stcs(v.deriv + pix, winner_derivatives(p0, p1, p2, wb, ax, ay));
     if (!kShade) return;
-    if (kA >= 0) {
+    if constexpr (kA >= 0) {
 #pragma unroll
         for (int a = 0; a < kA; ++a) __stcs(shade.attr_out + pix * kA + a, u * t0[a] + vv * t1[a] + w * t2[a]);
     } else {

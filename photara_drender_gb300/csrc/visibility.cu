@@ -23,6 +23,7 @@
 #include "../../include/pdr_capi.h"
 #include "pdr_common.cuh"
 #include "pdr_internal.h"
+#include "tile_order.cuh"
 #include "visibility.cuh"
 
 namespace pdr {
@@ -30,7 +31,7 @@ namespace {
 
 constexpr uint32_t kVisWarps = 4;
 constexpr size_t kKeyBytes = 512u << 20;
-constexpr uint32_t kShadeW = 16, kShadeH = 8;
+constexpr uint32_t kShadeW = kOrderTileW, kShadeH = kOrderTileH;
 
 // warp_triangles triangles per warp: 32, or fewer where 32 would leave the chip idle.
 __global__ void __launch_bounds__(32 * kVisWarps, 10)
@@ -51,8 +52,8 @@ visibility_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* 
     v.keys = keys + (size_t)blockIdx.y * W * H;
     const NdcAxis ax(v.vp.x, v.vp.z), ay(v.vp.y, v.vp.w);
     const uint32_t warp = threadIdx.x >> 5;
-    vis_warp(v, ax, ay, (blockIdx.x * kVisWarps + warp) * warp_triangles, warp_triangles, warps[warp], queue, queue_count,
-             blockIdx.y * T);
+    vis_warp(v, ax, ay, (blockIdx.x * kVisWarps + warp) * warp_triangles, warp_triangles, warps[warp], queue_count,
+             [&](uint32_t slot, uint32_t t) { queue[slot] = blockIdx.y * T + t; });
 }
 
 // Triangles with large candidate rectangles: bands of rows, enough of them to occupy the grid.
@@ -63,7 +64,7 @@ visibility_large_kernel(const float4* __restrict__ clip_all, uint32_t V, const u
                         const uint32_t* __restrict__ queue_count) {
     const uint32_t n = *queue_count;
     if (n == 0) return;
-    const uint32_t bands = min(64u, max(1u, 4u * gridDim.x / n));
+    const uint32_t bands = vis_bands(n);
     const uint64_t items = (uint64_t)n * bands;
     for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
         const uint32_t entry = queue[item / bands], band = (uint32_t)(item % bands);
@@ -78,26 +79,27 @@ visibility_large_kernel(const float4* __restrict__ clip_all, uint32_t V, const u
         v.cull = cull;
         v.vp = viewports[view0 + view];
         v.keys = keys + (size_t)view * W * H;
-        const NdcAxis ax(v.vp.x, v.vp.z), ay(v.vp.y, v.vp.w);
-        VisTriangle t;
-        if (!vis_setup(v, ax, ay, entry - view * T, t)) continue;
-        const uint64_t rows = t.y1 - t.y0 + 1u;
-        vis_rows(v, ax, ay, t, (uint32_t)(rows * band / bands), (uint32_t)(rows * (band + 1u) / bands));
+        vis_band(v, entry - view * T, band, bands);
     }
 }
 
-// The outputs of every pixel of a group of views from its key.
+// The outputs of every pixel of a group of views from its key, a CTA per tile in `order` (tile_order.cuh) or view by
+// view. Images are those of all views; a pixel's index counts from their first element. CTAs that stay resident
+// and load the next tile's keys ahead, which the adjoint gains from, measured slower here (1.39 -> 1.50 ms): the
+// stores bound this kernel.
 template <bool kDeriv, bool kShade, int kA>
 __global__ void __launch_bounds__(kShadeW * kShadeH, kShade ? 12 : 16)
 shade_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* __restrict__ idx, uint32_t T, uint32_t W,
-             uint32_t H, const float4* __restrict__ viewports, uint32_t view0, uint32_t tcx,
+             uint32_t H, const float4* __restrict__ viewports, uint32_t view0, FastDiv tcx,
              const unsigned long long* __restrict__ keys, float4* __restrict__ raster, float4* __restrict__ deriv,
-             ShadeArgs shade) {
-    const uint32_t view = view0 + blockIdx.y;
-    const uint32_t ty = blockIdx.x / tcx, tx = blockIdx.x - ty * tcx;
+             ShadeArgs shade, FastDiv tiles, const uint32_t* __restrict__ order) {
+    const uint32_t entry = order ? __ldg(order + blockIdx.x) : blockIdx.x;
+    const uint32_t group_view = tiles.quotient(entry), tile = entry - group_view * tiles.divisor;
+    const uint32_t ty = tcx.quotient(tile), tx = tile - ty * tcx.divisor;
     const uint32_t px = tx * kShadeW + threadIdx.x % kShadeW, py = ty * kShadeH + threadIdx.x / kShadeW;
     if (px >= W || py >= H) return;
     const size_t P = (size_t)W * H, pix = (size_t)py * W + px;
+    const uint32_t view = view0 + group_view;
     RasterView v;
     v.clip = clip_all + (size_t)view * V;
     v.idx = idx;
@@ -107,17 +109,26 @@ shade_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* __res
     v.H = H;
     v.cull = 0;
     v.vp = viewports[view];
-    v.raster = raster + view * P;
-    v.deriv = kDeriv ? deriv + view * P : nullptr;
+    v.raster = raster;
+    v.deriv = deriv;
     v.shade = shade;
-    if (kShade) {
-        if (shade.attr_out) v.shade.attr_out = shade.attr_out + view * P * shade.A;
-        if (shade.uv_out) v.shade.uv_out = shade.uv_out + view * P;
-        if (shade.sampled) v.shade.sampled = shade.sampled + view * P;
-        if (shade.sdiff) v.shade.sdiff = shade.sdiff + view * P * 2;
-    }
-    const unsigned long long key = __ldcs(keys + blockIdx.y * P + pix);
-    shade_pixel<kDeriv, kShade, kA>(v, px, py, pix, key == ~0ull ? 0u : (uint32_t)key + 1u);
+    const unsigned long long key = __ldcs(keys + group_view * P + pix);
+    shade_pixel<kDeriv, kShade, kA>(v, px, py, view * P + pix, key == ~0ull ? 0u : (uint32_t)key + 1u);
+}
+
+// The bin of every tile of a group of views: the uv of a vertex of the triangle seen at the probed pixels.
+__global__ void __launch_bounds__(kOrderThreads)
+order_bins_kernel(const uint3* __restrict__ idx, uint32_t W, uint32_t H, FastDiv tcx, FastDiv tiles, uint32_t total,
+                  uint32_t mode, const float2* __restrict__ uv_attrs, const unsigned long long* __restrict__ keys,
+                  TileOrder o) {
+    const size_t P = (size_t)W * H;
+    order_tile(
+        blockIdx.x * kOrderThreads + threadIdx.x, total, tiles, tcx, W, H, mode, o,
+        [&](uint32_t view, size_t pix) {
+            const unsigned long long key = __ldg(keys + view * P + pix);
+            return key == ~0ull ? 0u : (uint32_t)key + 1u;
+        },
+        [&](uint32_t, size_t, uint32_t winner) { return __ldg(uv_attrs + idx[winner - 1].x); });
 }
 
 uint32_t group_views(uint32_t views, uint32_t W, uint32_t H) {
@@ -127,21 +138,122 @@ uint32_t group_views(uint32_t views, uint32_t W, uint32_t H) {
 
 }  // namespace
 
+namespace {
+
+struct DirectWorkspace {
+    uint32_t *queue_count, *queue;
+    unsigned long long* keys;
+    void* order;
+    size_t bytes;
+};
+
+DirectWorkspace direct_workspace(void* base, uint32_t group, uint32_t T, uint32_t W, uint32_t H) {
+    char* c = static_cast<char*>(base);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char* r = c ? c + off : nullptr;
+        off += align_up(bytes);
+        return r;
+    };
+    DirectWorkspace w{};
+    const uint64_t tiles = (uint64_t)((W + kShadeW - 1) / kShadeW) * ((H + kShadeH - 1) / kShadeH) * group;
+    w.queue_count = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t)));
+    w.queue = reinterpret_cast<uint32_t*>(take((size_t)group * T * sizeof(uint32_t)));
+    w.keys = reinterpret_cast<unsigned long long*>(take((size_t)group * W * H * sizeof(unsigned long long)));
+    w.order = take(tile_order_bytes(tiles));
+    w.bytes = off;
+    return w;
+}
+
+__global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t* __restrict__ counts) {
+    // exclusive prefix sum of the kOrderBins counts, in place
+    __shared__ uint32_t warp_sums[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    constexpr uint32_t kPer = (kOrderBins + 1023u) / 1024u;
+    uint32_t v[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        const uint32_t i = threadIdx.x * kPer + k;
+        v[k] = i < kOrderBins ? counts[i] : 0u;
+        sum += v[k];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t s = warp_sums[lane];
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= d) s += y;
+        }
+        warp_sums[lane] = s;
+    }
+    __syncthreads();
+    uint32_t at = incl - sum + (warp ? warp_sums[warp - 1] : 0u);
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        const uint32_t i = threadIdx.x * kPer + k;
+        if (i < kOrderBins) counts[i] = at;
+        at += v[k];
+    }
+}
+
+__global__ void __launch_bounds__(kOrderThreads) order_scatter_kernel(TileOrder o, uint32_t total) {
+    __shared__ uint32_t warp_empty[kOrderThreads / 32], block_at;
+    const uint32_t entry = blockIdx.x * kOrderThreads + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const bool live = entry < total;
+    const uint32_t bin = live ? o.bins[entry] : 0x10000u;
+    // tiles without a sample: one atomic per block
+    const bool empty = live && bin == kOrderBins - 1u;
+    const unsigned empties = __ballot_sync(0xffffffffu, empty);
+    if (lane == 0) warp_empty[warp] = __popc(empties);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        for (int w = 0; w < kOrderThreads / 32; ++w) {
+            const uint32_t c = warp_empty[w];
+            warp_empty[w] = n;
+            n += c;
+        }
+        block_at = n ? atomicAdd(o.counts + kOrderBins - 1u, n) : 0u;
+    }
+    __syncthreads();
+    if (empty) o.order[block_at + warp_empty[warp] + __popc(empties & below)] = entry;
+    const unsigned peers = __match_any_sync(0xffffffffu, empty ? 0x10000u : bin);
+    const int leader = __ffs(peers) - 1;
+    uint32_t at = 0;
+    if (live && !empty && (int)lane == leader) at = atomicAdd(o.counts + bin, (uint32_t)__popc(peers));
+    at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & below);
+    if (live && !empty) o.order[at] = entry;
+}
+
+}  // namespace
+
+cudaError_t launch_order_tiles(const TileOrder& o, uint64_t tiles, cudaStream_t stream) {
+    order_scan_kernel<<<1, 1024, 0, stream>>>(o.counts);
+    order_scatter_kernel<<<(unsigned)((tiles + kOrderThreads - 1) / kOrderThreads), kOrderThreads, 0, stream>>>(
+        o, (uint32_t)tiles);
+    return cudaGetLastError();
+}
+
 size_t direct_workspace_bytes(uint32_t views, uint32_t T, uint32_t W, uint32_t H) {
-    const size_t g = group_views(views, W, H);
-    return align_up(sizeof(uint32_t)) + align_up(g * T * sizeof(uint32_t)) +
-           align_up(g * W * H * sizeof(unsigned long long));
+    return direct_workspace(nullptr, group_views(views, W, H), T, W, H).bytes;
 }
 
 cudaError_t launch_raster_direct(const float* clip, uint32_t views, uint32_t V, const uint32_t* idx, uint32_t T,
                                  uint32_t W, uint32_t H, const float* viewports, uint32_t cull, void* workspace,
                                  float* raster, float* deriv, const RasterShade* shade, cudaStream_t stream) {
     const uint32_t group = group_views(views, W, H);
-    char* ws = static_cast<char*>(workspace);
-    uint32_t* queue_count = reinterpret_cast<uint32_t*>(ws);
-    uint32_t* queue = reinterpret_cast<uint32_t*>(ws + align_up(sizeof(uint32_t)));
-    unsigned long long* keys =
-        reinterpret_cast<unsigned long long*>(ws + align_up(sizeof(uint32_t)) + align_up((size_t)group * T * sizeof(uint32_t)));
+    const DirectWorkspace ws = direct_workspace(workspace, group, T, W, H);
+    uint32_t *queue_count = ws.queue_count, *queue = ws.queue;
+    unsigned long long* keys = ws.keys;
     const float4* c4 = reinterpret_cast<const float4*>(clip);
     const uint3* i3 = reinterpret_cast<const uint3*>(idx);
     const float4* v4 = reinterpret_cast<const float4*>(viewports);
@@ -163,9 +275,21 @@ cudaError_t launch_raster_direct(const float* clip, uint32_t views, uint32_t V, 
             c4, V, i3, T, W, H, v4, cull, view0, per_warp, keys, queue, queue_count);
         visibility_large_kernel<<<(unsigned)num_sms() * 4u, 256, 0, stream>>>(c4, V, i3, T, W, H, v4, cull, view0, keys,
                                                                              queue, queue_count);
-        const dim3 grid(tcx * tcy, n);
+        const uint32_t tiles = tcx * tcy, total = tiles * n;
+        const uint32_t* order = nullptr;
+        if (shade && sa.sampled && order_pays((uint64_t)sa.tw * sa.th, n, P)) {
+            const TileOrder o = tile_order_at(ws.order, total);
+            e = cudaMemsetAsync(o.counts, 0, kOrderBins * sizeof(uint32_t), stream);
+            if (e != cudaSuccess) return e;
+            order_bins_kernel<<<(total + kOrderThreads - 1) / kOrderThreads, kOrderThreads, 0, stream>>>(
+                i3, W, H, fast_div(tcx), fast_div(tiles), total, sa.mode, sa.uv_attrs, keys, o);
+            e = launch_order_tiles(o, total, stream);
+            if (e != cudaSuccess) return e;
+            order = o.order;
+        }
 #define PDR_SHADE(D, S, A) \
-    shade_kernel<D, S, A><<<grid, kShadeW * kShadeH, 0, stream>>>(c4, V, i3, T, W, H, v4, view0, tcx, keys, r4, d4, sa)
+    shade_kernel<D, S, A><<<total, kShadeW * kShadeH, 0, stream>>>(c4, V, i3, T, W, H, v4, view0, fast_div(tcx), keys, \
+                                                                   r4, d4, sa, fast_div(tiles), order)
 #define PDR_SHADE_A(A)            \
     case A:                       \
         if (d4)                   \

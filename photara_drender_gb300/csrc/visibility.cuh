@@ -127,10 +127,11 @@ struct VisWarp {
 // Triangles [first, first + count) of a view, count <= 32, one per lane. Their rows are numbered with a prefix
 // sum and taken 32 at a time, one per lane (its span of candidate columns); the rows' candidates are numbered
 // the same way and taken 32 at a time, one per lane. So lanes stay busy whatever the triangles' sizes. A lane
-// finds the owner of its row or candidate from the mask of owners whose last one falls in the batch.
+// finds the owner of its row or candidate from the mask of owners whose last one falls in the batch. Large
+// triangles take a slot of the caller's queue instead: enqueue(slot, triangle).
+template <class Enqueue>
 __device__ __forceinline__ void vis_warp(const VisView& v, const NdcAxis& ax, const NdcAxis& ay, uint32_t first,
-                                         uint32_t count, VisWarp& w, uint32_t* queue, uint32_t* queue_count,
-                                         uint32_t queue_base) {
+                                         uint32_t count, VisWarp& w, uint32_t* queue_count, Enqueue&& enqueue) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     uint32_t rows = 0;
@@ -165,7 +166,7 @@ __device__ __forceinline__ void vis_warp(const VisView& v, const NdcAxis& ax, co
         uint32_t at = 0;
         if (lane == 0) at = atomicAdd(queue_count, (uint32_t)__popc(larges));
         at = __shfl_sync(0xffffffffu, at, 0);
-        if (large) queue[at + __popc(larges & below)] = queue_base + first + lane;
+        if (large) enqueue(at + __popc(larges & below), first + lane);
     }
     uint32_t last_row = rows;  // inclusive prefix sum
 #pragma unroll
@@ -262,6 +263,17 @@ __device__ __forceinline__ void vis_rows(const VisView& v, const NdcAxis& ax, co
                       vis_key(t.p0, t.p1, t.p2, psx, psy, __float_as_uint(t.edge_b.w)));
         }
     }
+}
+
+// Bands of rows per queued triangle: enough items to occupy the grid.
+__device__ __forceinline__ uint32_t vis_bands(uint32_t queued) { return min(64u, max(1u, 4u * gridDim.x / queued)); }
+
+__device__ __forceinline__ void vis_band(const VisView& v, uint32_t triangle, uint32_t band, uint32_t bands) {
+    const NdcAxis ax(v.vp.x, v.vp.z), ay(v.vp.y, v.vp.w);
+    VisTriangle t;
+    if (!vis_setup(v, ax, ay, triangle, t)) return;
+    const uint64_t rows = t.y1 - t.y0 + 1u;
+    vis_rows(v, ax, ay, t, (uint32_t)(rows * band / bands), (uint32_t)(rows * (band + 1u) / bands));
 }
 
 }  // namespace pdr

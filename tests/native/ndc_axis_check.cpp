@@ -1,4 +1,4 @@
-// The raster kernels' division by a viewport size (csrc/raster_tile.cuh NdcAxis::quotient: a product with the
+// The raster kernels' division by a viewport size (csrc/ndc_axis.cuh NdcAxis::quotient: a product with the
 // rounded reciprocal and two fused steps) against the division, bit for bit: every pixel of every integer size up
 // to 2100 and some larger ones, random sizes and origins, and random dividends of moderate size.
 #include <cmath>

@@ -77,3 +77,57 @@ def test_direct_shading_matches_separate_kernels(attributes):
         pairs.append((o.interpolated, r.interpolate_forward(attrs, tidx, raster)))
     for a, b in pairs:
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("address", ["clamp", "wrap"])
+def test_sorted_tiles_match_separate_kernels(address):
+    """Views of a texture above L2's size, sampled densely enough that the shading and the adjoint take their tiles
+    by what they sample: images bit for bit, gradients up to the summation order of the atomics."""
+    rng = np.random.default_rng(3)
+    pos3, idx = S.icosphere(5)
+    mats, _ = S.orbit_cameras(6)
+    dev = torch.device("cuda", 0)
+    t = lambda a: torch.tensor(np.asarray(a, np.float32), device=dev, requires_grad=True)  # noqa: E731
+    inputs = [S.clip_positions(pos3, mats), rng.uniform(size=(len(pos3), 3)), S.spherical_uv(pos3) * 1.4 - 0.2]
+    tidx = torch.tensor(idx.astype(np.int32), device=dev)
+    texture = torch.rand((2900, 2900, 4), device=dev, generator=torch.Generator(dev).manual_seed(1))
+    res = (870, 1013)  # ragged in both directions
+    g_attr, g_tex = torch.randn((6,) + res + (3,), device=dev), torch.randn((6,) + res + (4,), device=dev)
+    r = pdr.Rasterizer()
+    results = []
+    for fused in (True, False):
+        clip, attrs, uv = (t(a) for a in inputs)
+        tex = texture.clone().requires_grad_(True)
+        if fused:
+            raster, _, a, u, s = pdr.render(clip, tidx, res, rasterizer=r, vertex_attributes=attrs, vertex_uv=uv,
+                                            texture=tex, address_mode=address)
+        else:
+            raster, _ = pdr.rasterize(clip, tidx, res, rasterizer=r)
+            a, u = (pdr.interpolate(x, raster, tidx, rasterizer=r) for x in (attrs, uv))
+            s = pdr.texture(tex, u, raster, rasterizer=r, address_mode=address)
+        torch.autograd.backward([a, s], [g_attr, g_tex])
+        results.append(([raster, a, u, s], [clip.grad, attrs.grad, uv.grad, tex.grad]))
+    for x, y in zip(results[0][0], results[1][0]):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+    for x, y in zip(results[0][1], results[1][1]):
+        assert float((x - y).abs().max()) <= 1e-4 * float(y.abs().max()) + 1e-7
+
+
+def test_batch_in_groups_of_jobs():
+    """A batch whose keys exceed one group: views on both sides of the border equal single renders."""
+    from photara_drender_gb300.batch import BatchMesh, MeshBatch
+
+    dev = torch.device("cuda", 0)
+    r = pdr.Rasterizer()
+    meshes = []
+    for sub, views, side in ((2, 3, 70), (3, 66, 1024)):
+        pos3, idx = S.icosphere(sub)
+        mats, _ = S.orbit_cameras(views)
+        meshes.append(BatchMesh(torch.tensor(S.clip_positions(pos3, mats), device=dev),
+                                torch.tensor(idx.astype(np.int32), device=dev), side, side))
+    MeshBatch(r, meshes).forward()
+    for m, views in zip(meshes, ((0, 2), (0, 62, 63, 64, 65))):
+        for k in views:
+            one, d = r.forward(m.clip[k], m.indices, (m.height, m.width))
+            assert torch.equal(m.outputs["raster"][k].view(torch.int32), one.view(torch.int32)), k
+            assert torch.equal(m.outputs["deriv"][k].view(torch.int32), d.view(torch.int32)), k

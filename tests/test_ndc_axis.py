@@ -1,4 +1,4 @@
-"""The raster kernels' division by a viewport size without a division (csrc/raster_tile.cuh NdcAxis) rounds
+"""The raster kernels' division by a viewport size without a division (csrc/ndc_axis.cuh NdcAxis) rounds
 exactly like the division: tests/native/ndc_axis_check.cpp, compiled for the host."""
 import os
 import shutil
