@@ -15,6 +15,8 @@
 #include "pdr_internal.h"
 #include "bin_rect.cuh"
 #include "raster_tile.cuh"
+#include "render_bwd_tile.cuh"
+#include "vertex_sums.cuh"
 
 namespace pdr {
 namespace {
@@ -417,74 +419,75 @@ raster_overflow_kernel(const float4* __restrict__ clip_all, uint32_t V, const ui
 // ---- rasterize backward: shaders/rasterize_backward.hlsl:36-158 -------------------------
 // One thread per pixel. A pixel contributes to triangle t exactly when the reference's
 // per-triangle loop would visit it: raster id == t+1, inside t's clamped pixel bounds
-// (rasterize_backward.hlsl:78-90) and a non-zero (u, v) gradient. Corner sums use atomics.
+// (rasterize_backward.hlsl:78-90) and a non-zero (u, v) gradient.
 // With near-plane clipping (near != 0) a triangle with a vertex at w <= 1e-8, which the reference
 // never visits, owns the pixels the clipped raster gave it and is visited on all of them (its
 // projected bounds do not exist); every other triangle keeps the reference's rule.
-__global__ void raster_backward_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* __restrict__ idx,
+// Corner gradients are summed over the warp's pixels on the same triangle (vertex_sums.cuh), nine atomics per
+// triangle and warp instead of per pixel: 8 views of 200k triangles at 1024 x 1024 0.24 -> 0.14 ms.
+constexpr int kBackTileW = 16, kBackTileH = 8;  // a warp covers two rows of 16 pixels
+constexpr int kBackThreads = kBackTileW * kBackTileH;
+
+__device__ __forceinline__ void add_clip_sums(VertexSums<9>& s, bool valid, uint32_t id, uint3 vi, float* grad_view) {
+    add_vertex_sums(
+        s, valid, id, vi, 3u,
+        [](const VertexSums<9>& q, uint32_t l, uint32_t corner, uint32_t c) { return q.vals[l][corner * 3u + c]; },
+        [&](uint32_t vertex, uint32_t c, float sum) { atomicAdd(grad_view + (size_t)vertex * 4 + (c == 2 ? 3 : c), sum); });
+}
+
+__global__ void __launch_bounds__(kBackThreads)
+raster_backward_kernel(const float4* __restrict__ clip_all, uint32_t V, const uint3* __restrict__ idx,
                                        uint32_t T, uint32_t W, uint32_t H, const float4* __restrict__ viewports,
                                        const float4* __restrict__ raster, const float4* __restrict__ grad_raster,
-                                       float* __restrict__ grad_clip, uint32_t near) {
-    const uint32_t view = blockIdx.y;
-    const size_t P = (size_t)W * H;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    const size_t pix = (size_t)view * P + p;
-    const float rw = raster[pix].w;
-    const uint32_t id = raster_id(rw);
-    if (id == 0 || id > T) return;
-    const float4 g = grad_raster[pix];
-    if (g.x == 0.0f && g.y == 0.0f) return;
-    const uint3 vi = idx[id - 1];
-    if (vi.x >= V || vi.y >= V || vi.z >= V) return;
-    const float4* __restrict__ clip = clip_all + (size_t)view * V;
-    const float4 p0 = clip[vi.x], p1 = clip[vi.y], p2 = clip[vi.z];
-    const bool behind = p0.w <= 1e-8f || p1.w <= 1e-8f || p2.w <= 1e-8f;
-    if (behind && !near) return;
-    const float4 vp = viewports[view];
-    const uint32_t x = (uint32_t)(p % W), y = (uint32_t)(p / W);
-    if (!behind) {
-        const float s0x = p0.x / p0.w, s0y = p0.y / p0.w;
-        const float s1x = p1.x / p1.w, s1y = p1.y / p1.w;
-        const float s2x = p2.x / p2.w, s2y = p2.y / p2.w;
-        const float mnx = fminf(s0x, fminf(s1x, s2x)), mny = fminf(s0y, fminf(s1y, s2y));
-        const float mxx = fmaxf(s0x, fmaxf(s1x, s2x)), mxy = fmaxf(s0y, fmaxf(s1y, s2y));
-        const int32_t x0 = clampi(f2i_sat(floorf((mnx * 0.5f + 0.5f) * vp.z + vp.x)), 0, (int32_t)W);
-        const int32_t x1 = clampi(f2i_sat(ceilf((mxx * 0.5f + 0.5f) * vp.z + vp.x)), 0, (int32_t)W);
-        const int32_t y0 = clampi(f2i_sat(floorf((mny * 0.5f + 0.5f) * vp.w + vp.y)), 0, (int32_t)H);
-        const int32_t y1 = clampi(f2i_sat(ceilf((mxy * 0.5f + 0.5f) * vp.w + vp.y)), 0, (int32_t)H);
-        if ((int32_t)x < x0 || (int32_t)x >= x1 || (int32_t)y < y0 || (int32_t)y >= y1) return;
+                                       float* __restrict__ grad_clip, uint32_t near, FastDiv tcx) {
+    __shared__ VertexSums<9> sums[kBackThreads / 32];
+    VertexSums<9>& s = sums[threadIdx.x >> 5];
+    const uint32_t view = blockIdx.y, lane = threadIdx.x & 31u;
+    const uint32_t ty = tcx.quotient(blockIdx.x), tx = blockIdx.x - ty * tcx.divisor;
+    const uint32_t x = tx * kBackTileW + threadIdx.x % kBackTileW, y = ty * kBackTileH + threadIdx.x / kBackTileW;
+    const bool in_image = x < W && y < H;
+    const size_t pix = (size_t)view * W * H + (size_t)y * W + x;
+    const uint32_t id = in_image ? raster_id(raster[pix].w) : 0u;
+    bool valid = id != 0 && id <= T;
+    uint3 vi = make_uint3(0u, 0u, 0u);
+    float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
+        g = grad_raster[pix];
+        vi = idx[id - 1];
+        valid = !(g.x == 0.0f && g.y == 0.0f) && vi.x < V && vi.y < V && vi.z < V;
     }
-    const float sx = sample_ndc(x, vp.x, vp.z);
-    const float sy = sample_ndc(y, vp.y, vp.w);
-    const float q0x = p0.x - sx * p0.w, q0y = p0.y - sy * p0.w;
-    const float q1x = p1.x - sx * p1.w, q1y = p1.y - sy * p1.w;
-    const float q2x = p2.x - sx * p2.w, q2y = p2.y - sy * p2.w;
-    const float area = cross2(q1x, q1y, q2x, q2y) + cross2(q2x, q2y, q0x, q0y) + cross2(q0x, q0y, q1x, q1y);
-    if (fabsf(area) <= 1e-12f) return;
-    const float eps = area >= 0.0f ? 1e-6f : -1e-6f;
-    const float inv = 1.0f / (area + eps);
-    const float a0 = cross2(q1x, q1y, q2x, q2y);
-    const float a1 = cross2(q2x, q2y, q0x, q0y);
-    const float b0 = a0 * inv, b1 = a1 * inv;
-    const float gb0 = g.x * inv, gb1 = g.y * inv;
-    const float gc = gb0 * b0 + gb1 * b1;
-    const float g0x = gc * (q2y - q1y) - gb1 * q2y;
-    const float g1x = gc * (q0y - q2y) + gb0 * q2y;
-    const float g2x = gc * (q1y - q0y) - gb0 * q1y + gb1 * q0y;
-    const float g0y = gc * (q1x - q2x) + gb1 * q2x;
-    const float g1y = gc * (q2x - q0x) - gb0 * q2x;
-    const float g2y = gc * (q0x - q1x) + gb0 * q1x - gb1 * q0x;
-    float* gv = grad_clip + (size_t)view * V * 4;
-    atomicAdd(gv + (size_t)vi.x * 4 + 0, g0x);
-    atomicAdd(gv + (size_t)vi.x * 4 + 1, g0y);
-    atomicAdd(gv + (size_t)vi.x * 4 + 3, -sx * g0x - sy * g0y);
-    atomicAdd(gv + (size_t)vi.y * 4 + 0, g1x);
-    atomicAdd(gv + (size_t)vi.y * 4 + 1, g1y);
-    atomicAdd(gv + (size_t)vi.y * 4 + 3, -sx * g1x - sy * g1y);
-    atomicAdd(gv + (size_t)vi.z * 4 + 0, g2x);
-    atomicAdd(gv + (size_t)vi.z * 4 + 1, g2y);
-    atomicAdd(gv + (size_t)vi.z * 4 + 3, -sx * g2x - sy * g2y);
+    if (valid) {
+        const float4* __restrict__ clip = clip_all + (size_t)view * V;
+        const float4 p0 = clip[vi.x], p1 = clip[vi.y], p2 = clip[vi.z];
+        const float4 vp = viewports[view];
+        const bool behind = p0.w <= 1e-8f || p1.w <= 1e-8f || p2.w <= 1e-8f;
+        valid = behind ? near != 0 : visited(p0, p1, p2, vp, x, y, W, H);
+        const NdcAxis ax(vp.x, vp.z, __frcp_rn(vp.z)), ay(vp.y, vp.w, __frcp_rn(vp.w));
+        const float sx = ax.at(x), sy = ay.at(y);
+        const float q0x = p0.x - sx * p0.w, q0y = p0.y - sy * p0.w;
+        const float q1x = p1.x - sx * p1.w, q1y = p1.y - sy * p1.w;
+        const float q2x = p2.x - sx * p2.w, q2y = p2.y - sy * p2.w;
+        const float a0 = cross2(q1x, q1y, q2x, q2y);
+        const float a1 = cross2(q2x, q2y, q0x, q0y);
+        const float area = a0 + a1 + cross2(q0x, q0y, q1x, q1y);
+        if (fabsf(area) <= 1e-12f) valid = false;
+        const float eps = area >= 0.0f ? 1e-6f : -1e-6f;
+        const float inv = 1.0f / (area + eps);
+        const float b0 = a0 * inv, b1 = a1 * inv;
+        const float gb0 = g.x * inv, gb1 = g.y * inv;
+        const float gc = gb0 * b0 + gb1 * b1;
+        const float g0x = gc * (q2y - q1y) - gb1 * q2y;
+        const float g1x = gc * (q0y - q2y) + gb0 * q2y;
+        const float g2x = gc * (q1y - q0y) - gb0 * q1y + gb1 * q0y;
+        const float g0y = gc * (q1x - q2x) + gb1 * q2x;
+        const float g1y = gc * (q2x - q0x) - gb0 * q2x;
+        const float g2y = gc * (q0x - q1x) + gb0 * q1x - gb1 * q0x;
+        const float out[9] = {g0x, g0y, -sx * g0x - sy * g0y, g1x, g1y, -sx * g1x - sy * g1y,
+                              g2x, g2y, -sx * g2x - sy * g2y};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) s.vals[lane][k] = out[k];
+    }
+    add_clip_sums(s, valid, id, vi, grad_clip + (size_t)view * V * 4);
 }
 
 }  // namespace
@@ -629,25 +632,15 @@ cudaError_t launch_raster_forward(const float* clip, uint32_t views, uint32_t V,
 // with a_i = cross(q_j, q_k) of the sample-relative positions q = p.xy - s p.w, A = a0 + a1 + a2,
 // b_i = clamp(a_i / A, 0, 1) (no gradient through a clamped b_i) and da_i/dx, da_i/dy the products of
 // clip coordinates. Added to grad_clip (x, y, w; z has no influence) after the barycentric adjoint.
-__global__ void raster_deriv_backward_kernel(const float4* __restrict__ clip_all, uint32_t V,
-                                             const uint3* __restrict__ idx, uint32_t T, uint32_t W, uint32_t H,
-                                             const float4* __restrict__ viewports, const float4* __restrict__ raster,
-                                             const float4* __restrict__ grad_deriv, float* __restrict__ grad_clip) {
-    const uint32_t view = blockIdx.y;
-    const size_t P = (size_t)W * H;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    const size_t pix = (size_t)view * P + p;
-    const uint32_t id = raster_id(raster[pix].w);
-    if (id == 0 || id > T) return;
-    const float4 g = grad_deriv[pix];
-    if (g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f) return;
-    const uint3 vi = idx[id - 1];
-    if (vi.x >= V || vi.y >= V || vi.z >= V) return;
-    const float4* __restrict__ clip = clip_all + (size_t)view * V;
+__device__ __forceinline__ bool deriv_adjoint(const float4* __restrict__ clip, uint32_t V, const uint3* __restrict__ idx,
+                                              uint32_t T, float4 vp, uint32_t x, uint32_t y, uint32_t id,
+                                              const float4* grad, uint3& vi, float* out) {
+    if (id == 0 || id > T) return false;
+    const float4 g = *grad;
+    if (g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f) return false;
+    vi = idx[id - 1];
+    if (vi.x >= V || vi.y >= V || vi.z >= V) return false;
     const float4 p0 = clip[vi.x], p1 = clip[vi.y], p2 = clip[vi.z];
-    const float4 vp = viewports[view];
-    const uint32_t x = (uint32_t)(p % W), y = (uint32_t)(p / W);
     const float sx = sample_ndc(x, vp.x, vp.z);
     const float sy = sample_ndc(y, vp.y, vp.w);
     // forward quantities
@@ -658,7 +651,7 @@ __global__ void raster_deriv_backward_kernel(const float4* __restrict__ clip_all
     const float a1 = cross2(q2x, q2y, q0x, q0y);
     const float a2 = cross2(q0x, q0y, q1x, q1y);
     const float ha = a0 + a1 + a2;
-    if (fabsf(ha) <= 1e-12f) return;
+    if (fabsf(ha) <= 1e-12f) return false;
     const float binv = 1.0f / ha;
     const float r0 = a0 * binv, r1 = a1 * binv;
     const float b0 = clamp_hlsl(r0, 0.0f, 1.0f), b1 = clamp_hlsl(r1, 0.0f, 1.0f);
@@ -702,15 +695,38 @@ __global__ void raster_deriv_backward_kernel(const float4* __restrict__ clip_all
     // d2x = -p0.w p1.y + p0.y p1.w ; d2y = -p0.x p1.w + p0.w p1.x
     g0[2] += -G2x * p1.y + G2y * p1.x; g1[1] += -G2x * p0.w; g0[1] += G2x * p1.w; g1[2] += G2x * p0.y - G2y * p0.x;
     g0[0] += -G2y * p1.w; g1[0] += G2y * p0.w;
-    float* gv = grad_clip + (size_t)view * V * 4;
-    const uint32_t vs[3] = {vi.x, vi.y, vi.z};
-    const float* gs[3] = {g0, g1, g2};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        atomicAdd(gv + (size_t)vs[k] * 4 + 0, gs[k][0]);
-        atomicAdd(gv + (size_t)vs[k] * 4 + 1, gs[k][1]);
-        atomicAdd(gv + (size_t)vs[k] * 4 + 3, gs[k][2]);
+        out[k] = g0[k];
+        out[3 + k] = g1[k];
+        out[6 + k] = g2[k];
     }
+    return true;
+}
+
+__global__ void __launch_bounds__(kBackThreads)
+raster_deriv_backward_kernel(const float4* __restrict__ clip_all, uint32_t V,
+                                             const uint3* __restrict__ idx, uint32_t T, uint32_t W, uint32_t H,
+                                             const float4* __restrict__ viewports, const float4* __restrict__ raster,
+                                             const float4* __restrict__ grad_deriv, float* __restrict__ grad_clip,
+                                             FastDiv tcx) {
+    __shared__ VertexSums<9> sums[kBackThreads / 32];
+    const uint32_t view = blockIdx.y;
+    const uint32_t ty = tcx.quotient(blockIdx.x), tx = blockIdx.x - ty * tcx.divisor;
+    const uint32_t x = tx * kBackTileW + threadIdx.x % kBackTileW, y = ty * kBackTileH + threadIdx.x / kBackTileW;
+    const bool in_image = x < W && y < H;
+    const size_t pix = (size_t)view * W * H + (size_t)y * W + x;
+    const uint32_t id = in_image ? raster_id(raster[pix].w) : 0u;
+    uint3 vi = make_uint3(0u, 0u, 0u);
+    float out[9];
+    const bool valid = deriv_adjoint(clip_all + (size_t)view * V, V, idx, T, viewports[view], x, y, id,
+                                     in_image ? grad_deriv + pix : nullptr, vi, out);
+    VertexSums<9>& s = sums[threadIdx.x >> 5];
+    if (valid) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) s.vals[threadIdx.x & 31u][k] = out[k];
+    }
+    add_clip_sums(s, valid, id, vi, grad_clip + (size_t)view * V * 4);
 }
 
 cudaError_t launch_raster_backward(const float* clip, uint32_t views, uint32_t V, const uint32_t* idx, uint32_t T,
@@ -719,18 +735,18 @@ cudaError_t launch_raster_backward(const float* clip, uint32_t views, uint32_t V
                                    const float* grad_derivatives, bool near) {
     cudaError_t err = cudaMemsetAsync(grad_clip, 0, (size_t)views * V * 4 * sizeof(float), stream);
     if (err != cudaSuccess) return err;
-    const size_t P = (size_t)W * H;
-    const dim3 grid((uint32_t)((P + 255) / 256), views);
+    const uint32_t tcx = (W + kBackTileW - 1) / kBackTileW;
+    const dim3 grid(tcx * ((H + kBackTileH - 1) / kBackTileH), views);
     if (grad_raster)
-        raster_backward_kernel<<<grid, 256, 0, stream>>>(
-        reinterpret_cast<const float4*>(clip), V, reinterpret_cast<const uint3*>(idx), T, W, H,
-        reinterpret_cast<const float4*>(viewports), reinterpret_cast<const float4*>(raster),
-        reinterpret_cast<const float4*>(grad_raster), grad_clip, near ? 1u : 0u);
-    if (grad_derivatives)
-        raster_deriv_backward_kernel<<<grid, 256, 0, stream>>>(
+        raster_backward_kernel<<<grid, kBackThreads, 0, stream>>>(
             reinterpret_cast<const float4*>(clip), V, reinterpret_cast<const uint3*>(idx), T, W, H,
             reinterpret_cast<const float4*>(viewports), reinterpret_cast<const float4*>(raster),
-            reinterpret_cast<const float4*>(grad_derivatives), grad_clip);
+            reinterpret_cast<const float4*>(grad_raster), grad_clip, near ? 1u : 0u, fast_div(tcx));
+    if (grad_derivatives)
+        raster_deriv_backward_kernel<<<grid, kBackThreads, 0, stream>>>(
+            reinterpret_cast<const float4*>(clip), V, reinterpret_cast<const uint3*>(idx), T, W, H,
+            reinterpret_cast<const float4*>(viewports), reinterpret_cast<const float4*>(raster),
+            reinterpret_cast<const float4*>(grad_derivatives), grad_clip, fast_div(tcx));
     return cudaGetLastError();
 }
 

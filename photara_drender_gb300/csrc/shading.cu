@@ -11,16 +11,21 @@
 
 #include "pdr_common.cuh"
 #include "pdr_internal.h"
+#include "vertex_sums.cuh"
 
 namespace pdr {
 namespace {
 
-__global__ void interpolate_forward_kernel(const float* __restrict__ attr_all, size_t attr_stride, uint32_t V,
-                                           uint32_t A, const uint3* __restrict__ idx, uint32_t T,
-                                           const float4* __restrict__ raster, size_t P, float* __restrict__ out) {
+// kA attributes, their gathers in flight together; 0: any number, one after the other.
+template <int kA>
+__global__ void __launch_bounds__(256)
+interpolate_forward_kernel(const float* __restrict__ attr_all, size_t attr_stride, uint32_t V, uint32_t count,
+                           const uint3* __restrict__ idx, uint32_t T, const float4* __restrict__ raster, size_t P,
+                           float* __restrict__ out) {
     const uint32_t view = blockIdx.y;
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
+    const uint32_t A = kA > 0 ? (uint32_t)kA : count;
     const size_t pix = (size_t)view * P + p;
     const float4 r = raster[pix];
     const uint32_t id = raster_id(r.w);
@@ -32,70 +37,99 @@ __global__ void interpolate_forward_kernel(const float* __restrict__ attr_all, s
         ok = vi.x < V && vi.y < V && vi.z < V;
     }
     if (!ok) {
+#pragma unroll
         for (uint32_t a = 0; a < A; ++a) o[a] = 0.0f;
         return;
     }
     const float* attr = attr_all + (size_t)view * attr_stride;
     const float u = r.x, v = r.y, w = 1.0f - u - v;
+#pragma unroll
     for (uint32_t a = 0; a < A; ++a) {
-        const float a0 = attr[(size_t)vi.x * A + a], a1 = attr[(size_t)vi.y * A + a], a2 = attr[(size_t)vi.z * A + a];
+        const float a0 = __ldg(attr + (size_t)vi.x * A + a), a1 = __ldg(attr + (size_t)vi.y * A + a);
+        const float a2 = __ldg(attr + (size_t)vi.z * A + a);
         o[a] = u * a0 + v * a1 + w * a2;
     }
 }
 
 // grad_raster follows interpolate_grad_raster.hlsl; grad_attr receives weight * grad per distinct
 // vertex of the pixel's triangle, the weight accumulated as interpolate_grad_attributes.hlsl:42-54.
-__global__ void interpolate_backward_kernel(const float* __restrict__ attr_all, size_t attr_stride, uint32_t V,
-                                            uint32_t A, const uint3* __restrict__ idx, uint32_t T,
-                                            const float4* __restrict__ raster, size_t P,
-                                            const float* __restrict__ grad_out, float* __restrict__ grad_attr_all,
-                                            float4* __restrict__ grad_raster, bool accumulate) {
-    const uint32_t view = blockIdx.y;
+// kA attributes, or (0) any number in chunks of kAttrChunk. The vertex gradients are summed over the warp's pixels
+// on the same triangle first (vertex_sums.cuh): with an atomic per pixel, corner and attribute the atomics bound it,
+// 5 and 2 attributes of 8 views of 200k triangles at 1024 x 1024 took 0.57 ms, now 0.15 and 0.10 (latency of the
+// raster value, triangle and attribute loads).
+constexpr int kAttrChunk = 8;
+
+template <int kA>
+__global__ void __launch_bounds__(256)
+interpolate_backward_kernel(const float* __restrict__ attr_all, size_t attr_stride, uint32_t V, uint32_t count,
+                            const uint3* __restrict__ idx, uint32_t T, const float4* __restrict__ raster, size_t P,
+                            const float* __restrict__ grad_out, float* __restrict__ grad_attr_all,
+                            float4* __restrict__ grad_raster, bool accumulate) {
+    constexpr int kC = kA > 0 ? kA : kAttrChunk;
+    __shared__ VertexSums<kC + 3> sums[8];  // per pixel: the corners' weights, then the chunk's gradients
+    const uint32_t view = blockIdx.y, lane = threadIdx.x & 31u;
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
+    const uint32_t A = kA > 0 ? (uint32_t)kA : count;
     const size_t pix = (size_t)view * P + p;
-    const float4 r = raster[pix];
+    const float4 r = p < P ? raster[pix] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const uint32_t id = raster_id(r.w);
-    if (id == 0 || id > T) {
-        if (grad_raster && !accumulate) grad_raster[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return;
-    }
-    const uint3 vi = idx[id - 1];
+    const bool valid = id != 0 && id <= T;
+    const uint3 vi = valid ? idx[id - 1] : make_uint3(0u, 0u, 0u);
     const float* g = grad_out + pix * A;
-    const float u = r.x, v = r.y;
-    if (grad_attr_all) {
-        float* grad_attr = grad_attr_all + (size_t)view * attr_stride;
+    const float* attr = attr_all + (size_t)view * attr_stride;
+    const bool inside = valid && vi.x < V && vi.y < V && vi.z < V;
+    VertexSums<kC + 3>& s = sums[threadIdx.x >> 5];
+    if (valid && grad_attr_all) {
         const uint32_t vs[3] = {vi.x, vi.y, vi.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const uint32_t vx = vs[k];
             bool first = true;
+#pragma unroll
             for (int j = 0; j < k; ++j) first = first && vs[j] != vx;
-            if (!first || vx >= V) continue;
             float wgt = 0.0f;
-            if (vi.x == vx) wgt += u;
-            if (vi.y == vx) wgt += v;
-            if (vi.z == vx) wgt += 1.0f - u - v;
-            for (uint32_t a = 0; a < A; ++a) atomicAdd(grad_attr + (size_t)vx * A + a, wgt * g[a]);
+            if (vi.x == vx) wgt += r.x;
+            if (vi.y == vx) wgt += r.y;
+            if (vi.z == vx) wgt += 1.0f - r.x - r.y;
+            s.vals[lane][k] = first ? wgt : 0.0f;
         }
     }
-    if (grad_raster) {
-        float gx = 0.0f, gy = 0.0f;
-        if (vi.x < V && vi.y < V && vi.z < V) {
-            const float* attr = attr_all + (size_t)view * attr_stride;
-            for (uint32_t a = 0; a < A; ++a) {
-                const float a0 = attr[(size_t)vi.x * A + a], a1 = attr[(size_t)vi.y * A + a];
-                const float a2 = attr[(size_t)vi.z * A + a];
-                gx += g[a] * (a0 - a2);
-                gy += g[a] * (a1 - a2);
+    float gx = 0.0f, gy = 0.0f;
+    for (uint32_t a0 = 0; a0 < A; a0 += kC) {
+        const uint32_t n = kA > 0 ? (uint32_t)kA : min((uint32_t)kC, A - a0);
+        if (valid) {
+#pragma unroll
+            for (uint32_t a = 0; a < (uint32_t)kC; ++a) {
+                if (a >= n) break;
+                const float ga = g[a0 + a];
+                if (grad_attr_all) s.vals[lane][3 + a] = ga;
+                if (grad_raster && inside) {
+                    const float x = __ldg(attr + (size_t)vi.x * A + a0 + a), y = __ldg(attr + (size_t)vi.y * A + a0 + a);
+                    const float z = __ldg(attr + (size_t)vi.z * A + a0 + a);
+                    gx += ga * (x - z);
+                    gy += ga * (y - z);
+                }
             }
         }
-        if (accumulate) {
-            const float4 o = grad_raster[pix];
-            grad_raster[pix] = make_float4(o.x + gx, o.y + gy, o.z, o.w);
-        } else {
-            grad_raster[pix] = make_float4(gx, gy, 0.0f, 0.0f);
+        if (grad_attr_all) {
+            float* grad_attr = grad_attr_all + (size_t)view * attr_stride;
+            add_vertex_sums(
+                s, valid, id, vi, n,
+                [](const VertexSums<kC + 3>& q, uint32_t l, uint32_t corner, uint32_t c) {
+                    return q.vals[l][corner] * q.vals[l][3 + c];
+                },
+                [&](uint32_t vertex, uint32_t c, float sum) {
+                    if (vertex < V) atomicAdd(grad_attr + (size_t)vertex * A + a0 + c, sum);
+                });
         }
+    }
+    if (!grad_raster || p >= P) return;
+    if (accumulate) {
+        if (!valid) return;
+        const float4 o = grad_raster[pix];
+        grad_raster[pix] = make_float4(o.x + gx, o.y + gy, o.z, o.w);
+    } else {
+        grad_raster[pix] = make_float4(gx, gy, 0.0f, 0.0f);
     }
 }
 
@@ -218,6 +252,21 @@ __global__ void texture_backward_kernel(const float* __restrict__ tex_all, size_
         const Taps t = taps_fp32(u, tw, th, mode, &fx, &fy);
         const float* tex = tex_all + (size_t)view * tex_stride;
         float gx = 0.0f, gy = 0.0f;
+        if constexpr (kC == 4) {
+            const float4* t4 = reinterpret_cast<const float4*>(tex);
+            const float4 q00 = __ldg(t4 + t.o[0]), q10 = __ldg(t4 + t.o[1]), q01 = __ldg(t4 + t.o[2]), q11 = __ldg(t4 + t.o[3]);
+            const float4 gg = reinterpret_cast<const float4*>(grad)[pix];
+            const float a00[4] = {q00.x, q00.y, q00.z, q00.w}, a10[4] = {q10.x, q10.y, q10.z, q10.w};
+            const float a01[4] = {q01.x, q01.y, q01.z, q01.w}, a11[4] = {q11.x, q11.y, q11.z, q11.w};
+            const float g4[4] = {gg.x, gg.y, gg.z, gg.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float dx = (1.0f - fy) * (a10[c] - a00[c]) + fy * (a11[c] - a01[c]);
+                const float dy = (1.0f - fx) * (a01[c] - a00[c]) + fx * (a11[c] - a10[c]);
+                gx += g4[c] * (dx * (float)tw);
+                gy += g4[c] * (dy * (float)th);
+            }
+        } else
         for (uint32_t c = 0; c < nc; ++c) {
             const float c00 = __ldg(tex + (size_t)t.o[0] * nc + c), c10 = __ldg(tex + (size_t)t.o[1] * nc + c);
             const float c01 = __ldg(tex + (size_t)t.o[2] * nc + c), c11 = __ldg(tex + (size_t)t.o[3] * nc + c);
@@ -236,9 +285,22 @@ cudaError_t launch_interpolate_forward(const float* attr, size_t attr_view_strid
                                        const uint32_t* idx, uint32_t T, const float* raster, uint32_t views,
                                        size_t P, float* out, cudaStream_t stream) {
     const dim3 grid((uint32_t)((P + 255) / 256), views);
-    interpolate_forward_kernel<<<grid, 256, 0, stream>>>(attr, attr_view_stride, V, A,
-                                                         reinterpret_cast<const uint3*>(idx), T,
-                                                         reinterpret_cast<const float4*>(raster), P, out);
+#define PDR_INTERPOLATE(KA)                                                                                        \
+    interpolate_forward_kernel<KA><<<grid, 256, 0, stream>>>(attr, attr_view_stride, V, A,                         \
+                                                             reinterpret_cast<const uint3*>(idx), T,               \
+                                                             reinterpret_cast<const float4*>(raster), P, out)
+    switch (A) {
+        case 1: PDR_INTERPOLATE(1); break;
+        case 2: PDR_INTERPOLATE(2); break;
+        case 3: PDR_INTERPOLATE(3); break;
+        case 4: PDR_INTERPOLATE(4); break;
+        case 5: PDR_INTERPOLATE(5); break;
+        case 6: PDR_INTERPOLATE(6); break;
+        case 7: PDR_INTERPOLATE(7); break;
+        case 8: PDR_INTERPOLATE(8); break;
+        default: PDR_INTERPOLATE(0); break;
+    }
+#undef PDR_INTERPOLATE
     return cudaGetLastError();
 }
 
@@ -252,11 +314,22 @@ cudaError_t launch_interpolate_backward(const float* attr, size_t attr_view_stri
         if (err != cudaSuccess) return err;
     }
     const dim3 grid((uint32_t)((P + 255) / 256), views);
-    interpolate_backward_kernel<<<grid, 256, 0, stream>>>(attr, attr_view_stride, V, A,
-                                                          reinterpret_cast<const uint3*>(idx), T,
-                                                          reinterpret_cast<const float4*>(raster), P, grad_out,
-                                                          grad_attr, reinterpret_cast<float4*>(grad_raster),
-                                                          accumulate_raster);
+#define PDR_INTERPOLATE_BWD(KA)                                                                                      \
+    interpolate_backward_kernel<KA><<<grid, 256, 0, stream>>>(                                                       \
+        attr, attr_view_stride, V, A, reinterpret_cast<const uint3*>(idx), T, reinterpret_cast<const float4*>(raster), \
+        P, grad_out, grad_attr, reinterpret_cast<float4*>(grad_raster), accumulate_raster)
+    switch (A) {
+        case 1: PDR_INTERPOLATE_BWD(1); break;
+        case 2: PDR_INTERPOLATE_BWD(2); break;
+        case 3: PDR_INTERPOLATE_BWD(3); break;
+        case 4: PDR_INTERPOLATE_BWD(4); break;
+        case 5: PDR_INTERPOLATE_BWD(5); break;
+        case 6: PDR_INTERPOLATE_BWD(6); break;
+        case 7: PDR_INTERPOLATE_BWD(7); break;
+        case 8: PDR_INTERPOLATE_BWD(8); break;
+        default: PDR_INTERPOLATE_BWD(0); break;
+    }
+#undef PDR_INTERPOLATE_BWD
     return cudaGetLastError();
 }
 
