@@ -66,6 +66,11 @@ PDR_API pdr_status pdr_device_info(int32_t device, char* name, size_t name_capac
 PDR_API pdr_status pdr_validate_indices(const uint32_t* indices, uint64_t n, uint32_t vertex_count,
                                         uint32_t* status, void* stream);
 
+/* pdr_validate_indices with its answer on return: host_status is PDR_STATUS_WORDS words of pinned host memory
+ * that the device can address; waits for the stream. */
+PDR_API pdr_status pdr_check_indices(const uint32_t* indices, uint64_t n, uint32_t vertex_count,
+                                     uint32_t* host_status, void* stream);
+
 /* Tile binning (src/rasterizer.cpp:61-138 build_tile_bins) for all views at once: CSR over
  * (view, 16x16 tile) with triangle ids ascending in every tile, bit-identical to the reference's
  * lists. tile_offsets has views*tiles+1 entries; tile_triangles holds `capacity` entries; the

@@ -41,6 +41,7 @@ _SIGNATURES = {
     "pdr_device_info": (_i32, [_i32, C.c_char_p, _sz, C.POINTER(_u32), C.POINTER(_u32), C.POINTER(_u32),
                                C.POINTER(_i32)]),
     "pdr_validate_indices": (_i32, [_vp, _u64, _u32, _vp, _vp]),
+    "pdr_check_indices": (_i32, [_vp, _u64, _u32, _vp, _vp]),
     "pdr_bin_tiles_workspace_bytes": (_sz, [_u32, _u32, _u32, _u32, _u64]),
     "pdr_bin_tiles": (_i32, [_vp, _u32, _u32, _vp, _u32, _u32, _u32, _vp, _vp, _vp, _u64, _vp, _sz, _vp, _vp]),
     "pdr_rasterize_forward": (_i32, [_vp, _u32, _u32, _vp, _u32, _u32, _u32, _vp, _u32, _vp, _vp, _u64, _vp, _vp,

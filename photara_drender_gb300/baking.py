@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .rasterizer import Context, DeviceInfo, Rasterizer, _Io, _ptr, _viewports
+from .rasterizer import Context, DeviceInfo, Rasterizer, _CheckedIndices, _Io, _ptr, _viewport_rows
 
 @dataclass
 class _RefineState:
@@ -158,7 +158,8 @@ class TextureBaker:
         for (h, w), ks in groups.items():
             n = len(ks)
             sub = clip if n == clip.shape[0] else clip[ks].contiguous()
-            vps, _ = _viewports([viewports[k] for k in ks], n, w, h, ctx.device)
+            rows = [None if viewports[k] is None else tuple(viewports[k]) for k in ks]
+            vps = self.rasterizer._device_viewports(rows[0] if rows.count(rows[0]) == n else rows, n, w, h)
             raster = torch.empty((n, h, w, 4), dtype=torch.float32, device=ctx.device)
             self.rasterizer._raster(sub, idx, w, h, vps, 0, raster, None)
             for j, k in enumerate(ks):
@@ -264,7 +265,7 @@ class TextureBaker:
                     or not math.isfinite(min_view_cosine) or min_view_cosine < -1.0 or min_view_cosine > 1.0):
                 raise ValueError("projection confidence parameters are invalid")
             vp = None if viewports is None else viewports[k]
-            _, rows = _viewports(vp, 1, img.shape[1], img.shape[0], "cpu")
+            rows = _viewport_rows(vp, 1, img.shape[1], img.shape[0])
             imgs.append(img)
             masks.append(m)
             sizes.append((img.shape[0], img.shape[1]))
@@ -274,8 +275,8 @@ class TextureBaker:
         aclip = torch.empty((1, V, 4), dtype=torch.float32, device=ctx.device)
         _native.call("pdr_atlas_clip_positions", _ptr(uvt), V, _ptr(aclip), ctx.stream())
         araster = self._rasters(aclip, idx, [(h, w)], [None])[0]
-        apos = self.rasterizer.interpolate_forward(pos, idx, araster)
-        anrm = self.rasterizer.interpolate_forward(nrm, idx, araster)
+        apos = self.rasterizer.interpolate_forward(pos, _CheckedIndices(idx, V), araster)
+        anrm = self.rasterizer.interpolate_forward(nrm, _CheckedIndices(idx, V), araster)
 
         scale = float(softmax_scale)
         if blend_mode == "softmax" and (not (scale > 0.0) or not math.isfinite(scale)):
@@ -446,7 +447,7 @@ class TextureBaker:
                 if tuple(m.shape) != tuple(img.shape[:2]):
                     raise ValueError("each visibility mask must match its image dimensions")
             vp = None if viewports is None else viewports[k]
-            _, rows = _viewports(vp, 1, img.shape[1], img.shape[0], "cpu")
+            rows = _viewport_rows(vp, 1, img.shape[1], img.shape[0])
             imgs.append(img)
             masks.append(m)
             sizes.append((img.shape[0], img.shape[1]))
@@ -457,15 +458,16 @@ class TextureBaker:
         keep, weights = [], []
         for k in range(n):
             P = sizes[k][0] * sizes[k][1]
-            uvk = self.rasterizer.interpolate_forward(uvt, idx, rasters[k])
+            uvk = self.rasterizer.interpolate_forward(uvt, _CheckedIndices(idx, V), rasters[k])
             tgt = torch.empty((P, 3), dtype=torch.float32, device=ctx.device)
             msk = torch.empty((P,), dtype=torch.float32, device=ctx.device)
             _native.call("pdr_refine_prepare_view", _ptr(imgs[k]), imgs[k].shape[2], _ptr(masks[k]), _ptr(rasters[k]),
                          P, _ptr(tgt), _ptr(msk), ctx.stream())
             keep += [uvk, tgt, msk]
-            weights.append(float(msk.double().sum().item()))
+            weights.append(msk.sum(dtype=torch.float64))
             table[k].uv, table[k].target, table[k].mask, table[k].pixel_count = (uvk.data_ptr(), tgt.data_ptr(),
                                                                                  msk.data_ptr(), P)
+        weights = torch.stack(weights).tolist()  # one wait for all views
         table_dev = torch.frombuffer(bytearray(bytes(table)), dtype=torch.uint8).to(ctx.device)
         max_pixels = max(s[0] * s[1] for s in sizes)
         torch.cuda.synchronize(ctx.device)

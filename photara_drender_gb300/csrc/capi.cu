@@ -109,6 +109,15 @@ pdr_status pdr_validate_indices(const uint32_t* indices, uint64_t n, uint32_t ve
     return cuda_status(cudaGetLastError(), "validate_indices");
 }
 
+pdr_status pdr_check_indices(const uint32_t* indices, uint64_t n, uint32_t vertex_count, uint32_t* host_status,
+                             void* stream) {
+    if (!host_status || (n && !indices)) return fail(PDR_INVALID_ARGUMENT, "indices and status are required");
+    host_status[PDR_STATUS_INDEX_ERROR] = 0u;
+    // the kernel writes the word where the host reads it: one launch and one wait
+    const pdr_status st = pdr_validate_indices(indices, n, vertex_count, host_status, stream);
+    return st ? st : cuda_status(cudaStreamSynchronize((cudaStream_t)stream), "check_indices");
+}
+
 size_t pdr_bin_tiles_workspace_bytes(uint32_t views, uint32_t triangle_count, uint32_t width, uint32_t height,
                                      uint64_t capacity) {
     return bins_workspace_bytes(views, triangle_count, width, height, capacity);

@@ -12,6 +12,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import threading
+import weakref
 from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
@@ -23,6 +24,7 @@ from . import _native
 CULL_MODES = {"none": 0, "back": 1, "front": 2}
 ADDRESS_MODES = {"clamp": 0, "wrap": 1, "mirror": 2}
 TILE = 16
+_VIEWPORT_CACHE = 256
 NEAR_MAX_TRIANGLES = 8388608  # PDR_NEAR_MAX_TRIANGLES: ids of the clipped mesh (2 T) stay exact in fp32
 
 
@@ -73,6 +75,29 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+class _HostWords:
+    """Status blocks in pinned host memory, one per context, cut from pages of 128 (pinning one takes 0.2 ms). A
+    context gives its block back when it goes; it waits for the device on every use, so nothing writes to it then."""
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._free = []
+
+    def take(self) -> torch.Tensor:
+        with self._lock:
+            if not self._free:
+                page = torch.zeros((128, _native.STATUS_WORDS), dtype=torch.int32, pin_memory=True)
+                self._free = list(page.unbind(0))
+            return self._free.pop()
+
+    def give(self, block: torch.Tensor) -> None:
+        with self._lock:
+            self._free.append(block)
+
+
+_host_words = _HostWords()
+
+
 class Context:
     """One CUDA device plus a lock that serialises calls, as the reference's per-context
     dispatch mutex does (src/context_internal.hpp:101)."""
@@ -89,9 +114,22 @@ class Context:
         self.status = torch.zeros(_native.STATUS_WORDS, dtype=torch.int32, device=self.device)
         self._pending = []  # (event, pinned copy of the status block, kind) of calls that did not wait
         self._spare = []    # pinned buffers ready for reuse
+        self._host_status = _host_words.take()
+        weakref.finalize(self, _host_words.give, self._host_status)
 
     def stream(self):
         return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+
+    def read_status(self):
+        """Waits for the work enqueued so far; the status block's words."""
+        self._host_status.copy_(self.status, non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        return self._host_status.tolist()
+
+    def indices_in_range(self, idx: torch.Tensor, vertex_count: int) -> bool:
+        """Whether every element of an int32 tensor on this device names one of vertex_count vertices (waits)."""
+        _native.call("pdr_check_indices", _ptr(idx), idx.numel(), vertex_count, _ptr(self._host_status), self.stream())
+        return int(self._host_status[_native.STATUS_INDEX_ERROR]) == 0
 
     def defer_status(self, kind: str) -> None:
         """Queues a copy of the status block to pinned host memory behind the work just enqueued,
@@ -127,6 +165,14 @@ class Context:
         return done
 
 
+class _CheckedIndices:
+    """Triangle indices that were validated against `vertex_count` before: what an autograd forward checked and
+    saved comes back to the adjoints in this wrapper."""
+
+    def __init__(self, tensor: torch.Tensor, vertex_count: int):
+        self.tensor, self.vertex_count = tensor, vertex_count
+
+
 class _Io:
     """Converts caller arrays to device tensors and results back to the caller's kind."""
 
@@ -146,12 +192,21 @@ class _Io:
 
     def indices(self, x, vertex_count: int, exc=IndexError,
                 msg="triangle_indices contains an invalid vertex index") -> torch.Tensor:
+        if isinstance(x, _CheckedIndices):
+            if x.vertex_count <= vertex_count:
+                return x.tensor.detach().to(self.ctx.device, torch.int32).contiguous()
+            x = x.tensor
         if isinstance(x, torch.Tensor):
             t = x.detach()
             if t.ndim != 2 or t.shape[1] != 3 or t.shape[0] <= 0:
                 raise ValueError("indices must have shape [triangle_count, 3]")
             if t.dtype.is_floating_point:
                 raise ValueError("indices must be an integer tensor")
+            if t.dtype == torch.int32 and t.device == self.ctx.device and vertex_count <= 0x7fffffff:
+                t = t.contiguous()  # one kernel and one wait; a negative index is a large unsigned one
+                if not self.ctx.indices_in_range(t, vertex_count):
+                    raise exc(msg)
+                return t
             if t.numel() and bool(((t.to(torch.int64) < 0) | (t.to(torch.int64) >= vertex_count)).any()):
                 raise exc(msg)
             return t.to(self.ctx.device, torch.int32).contiguous()
@@ -184,7 +239,7 @@ def _single_viewport(vp) -> bool:
     return a.ndim == 1 and a.shape[0] == 4
 
 
-def _viewports(viewport, views: int, width: int, height: int, device) -> Tuple[torch.Tensor, list]:
+def _viewport_rows(viewport, views: int, width: int, height: int) -> list:
     """src/rasterizer.cpp:48-59 resolve_viewport, per view."""
     if viewport is None or _single_viewport(viewport):
         per = [viewport] * views
@@ -202,6 +257,12 @@ def _viewports(viewport, views: int, width: int, height: int, device) -> Tuple[t
         if not all(math.isfinite(v) for v in vp) or vp[2] <= 0.0 or vp[3] <= 0.0:
             raise ValueError("viewport must contain finite values and positive dimensions")
         rows.append(vp)
+    return rows
+
+
+def _viewports(viewport, views: int, width: int, height: int, device) -> Tuple[torch.Tensor, list]:
+    """The rows of _viewport_rows on the device, and on the host."""
+    rows = _viewport_rows(viewport, views, width, height)
     return torch.tensor(rows, dtype=torch.float32, device=device), rows
 
 
@@ -211,10 +272,31 @@ class Rasterizer:
     def __init__(self, device_index: int = 0, enable_validation: bool = False):
         self.context = Context(device_index, enable_validation)
         self._capacity = 0
+        self._viewport_cache = {}  # (viewport, views, width, height) -> device rows, at most _VIEWPORT_CACHE of them
 
     @property
     def device_info(self) -> DeviceInfo:
         return self.context.info
+
+    def _device_viewports(self, viewport, views: int, width: int, height: int) -> torch.Tensor:
+        """The device rows of one viewport for all views, kept on the rasterizer: they are constants, their upload
+        waits for the host, and it is not allowed inside a CUDA graph capture. Rows given per view are kept too,
+        for the captures."""
+        try:
+            key = (views, width, height, None if viewport is None else tuple(
+                tuple(float(x) for x in v) if isinstance(v, (list, tuple)) else v if v is None else float(v)
+                for v in viewport))
+            rows = self._viewport_cache.get(key)
+        except TypeError:
+            return _viewports(viewport, views, width, height, self.context.device)[0]
+        if rows is None:
+            rows, _ = _viewports(viewport, views, width, height, self.context.device)
+            if len(self._viewport_cache) >= _VIEWPORT_CACHE:
+                self._viewport_cache.pop(next(iter(self._viewport_cache)))
+            self._viewport_cache[key] = rows
+        else:  # possibly made on another stream: its memory may not be reused under this one's work
+            rows.record_stream(torch.cuda.current_stream(self.context.device))
+        return rows
 
     # -- tile binning -------------------------------------------------------------------------
     def _bin(self, clip: torch.Tensor, idx: torch.Tensor, width: int, height: int, vps: torch.Tensor):
@@ -248,7 +330,7 @@ class Rasterizer:
             clip = self._clip(io, positions)
             idx = io.indices(indices, clip.shape[1])
             h, w = int(resolution[0]), int(resolution[1])
-            vps, _ = _viewports(viewport, clip.shape[0], w, h, self.context.device)
+            vps = self._device_viewports(viewport, clip.shape[0], w, h)
             offsets, lst, _, total = self._bin(clip, idx, w, h, vps)
             return io.out(offsets.view(torch.int32)), io.out(lst[:total])
 
@@ -298,7 +380,7 @@ class Rasterizer:
             h, w = int(resolution[0]), int(resolution[1])
             if h <= 0 or w <= 0:
                 raise ValueError("Rasterization width and height must be positive")
-            vps, _ = _viewports(viewport, views, w, h, ctx.device)
+            vps = self._device_viewports(viewport, views, w, h)
             raster = torch.empty((views, h, w, 4), dtype=torch.float32, device=ctx.device)
             deriv = torch.empty((views, h, w, 4), dtype=torch.float32, device=ctx.device) \
                 if output_barycentric_derivatives else None
@@ -344,7 +426,7 @@ class Rasterizer:
             if g.shape != r.shape:
                 raise ValueError("grad_raster must have shape [height, width, 4]")
             h, w = r.shape[1], r.shape[2]
-            vps, _ = _viewports(viewport, views, w, h, ctx.device)
+            vps = self._device_viewports(viewport, views, w, h)
             out = torch.empty((views, V, 4), dtype=torch.float32, device=ctx.device)
             gd = None
             if grad_barycentric_derivatives is not None:
@@ -471,7 +553,7 @@ class Rasterizer:
             ctx.status.zero_()
             _native.call("pdr_texture_backward", _ptr(tex), stride, tw, th, Cc, mode, _ptr(u), _ptr(r), views, h * w,
                          _ptr(g), _ptr(gt), _ptr(gu), _ptr(ctx.status), ctx.stream())
-            err = int(ctx.status[_native.STATUS_TEXEL_ERROR].item())
+            err = ctx.read_status()[_native.STATUS_TEXEL_ERROR]
             if err == 1:
                 raise ValueError("uv contains a non-finite value in a covered pixel")
             if err == 2:

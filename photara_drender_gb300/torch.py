@@ -11,7 +11,7 @@ from typing import NamedTuple, Optional, Sequence, Tuple
 
 import torch
 
-from .rasterizer import Rasterizer
+from .rasterizer import Rasterizer, _CheckedIndices
 
 _default_rasterizers: dict = {}
 
@@ -41,6 +41,7 @@ class _RasterizeFunction(torch.autograd.Function):
         ctx.cull_mode = cull_mode
         ctx.recompute = recompute
         ctx.differentiable_derivatives = bool(differentiable_derivatives and output_barycentric_derivatives)
+        ctx.set_materialize_grads(False)  # an unused output's gradient is None, not an image of zeros
         if recompute:
             ctx.save_for_backward(positions.detach(), indices.detach())
         else:
@@ -56,10 +57,12 @@ class _RasterizeFunction(torch.autograd.Function):
             return (None,) * 10
         if ctx.recompute:
             positions, indices = ctx.saved_tensors
+            indices = _CheckedIndices(indices, positions.shape[-2])
             raster, _ = ctx.rasterizer.forward(positions, indices, ctx.resolution, ctx.cull_mode, False, ctx.viewport,
                                                clip_near_plane=ctx.clip_near_plane)
         else:
             positions, indices, raster = ctx.saved_tensors
+            indices = _CheckedIndices(indices, positions.shape[-2])
         if grad_raster is None:
             grad_raster = torch.zeros_like(raster)
         grad_positions = ctx.rasterizer.backward(
@@ -88,8 +91,8 @@ class _InterpolateFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_interpolated):
         attributes, raster, indices = ctx.saved_tensors
-        grad_attributes, grad_raster = ctx.rasterizer.interpolate_backward(attributes, indices, raster,
-                                                                           grad_interpolated.contiguous())
+        grad_attributes, grad_raster = ctx.rasterizer.interpolate_backward(
+            attributes, _CheckedIndices(indices, attributes.shape[-2]), raster, grad_interpolated.contiguous())
         return grad_attributes, grad_raster, None, None
 
 
@@ -196,26 +199,6 @@ def _apply_status(reports) -> None:
             raise IndexError("uv is too large for portable texture addressing")
 
 
-def _cached_viewports(r: Rasterizer, viewport, views: int, w: int, h: int) -> torch.Tensor:
-    """The device viewport rows of render calls, kept per (viewport, views, size) on the rasterizer: an
-    upload from pageable host memory is not allowed inside a CUDA graph capture, so a captured call
-    reuses the rows an earlier call made."""
-    from .rasterizer import _viewports
-
-    try:
-        key = (views, w, h, None if viewport is None else tuple(
-            tuple(float(x) for x in v) if isinstance(v, (list, tuple)) else float(v) for v in viewport))
-    except TypeError:
-        key = None
-    cache = r.__dict__.setdefault("_render_viewports", {})
-    if key is not None and key in cache:
-        return cache[key]
-    vps, _ = _viewports(viewport, views, w, h, r.context.device)
-    if key is not None:
-        cache[key] = vps
-    return vps
-
-
 def check_deferred_errors(rasterizer: Rasterizer) -> None:
     """Waits for every `render(..., deferred_errors=True)` call made on this rasterizer and raises the
     first error the device recorded for them (ValueError / IndexError, as the synchronous path raises at once)."""
@@ -272,7 +255,7 @@ class _RenderFunction(torch.autograd.Function):
             clip = (clip if batched else clip.unsqueeze(0)).contiguous()
             idx = indices.detach().to(r.context.device, torch.int32).contiguous()
             h, w = int(resolution[0]), int(resolution[1])
-            vps = _cached_viewports(r, viewport, clip.shape[0], w, h)
+            vps = r._device_viewports(viewport, clip.shape[0], w, h)
             attrs = vertex_attributes.detach().contiguous() if vertex_attributes is not None else None
             uva = vertex_uv.detach().contiguous() if vertex_uv is not None else None
             tex = texture_values.detach().contiguous() if texture_values is not None else None
@@ -342,15 +325,11 @@ class _RenderFunction(torch.autograd.Function):
             if deferred:
                 r.context.defer_status("render_backward")
             else:
-                st = r.context.status.cpu()
-                if int(st[_native.STATUS_TEXEL_ERROR]) == 1:
-                    raise ValueError("uv contains a non-finite value in a covered pixel")
-                if int(st[_native.STATUS_TEXEL_ERROR]) == 2:
-                    raise IndexError("uv is too large for portable texture addressing")
+                _apply_status([("render_backward", r.context.read_status())])
         # upstream gradients on the raster or uv outputs themselves go through the separate adjoints
         extra = g_raster.contiguous() if g_raster is not None else None
         if g_uv is not None and uva is not None:
-            gua, gr = r.interpolate_backward(uva, idx, raster, g_uv.contiguous())
+            gua, gr = r.interpolate_backward(uva, idx, raster, g_uv.contiguous())  # validates idx: render does not
             grad_uv = grad_uv + gua
             extra = gr if extra is None else extra + gr
         if extra is not None:
