@@ -577,6 +577,14 @@ PDR_API pdr_status pdr_ray_visibility_views(const void* bvh, uint32_t triangle_c
                                             uint32_t atlas_texels, const pdr_projection_view* views,
                                             uint32_t view_count, float ray_origin_bias, uint32_t* visibility,
                                             void* stream);
+/* pdr_ray_visibility_views of an atlas of rows of atlas_width texels (0: unknown): neighbours in both directions then
+ * share a warp. The bits are the same. */
+PDR_API pdr_status pdr_ray_visibility_atlas(const void* bvh, uint32_t triangle_count, const float* atlas_positions,
+                                            const float* atlas_normals, const float* atlas_raster,
+                                            uint32_t atlas_texels, uint32_t atlas_width,
+                                            const pdr_projection_view* views, uint32_t view_count,
+                                            float ray_origin_bias, uint32_t* visibility,
+                                            void* stream);
 /* pdr_project_views for visibility modes 1 (ray x shadow map) and 2 (ray) with the visibility bits of
  * pdr_ray_visibility instead of per-view arrays. */
 PDR_API pdr_status pdr_project_views_bits(const float* atlas_positions, const float* atlas_normals,
@@ -585,6 +593,14 @@ PDR_API pdr_status pdr_project_views_bits(const float* atlas_positions, const fl
                                           uint32_t pcf_radius, uint32_t visibility_mode, const uint32_t* visibility,
                                           float* color, float* confidence, uint32_t* source_view, float* valid_mask,
                                           float* coverage_mask, uint32_t* face_ids, void* stream);
+/* Both of them for an atlas of rows of atlas_width texels (0: unknown), with or without (NULL) visibility bits; the
+ * results are the same, neighbours in both directions share a warp. */
+PDR_API pdr_status pdr_project_views_atlas(const float* atlas_positions, const float* atlas_normals,
+                                           const float* atlas_raster, uint32_t atlas_texels, uint32_t atlas_width,
+                                           const pdr_projection_view* views, uint32_t view_count, uint32_t blend_mode,
+                                           uint32_t pcf_radius, uint32_t visibility_mode, const uint32_t* visibility,
+                                           float* color, float* confidence, uint32_t* source_view, float* valid_mask,
+                                           float* coverage_mask, uint32_t* face_ids, void* stream);
 
 /* ---- atlas padding and surface fill (src/texture_padding.cpp) --------------------------------------- */
 

@@ -316,14 +316,10 @@ class TextureBaker:
         valid = torch.empty((h, w), dtype=torch.float32, device=ctx.device)
         cov = torch.empty((h, w), dtype=torch.float32, device=ctx.device)
         faces = torch.empty((h, w), dtype=torch.int32, device=ctx.device)
-        if ray_bits is None:
-            _native.call("pdr_project_views", _ptr(apos), _ptr(anrm), _ptr(araster), N, _ptr(table_dev), n,
-                         BLEND_MODES[blend_mode], int(pcf_radius), effective_visibility, _ptr(color), _ptr(conf),
-                         _ptr(src), _ptr(valid), _ptr(cov), _ptr(faces), ctx.stream())
-        else:
-            _native.call("pdr_project_views_bits", _ptr(apos), _ptr(anrm), _ptr(araster), N, _ptr(table_dev), n,
-                         BLEND_MODES[blend_mode], int(pcf_radius), effective_visibility, _ptr(ray_bits), _ptr(color),
-                         _ptr(conf), _ptr(src), _ptr(valid), _ptr(cov), _ptr(faces), ctx.stream())
+        _native.call("pdr_project_views_atlas", _ptr(apos), _ptr(anrm), _ptr(araster), N, w, _ptr(table_dev), n,
+                     BLEND_MODES[blend_mode], int(pcf_radius), effective_visibility,
+                     None if ray_bits is None else _ptr(ray_bits), _ptr(color), _ptr(conf), _ptr(src), _ptr(valid),
+                     _ptr(cov), _ptr(faces), ctx.stream())
         host = io.numpy or not isinstance(positions, torch.Tensor)
 
         def out(t, u32=False):
@@ -353,8 +349,8 @@ class TextureBaker:
         N = araster.numel() // 4
         bits = torch.empty((N, (n + 31) // 32), dtype=torch.int32, device=ctx.device)
         if views is not None:
-            _native.call("pdr_ray_visibility_views", _ptr(bvh), T, _ptr(apos), _ptr(anrm), _ptr(araster), N,
-                         _ptr(views), n, float(bias), _ptr(bits), ctx.stream())
+            _native.call("pdr_ray_visibility_atlas", _ptr(bvh), T, _ptr(apos), _ptr(anrm), _ptr(araster), N,
+                         araster.shape[-2], _ptr(views), n, float(bias), _ptr(bits), ctx.stream())
             return bits
         cam4 = torch.zeros((n, 4), dtype=torch.float32, device=ctx.device)
         cam4[:, :3] = torch.from_numpy(np.ascontiguousarray(cams, dtype=np.float32)).to(ctx.device)

