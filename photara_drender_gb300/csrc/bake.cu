@@ -19,6 +19,8 @@ namespace {
 
 __device__ __forceinline__ float lerp_hlsl(float x, float y, float s) { return x * (1.0f - s) + y * s; }
 
+// Positions become texel indices by __float2int_rz, which saturates and takes NaN to 0 as the shader's conversion does.
+
 // project_texture.hlsl:46-56: the bilinear photo sample with clamped taps, for channels 0..2 (and 3 when
 // the image has four). The tap positions and weights are the same for every channel, so they are
 // computed once and each tap's channels are read together.
@@ -28,15 +30,26 @@ struct PhotoSample {
 
 __device__ __forceinline__ PhotoSample sample_photo_rgba(const pdr_projection_view& v, float ppx, float ppy) {
     const float tx = ppx - 0.5f, ty = ppy - 0.5f;
-    const int32_t bx = f2i_sat(floorf(tx)), by = f2i_sat(floorf(ty));
+    const int32_t bx = __float2int_rz(floorf(tx)), by = __float2int_rz(floorf(ty));
     const float fx = tx - floorf(tx), fy = ty - floorf(ty);
     const int32_t w = (int32_t)v.width - 1, h = (int32_t)v.height - 1;
     const uint32_t x0 = (uint32_t)clampi(bx, 0, w), x1 = (uint32_t)clampi(add1(bx), 0, w);
     const uint32_t y0 = (uint32_t)clampi(by, 0, h), y1 = (uint32_t)clampi(add1(by), 0, h);
     const uint32_t C = v.channel_count;
     const float* img = v.image;
-    const size_t t00 = ((size_t)y0 * v.width + x0) * C, t10 = ((size_t)y0 * v.width + x1) * C;
-    const size_t t01 = ((size_t)y1 * v.width + x0) * C, t11 = ((size_t)y1 * v.width + x1) * C;
+    const size_t t00 = ((size_t)y0 * v.width + x0) * C, t10 = t00 + (x1 - x0) * C;
+    const size_t down = y1 != y0 ? (size_t)v.width * C : 0, t01 = t00 + down, t11 = t10 + down;
+    const auto blend = [&](float v00, float v10, float v01, float v11) {
+        return lerp_hlsl(lerp_hlsl(v00, v10, fx), lerp_hlsl(v01, v11, fx), fy);
+    };
+    if (C == 4 && ((uintptr_t)img & 15u) == 0) {  // one load a tap
+        const float4 a = __ldg(reinterpret_cast<const float4*>(img + t00));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(img + t10));
+        const float4 c = __ldg(reinterpret_cast<const float4*>(img + t01));
+        const float4 d = __ldg(reinterpret_cast<const float4*>(img + t11));
+        return {blend(a.x, b.x, c.x, d.x), blend(a.y, b.y, c.y, d.y), blend(a.z, b.z, c.z, d.z),
+                blend(a.w, b.w, c.w, d.w)};
+    }
     float r[4];
 #pragma unroll
     for (uint32_t ch = 0; ch < 4; ++ch) {
@@ -46,7 +59,7 @@ __device__ __forceinline__ PhotoSample sample_photo_rgba(const pdr_projection_vi
         }
         const float v00 = __ldg(img + t00 + ch), v10 = __ldg(img + t10 + ch);
         const float v01 = __ldg(img + t01 + ch), v11 = __ldg(img + t11 + ch);
-        r[ch] = lerp_hlsl(lerp_hlsl(v00, v10, fx), lerp_hlsl(v01, v11, fx), fy);
+        r[ch] = blend(v00, v10, v01, v11);
     }
     return {r[0], r[1], r[2], r[3]};
 }
@@ -61,7 +74,7 @@ __device__ __forceinline__ float mask_tap(const pdr_projection_view& v, int32_t 
 __device__ __forceinline__ float sample_mask(const pdr_projection_view& v, float ppx, float ppy, float floor_value) {
     const int32_t w = (int32_t)v.width, h = (int32_t)v.height;
     const float tx = ppx - 0.5f, ty = ppy - 0.5f;
-    const int32_t bx = f2i_sat(floorf(tx)), by = f2i_sat(floorf(ty));
+    const int32_t bx = __float2int_rz(floorf(tx)), by = __float2int_rz(floorf(ty));
     const float fx = tx - floorf(tx), fy = ty - floorf(ty);
     const int32_t x0 = clampi(bx, 0, w - 1), x1 = clampi(add1(bx), 0, w - 1);
     const int32_t y0 = clampi(by, 0, h - 1), y1 = clampi(add1(by), 0, h - 1);
@@ -70,13 +83,38 @@ __device__ __forceinline__ float sample_mask(const pdr_projection_view& v, float
     return lerp_hlsl(lerp_hlsl(v00, v10, fx), lerp_hlsl(v01, v11, fx), fy);
 }
 
+// The taps of shadow_visibility where all of them lie inside the view.
+template <int kRadius>
+__device__ __forceinline__ float inner_visibility(const float4* __restrict__ first, uint32_t width, float depth, float bias,
+                                                  int32_t r) {
+    const int32_t n = kRadius < 0 ? 2 * r + 1 : 2 * kRadius + 1;
+    uint32_t visible = 0, count = 0;
+    const float4* row = first;
+#pragma unroll
+    for (int32_t y = 0; y < n; ++y, row += width) {
+#pragma unroll
+        for (int32_t x = 0; x < n; ++x) {
+            const float2 s = __ldg(reinterpret_cast<const float2*>(row + x) + 1);  // depth, triangle
+            const bool covered = s.y > 0.5f;                                       // raster_id(s.y) != 0
+            visible += covered && depth <= s.x + bias;
+            count += covered;
+        }
+    }
+    return count > 0 ? (float)visible / (float)count : 0.0f;
+}
+
 // project_texture.hlsl:76-101
 __device__ __forceinline__ float shadow_visibility(const pdr_projection_view& v, float ppx, float ppy, float depth,
                                                    int32_t r) {
     const int32_t w = (int32_t)v.width, h = (int32_t)v.height;
-    const int32_t cx = f2i_sat(floorf(ppx)), cy = f2i_sat(floorf(ppy));
+    const int32_t cx = __float2int_rz(floorf(ppx)), cy = __float2int_rz(floorf(ppy));
     float visible = 0.0f, count = 0.0f;
     const float4* shadow = reinterpret_cast<const float4*>(v.shadow_raster);
+    if (cx >= r && cy >= r && cx < w - r && cy < h - r) {
+        const float4* first = shadow + (size_t)(cy - r) * v.width + (size_t)(cx - r);
+        return r == 1 ? inner_visibility<1>(first, v.width, depth, v.depth_bias, r)
+                      : inner_visibility<-1>(first, v.width, depth, v.depth_bias, r);
+    }
     for (int32_t y = -r; y <= r; ++y) {
         for (int32_t x = -r; x <= r; ++x) {
             const int32_t X = cx + x, Y = cy + y;
@@ -94,7 +132,10 @@ __device__ __forceinline__ float shadow_visibility(const pdr_projection_view& v,
 constexpr uint32_t kViewChunk = 32;
 static_assert(sizeof(pdr_projection_view) % sizeof(uint4) == 0, "view records are copied as 16-byte words");
 
-__global__ void __launch_bounds__(128, 12)  // 40 registers: 48 warps per SM for the gathers
+// Bound by issue and L1 together (73% and 88%). 24 views of 1024 x 1024 with shadow maps and 3 x 3 taps into 2048 x 2048
+// texels: 1070 us, with the gate 952, in tiles 845, with the divisions shared, inner taps unchecked and conversions left to
+// the instruction's own saturation 688; in 48 registers 597 (64: 648, 40 spill).
+__global__ void __launch_bounds__(128, 10)
 project_views_kernel(const float* __restrict__ apos, const float* __restrict__ anrm,
                                      const float4* __restrict__ araster, uint32_t N,
                                      const pdr_projection_view* __restrict__ views, uint32_t nviews,
@@ -138,7 +179,7 @@ project_views_kernel(const float* __restrict__ apos, const float* __restrict__ a
         for (uint32_t kk = 0; kk < cnt; ++kk) {
             const uint32_t k = k0 + kk;
             const pdr_projection_view& v = sv[kk];
-            // most texel-views end here: 24 views of a 2048 x 2048 atlas with shadow maps 1070 -> 952 us, in tiles 845
+            // most texel-views end here
             if (project_gate(gates[kk], px, py, pz, nx, ny, nz) == Gate::kReject) continue;
             ProjectedTexel pt;
             if (!project_texel(v, px, py, pz, nx, ny, nz, pt)) continue;

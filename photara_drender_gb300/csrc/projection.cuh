@@ -16,6 +16,25 @@ struct ProjectedTexel {
     float vl, cosv;       // distance to the camera and cosine of the view angle
 };
 
+// a / d, b / d and c / d with one division: quotients by a fixed divisor as in NdcAxis, under its conditions.
+__device__ __forceinline__ void quotients(float a, float b, float c, float d, float& qa, float& qb, float& qc) {
+    const float lo = fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)), hi = fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c));
+    if (lo >= 1e-25f && hi <= 1e25f && d >= 1e-6f && d <= 1e9f && (__float_as_uint(d) & 0x7fffffu) != 0x7fffffu) {
+        const float r = 1.0f / d;
+        const auto quotient = [&](float n) {
+            const float q = n * r;
+            return __fmaf_rn(__fmaf_rn(-q, d, n), r, q);
+        };
+        qa = quotient(a);
+        qb = quotient(b);
+        qc = quotient(c);
+    } else {
+        qa = a / d;
+        qb = b / d;
+        qc = c / d;
+    }
+}
+
 __device__ __forceinline__ bool project_texel(const pdr_projection_view& v, float px, float py, float pz, float nx,
                                               float ny, float nz, ProjectedTexel& o) {
     const float* M = v.world_to_clip;
@@ -24,7 +43,8 @@ __device__ __forceinline__ bool project_texel(const pdr_projection_view& v, floa
     const float cx = M[0] * px + M[1] * py + M[2] * pz + M[3] * 1.0f;
     const float cy = M[4] * px + M[5] * py + M[6] * pz + M[7] * 1.0f;
     const float cz = M[8] * px + M[9] * py + M[10] * pz + M[11] * 1.0f;
-    const float ndx = cx / cw, ndy = cy / cw, ndz = cz / cw;
+    float ndx, ndy, ndz;
+    quotients(cx, cy, cz, cw, ndx, ndy, ndz);
     if (ndx < -1.0f || ndy < -1.0f || ndx > 1.0f || ndy > 1.0f || ndz < -1.0f || ndz > 1.0f) return false;
     const float ppx = v.viewport[0] + (ndx * 0.5f + 0.5f) * v.viewport[2];
     const float ppy = v.viewport[1] + (ndy * 0.5f + 0.5f) * v.viewport[3];
@@ -36,7 +56,9 @@ __device__ __forceinline__ bool project_texel(const pdr_projection_view& v, floa
     const float vx0 = v.camera_position[0] - px, vy0 = v.camera_position[1] - py;
     const float vz0 = v.camera_position[2] - pz;
     const float vl = sqrtf(vx0 * vx0 + vy0 * vy0 + vz0 * vz0);
-    const float cosv = nx * (vx0 / vl) + ny * (vy0 / vl) + nz * (vz0 / vl);
+    float dx, dy, dz;
+    quotients(vx0, vy0, vz0, vl, dx, dy, dz);
+    const float cosv = nx * dx + ny * dy + nz * dz;
     if (cosv < v.min_view_cosine) return false;
     o.ppx = ppx;
     o.ppy = ppy;

@@ -49,10 +49,10 @@ struct ClampTaps {
     float w[4];
 };
 
-// atlas_photometric_gradient.hlsl:56-74 / atlas_seam_gradient.hlsl:31-48
+// atlas_photometric_gradient.hlsl:56-74 / atlas_seam_gradient.hlsl:31-48 (__float2int_rz saturates and takes NaN to 0)
 __device__ __forceinline__ ClampTaps clamp_taps(float u, float v, uint32_t tw, uint32_t th) {
     const float px = u * (float)tw - 0.5f, py = v * (float)th - 0.5f;
-    const int32_t bx = f2i_sat(floorf(px)), by = f2i_sat(floorf(py));
+    const int32_t bx = __float2int_rz(floorf(px)), by = __float2int_rz(floorf(py));
     const float fx = px - floorf(px), fy = py - floorf(py);
     const uint32_t x0 = (uint32_t)clampi(bx, 0, (int32_t)tw - 1), x1 = (uint32_t)clampi(add1(bx), 0, (int32_t)tw - 1);
     const uint32_t y0 = (uint32_t)clampi(by, 0, (int32_t)th - 1), y1 = (uint32_t)clampi(add1(by), 0, (int32_t)th - 1);

@@ -115,3 +115,30 @@ def test_gate_and_tiles(shape, views):
         all_decided &= decided
     assert not bits[~covered].any()
     assert np.array_equal(valid[all_decided] != 0, seen[all_decided])
+
+
+@pytest.mark.parametrize("channels,offset", [(3, 0), (4, 0), (4, 1)])
+@pytest.mark.parametrize("pcf", [0, 1, 2, 4])
+def test_inner_taps(channels, offset, pcf):
+    """Shadow-map and photograph taps inside and across the borders of a view, at every radius, and of images whose
+    rows are not 16-byte aligned, against the oracle's bake, bit for bit."""
+    from oracle import api
+    from tests.gpu_util import same_bits
+
+    baker = TextureBaker(0)
+    pos3, nrm, uv, idx, _, _ = S.displaced_sphere(2000, seed=pcf, amplitude=0.15, atlas_size=64)
+    mats, eyes = S.orbit_cameras(3, fov_y_deg=30.0)  # the surface reaches past the views' borders
+    rng = np.random.default_rng(9)
+    images = [rng.uniform(size=(48, 40, channels)).astype(np.float32) for _ in range(3)]
+    held = []
+    for im in images:
+        flat = torch.zeros(im.size + offset, device=baker.context.device)
+        flat[offset:] = torch.tensor(im.reshape(-1), device=flat.device)
+        held.append(flat[offset:].view(im.shape))
+    out = baker.bake_output(pos3, nrm, uv, idx, held, mats, eyes, resolution=(64, 64), blend_mode="weighted_average",
+                            visibility_mode="shadow_map", pcf_radius=pcf)
+    color, conf, src, valid, _, _ = api.bake(pos3, nrm, uv, idx, images, mats, eyes, resolution=(64, 64),
+                                             blend_mode="weighted_average", visibility_mode=0, pcf_radius=pcf)
+    assert same_bits(np.asarray(out.color.cpu() if hasattr(out.color, "cpu") else out.color), color)
+    assert same_bits(np.asarray(out.confidence.cpu() if hasattr(out.confidence, "cpu") else out.confidence), conf)
+    assert valid.any()
