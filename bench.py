@@ -337,9 +337,8 @@ def c1_leg(dev, hbm):
     g_samp = torch.tensor(rng.standard_normal((views, H, W, c["channels"])).astype(np.float32), device=dev)
     r = Rasterizer(dev.index or 0)
     V, T = pos3.shape[0], idx.shape[0]
-    pipe = RenderFwdBwd(r, t_idx, V, views, H, W, c["attributes"], tuple(tex.shape))
+    pipe = RenderFwdBwd(r, t_idx, V, views, H, W, c["attributes"], tuple(tex.shape), direct=True)
     pipe.step(clip, attrs, uv, tex, g_attr, g_samp)
-    entries = pipe.check_capacity()
 
     def timed(fn, n):
         for _ in range(5):
@@ -356,12 +355,11 @@ def c1_leg(dev, hbm):
     ms_launch = timed(lambda: pipe.step(clip, attrs, uv, tex, g_attr, g_samp), c["steps"])
     graph = pipe.capture(clip, attrs, uv, tex, g_attr, g_samp)
     ms_graph = timed(graph.replay, c["steps"])
-    pipe.check_capacity()
     P = views * H * W
     alg = P * 96 + 2 * c["texture"] ** 2 * c["channels"] * 4 + views * V * 16 * 2 + T * 12 + V * (c["attributes"] + 2) * 8
     best = min(ms_launch, ms_graph)
     res = {"workload": c["name"], "mpix_per_s": P / 1e6 / (best / 1e3), "ms_per_step_graph": ms_graph,
-           "ms_per_step_launches": ms_launch, "tile_entries": entries, "algorithmic_bytes": alg,
+           "ms_per_step_launches": ms_launch, "algorithmic_bytes": alg,
            "achieved_gbs": alg / (best / 1e3) / 1e9, "frac": alg / (best / 1e3) / 1e9 / hbm,
            "timing": f"CUDA events over {c['steps']} fused fwd+bwd steps, device-resident inputs (which fit in L2)"}
     host = {k: v.cpu().pin_memory() for k, v in dict(clip=clip, attrs=attrs, uv=uv, tex=tex, g_attr=g_attr,
@@ -679,9 +677,8 @@ C4 = dict(name="c4_uneven_batch_16_meshes", meshes=16, tri_min=10_000, tri_max=1
 
 def c4_leg(dev, hbm):
     """C4: 16 meshes of log-uniform 10k-1M triangles, 4-48 views each at 512^2, 1024^2 or 2048x1536,
-    8-channel attributes, 2048^2 or 4096^2 RGBA textures, forward + backward in one batch (one binning
-    pass, one raster launch, one adjoint launch) with the autotuned tile shape and bin depth; each mesh
-    is also timed alone for the per-mesh p50 / p99."""
+    8-channel attributes, 2048^2 or 4096^2 RGBA textures, forward + backward in one batch (one
+    visibility pass, one shading launch, one adjoint launch); each mesh is also timed alone for the per-mesh p50 / p99."""
     import torch
 
     from photara_drender_gb300 import Rasterizer
@@ -713,8 +710,6 @@ def c4_leg(dev, hbm):
         meshes.append(m)
         desc.append({"triangles": int(idx.shape[0]), "views": views, "resolution": [h, w], "texture": ts})
     batch = MeshBatch(r, meshes)
-    tune = batch.autotune(reps=2)
-    best = (batch.config.tile_width, batch.config.tile_height, batch.config.stage_triangles)
 
     def timed(b):
         b.forward()
@@ -734,7 +729,7 @@ def c4_leg(dev, hbm):
     batch_ms = timed(batch)
     per_mesh = []
     for m in meshes:
-        single = MeshBatch(r, [m], config=best)
+        single = MeshBatch(r, [m])
         per_mesh.append(timed(single))
         del single
     P = sum(d["views"] * d["resolution"][0] * d["resolution"][1] for d in desc)
@@ -757,8 +752,7 @@ def c4_leg(dev, hbm):
                "one_core": {"value": done1 * px / 1e6 / secs1, "unit": "Mpix/s", "cores": 1,
                             "sample": f"{done1} views on one thread, {secs1:.2f} s"}}
     return {"workload": c["name"], "batch_ms": batch_ms, "mpix_per_s": P / 1e6 / (batch_ms / 1e3), "cpu_baseline": cpu,
-            "pixels": P, "meshes": desc, "autotune_ms": {f"{a}x{b}/{k}": t for (a, b, k), t in tune.items()},
-            "config": {"tile": [best[0], best[1]], "stage_triangles": best[2]},
+            "pixels": P, "meshes": desc,
             "per_mesh_ms_p50": float(np.percentile(per_mesh, 50)), "per_mesh_ms_p99": float(np.percentile(per_mesh, 99)),
             "per_mesh_ms": per_mesh, "per_mesh_sum_ms": float(np.sum(per_mesh)),
             "algorithmic_bytes": alg, "achieved_gbs": alg / (batch_ms / 1e3) / 1e9,
@@ -871,25 +865,19 @@ def c5_leg(dev, hbm):
 
 # ---- GPU arm ------------------------------------------------------------------------------------------
 
-STAGES = ["bin_tiles", "rasterize_forward+shade", "render_backward"]
-# Source files each timed kernel is compiled from, and DRAM bytes per launch (dram__bytes_read.sum +
-# dram__bytes_write.sum) of that kernel on this 64-view workload from a single-pass ncu capture of the
+STAGES = ["visibility+shade", "render_backward"]
+# Source files each timed stage is compiled from, and its DRAM bytes (dram__bytes_read.sum +
+# dram__bytes_write.sum over its kernels) on this 64-view workload from an ncu capture of the
 # full-size run, recorded with the SHA-256 of those sources at capture time. A capture cannot run
 # inside the timed region; when the sources no longer hash to the recorded value the figure belongs to
 # other code and the line reports traffic as null.
 KERNEL_SOURCES = {
-    "bin_tiles": ["raster.cu", "bin_rect.cuh", "pdr_common.cuh"],
-    "rasterize_forward+shade": ["raster.cu", "raster_tile.cuh", "bin_rect.cuh", "pdr_common.cuh"],
-    "render_backward": ["fused.cu", "render_bwd_tile.cuh", "pdr_common.cuh"],
+    "visibility+shade": ["visibility.cu", "visibility.cuh", "raster_tile.cuh", "ndc_axis.cuh", "tile_order.cuh",
+                         "pdr_common.cuh"],
+    "render_backward": ["fused.cu", "render_bwd_tile.cuh", "vertex_sums.cuh", "tile_order.cuh", "pdr_common.cuh"],
 }
-# stage -> (fused tile configuration or None when the stage does not depend on it, sha256 of its sources,
-# bytes per launch); from `ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum`
-# on the full 64-view run (profiles/launch_list_fwdbwd_200k_64x1024sq.md)
+# stage -> (sha256 of its sources, bytes)
 KERNEL_TRAFFIC = {
-    "bin_tiles": ((16, 8, 128), "ed20208abe26a4d1", 340085248),
-    "rasterize_forward+shade": ((16, 8, 128), "55b8bd4c31220dd3", 7962652416),
-    # the adjoint kernel (16x8 tiles) and the finishing pass over the per-view vertex records
-    "render_backward": (None, "75c07abc353cd1c9", 7130837760),
 }
 
 
@@ -903,28 +891,22 @@ def kernel_source_hash(stage: str) -> str:
     return h.hexdigest()
 
 
-def recorded_traffic(stage: str, config):
-    """The recorded DRAM bytes per launch of `stage`, when its sources (and, for the binning and raster
-    stages, the fused tile configuration) are those the capture ran; else None."""
+def recorded_traffic(stage: str):
+    """The recorded DRAM bytes of `stage`, when its sources are those the capture ran; else None."""
     rec = KERNEL_TRAFFIC.get(stage)
-    if not rec or not kernel_source_hash(stage).startswith(rec[1]):
-        return None
-    return rec[2] if rec[0] is None or tuple(rec[0]) == tuple(config) else None
+    return rec[1] if rec and kernel_source_hash(stage).startswith(rec[0]) else None
 
 
-def stage_bytes(w, T, V, entries):
-    """Algorithmic bytes per launch of each timed stage: API-boundary tensors, each read or written
-    once (tile lists count for binning only, where they are the output)."""
+def stage_bytes(w, T, V):
+    """Algorithmic bytes of each timed stage: API-boundary tensors, each read or written once."""
     P = w["views"] * w["height"] * w["width"]
     A, Cc = w["attributes"], w["channels"]
     tex = w["atlas"] * w["atlas"] * Cc * 4
     mesh = w["views"] * V * 16 + T * 12
-    tiles = w["views"] * ((w["height"] + 15) // 16) * ((w["width"] + 15) // 16)
     return {
-        "bin_tiles": mesh + entries * 4 + (tiles + 1) * 4,
         # inputs: clip, indices, attributes, uv attributes, texture; outputs raster, derivatives,
         # attributes, uv, sampled
-        "rasterize_forward+shade": mesh + V * (A + 2) * 4 + tex + P * (16 + 16 + A * 4 + 8 + Cc * 4),
+        "visibility+shade": mesh + V * (A + 2) * 4 + tex + P * (16 + 16 + A * 4 + 8 + Cc * 4),
         # inputs: raster, uv, grad_interpolated, grad_sampled, texture, clip, attributes;
         # outputs: grad_texture, grad_clip, grad_attributes, grad_uv_attributes
         "render_backward": P * (16 + 8 + A * 4 + Cc * 4) + 2 * tex + 2 * mesh + 2 * V * (A + 2) * 4,
@@ -1053,20 +1035,18 @@ def run_gpu(args, world, rank, local):
     g_attr = torch.randn((views, H, W, w["attributes"]), device=dev, generator=g)
     g_samp = torch.randn((views, H, W, w["channels"]), device=dev, generator=g)
 
-    pipe = RenderFwdBwd(r, t_idx, V, views, H, W, w["attributes"], tuple(tex.shape), capacity=4 * T * views)
-    # tile shape and stage depth of the fused forward from the project's autotuner (outputs identical for
-    # every choice); it also sizes the tile list to the measured need
-    if args.tile:
+    if args.tile:  # the forward through tile lists of this shape and stage depth
         tw_th, k = args.tile.split("/")
         cfg = tuple(int(x) for x in tw_th.split("x")) + (int(k),)
-        pipe.set_tile_config(cfg)
-        tune = {}
-        pipe.step(clip, t_attrs, t_uv, tex, g_attr, g_samp, stream)
-        pipe.set_tile_config(cfg, int(pipe.check_capacity() * 1.25) + 1024)
-    else:
-        tune = pipe.autotune(clip, t_attrs, t_uv, tex)
+        pipe = RenderFwdBwd(r, t_idx, V, views, H, W, w["attributes"], tuple(tex.shape), capacity=4 * T * views,
+                            tile_config=cfg)
+    else:  # through the visibility buffer, as the public render
+        pipe = RenderFwdBwd(r, t_idx, V, views, H, W, w["attributes"], tuple(tex.shape), direct=True)
     pipe.step(clip, t_attrs, t_uv, tex, g_attr, g_samp, stream)
-    entries = pipe.check_capacity()
+    if args.tile:
+        pipe.set_tile_config(cfg, int(pipe.check_capacity() * 1.25) + 1024)
+        pipe.step(clip, t_attrs, t_uv, tex, g_attr, g_samp, stream)
+    pipe.check_capacity()
     for _ in range(args.warmup):
         pipe.step(clip, t_attrs, t_uv, tex, g_attr, g_samp, stream)
     torch.cuda.synchronize(dev)
@@ -1094,8 +1074,7 @@ def run_gpu(args, world, rank, local):
     stage_ms = np.zeros(len(STAGES))
     a = pipe._args(clip, t_attrs, t_uv, tex, g_attr, g_samp)
     timed = [
-        lambda: _native.check(L.pdr_render_bin(C.addressof(a), stream)),
-        lambda: _native.check(L.pdr_render_raster(C.addressof(a), stream)),
+        lambda: _native.check((L.pdr_render_direct if pipe.direct else L.pdr_render_forward)(C.addressof(a), stream)),
         lambda: _native.check(L.pdr_render_backward(C.addressof(a), stream)),
     ]
     for _ in range(reps):
@@ -1109,7 +1088,7 @@ def run_gpu(args, world, rank, local):
             stage_ms[i] += e0.elapsed_time(e1)
     stage_ms /= reps
     hbm, peak_kind = load_peaks()
-    sbytes = stage_bytes(w, T, V, entries)
+    sbytes = stage_bytes(w, T, V)
     dom = int(np.argmax(stage_ms))
     dom_name = STAGES[dom]
     achieved = sbytes[dom_name] / (stage_ms[dom] / 1e3) / 1e9
@@ -1180,16 +1159,15 @@ def run_gpu(args, world, rank, local):
             "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded displaced sphere, orbit cameras)",
             "config": {"workload": w["name"], "views": views, "resolution": [H, W], "triangles": int(T),
                        "vertices": int(V), "atlas": [w["atlas"], w["atlas"], w["channels"]],
-                       "attributes": w["attributes"], "tile_entries": entries,
-                       "tile": list(pipe.tile_config[:2]), "stage_triangles": pipe.tile_config[2],
-                       "autotune_forward_ms": {f"{a}x{b}/{k}": v for (a, b, k), v in tune.items()},
+                       "attributes": w["attributes"],
+                       "forward": "visibility buffer" if pipe.direct else f"tile lists {args.tile}",
                        "l2": "inputs larger than L2 (6.5 GB of per-view buffers per step)",
                        "parallelism": f"replicas x{world}"},
             "gpu_launches": pipe.kernels_per_step() * args.steps,
             "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": achieved, "peak": hbm,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / hbm,
-                         "traffic": recorded_traffic(dom_name, pipe.tile_config)
-                         if views == 64 and w["atlas"] == 4096 else None,
+                         "traffic": recorded_traffic(dom_name)
+                         if pipe.direct and views == 64 and w["atlas"] == 4096 else None,
                          "traffic_source_sha256": kernel_source_hash(dom_name),
                          "algorithmic_bytes": sbytes[dom_name], "ms": float(stage_ms[dom])},
             "stages_ms": {n: float(t) for n, t in zip(STAGES, stage_ms)},
@@ -1243,7 +1221,8 @@ def main():
     ap.add_argument("--skip-c4", action="store_true", help="omit the uneven multi-mesh batch leg")
     ap.add_argument("--skip-precond", action="store_true", help="omit the learned-preconditioner leg")
     ap.add_argument("--c4-meshes", type=int, default=None, help="override the C4 mesh count (small profiling cases)")
-    ap.add_argument("--tile", default=None, help="fused tile shape and stage depth, e.g. 16x8/128 (default: autotune)")
+    ap.add_argument("--tile", default=None, help="forward through tile lists of this shape and stage depth, e.g. 16x8/128 (default: visibility "
+                         "buffer)")
     ap.add_argument("--refine-steps", type=int, default=None, help="override the refine leg's step count (profiling)")
     args = ap.parse_args()
     if args.views:

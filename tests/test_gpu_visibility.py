@@ -131,3 +131,37 @@ def test_batch_in_groups_of_jobs():
             one, d = r.forward(m.clip[k], m.indices, (m.height, m.width))
             assert torch.equal(m.outputs["raster"][k].view(torch.int32), one.view(torch.int32)), k
             assert torch.equal(m.outputs["deriv"][k].view(torch.int32), d.view(torch.int32)), k
+
+
+@pytest.mark.parametrize("capture", [False, True])
+def test_pipeline_through_the_visibility_buffer(capture):
+    """RenderFwdBwd(direct=True) gives the images of the tile lists bit for bit and the same gradients up to the order
+    of their sums, as launches and as a replayed graph."""
+    from photara_drender_gb300.pipeline import RenderFwdBwd
+
+    rng = np.random.default_rng(3)
+    pos3, idx = S.icosphere(4)
+    mats, _ = S.orbit_cameras(3)
+    dev = torch.device("cuda", 0)
+    t = lambda a: torch.tensor(np.ascontiguousarray(a, dtype=np.float32), device=dev)  # noqa: E731
+    V, H, W = pos3.shape[0], 75, 101
+    args = [t(S.clip_positions(pos3, mats)), t(rng.uniform(size=(V, 3))), t(S.spherical_uv(pos3)),
+            t(rng.uniform(size=(64, 48, 4))), t(rng.normal(size=(3, H, W, 3))), t(rng.normal(size=(3, H, W, 4)))]
+    tidx = torch.tensor(idx.astype(np.int32), device=dev)
+    pipes = [RenderFwdBwd(pdr.Rasterizer(), tidx, V, 3, H, W, 3, (64, 48, 4), direct=d,
+                          viewports=[None, (5.0, -3.0, 90.0, 70.0), None]) for d in (False, True)]
+    pipes[0].step(*args)
+    if capture:
+        graph = pipes[1].capture(*args)
+        for k in ("raster", "sampled", "grad_clip", "grad_tex"):
+            getattr(pipes[1], k).fill_(9.0)
+        graph.replay()
+    else:
+        pipes[1].step(*args)
+    torch.cuda.synchronize()
+    for k in ("raster", "deriv", "attr_out", "uv", "sampled"):
+        assert torch.equal(*(getattr(p, k).view(torch.int32) for p in pipes)), k
+    for k in ("grad_clip", "grad_attr", "grad_uv_attr", "grad_tex"):
+        a, b = (getattr(p, k) for p in pipes)
+        assert float((a - b).abs().max()) <= 1e-5 * float(a.abs().max()), k
+    assert pipes[1].check_capacity() == 0 and pipes[1].autotune(*args[:4]) == {} and pipes[1].kernels_per_step() == 5
