@@ -23,8 +23,6 @@
 namespace photara_drender {
 namespace {
 
-constexpr std::uint32_t kTile = 16;
-
 void check(pdr_status st) {
     if (st == PDR_OK) return;
     const std::string msg = pdr_last_error();
@@ -148,7 +146,6 @@ public:
     cudaStream_t stream = nullptr;
     DeviceInfo info;
     std::mutex mutex;  // one dispatch at a time per context, as src/context_internal.hpp:101
-    std::uint64_t tile_capacity = 0;
 };
 
 Context::Context(const ContextOptions& options) : impl_(std::make_unique<Impl>(options)) {}
@@ -169,32 +166,27 @@ std::vector<DeviceInfo> Context::enumerate_devices() {
 
 namespace {
 
-// Bins and rasterizes `views` views of equal size; raster (and derivatives) stay on the device.
+// Rasterizes `views` views of equal size; raster (and derivatives) stay on the device.
 void rasterize_device(Context::Impl& ctx, const float* d_clip, std::uint32_t views, std::uint32_t V,
                       const std::uint32_t* d_idx, std::uint32_t T, std::uint32_t W, std::uint32_t H,
                       const float* d_viewports, std::uint32_t cull, float* d_raster, float* d_deriv) {
-    const std::uint64_t tiles = static_cast<std::uint64_t>((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile);
-    DeviceArray<std::uint32_t> offsets(tiles * views + 1);
-    DeviceArray<std::uint32_t> status(PDR_STATUS_WORDS);
-    std::uint64_t capacity = std::max<std::uint64_t>(ctx.tile_capacity, 2ull * T * views + 1024);
-    for (int attempt = 0; attempt < 3; ++attempt) {
-        DeviceArray<std::uint32_t> list(capacity);
-        const std::size_t ws_bytes = pdr_bin_tiles_workspace_bytes(views, T, W, H, capacity);
-        DeviceArray<unsigned char> ws(std::max<std::size_t>(ws_bytes, 1));
-        status.zero(ctx.stream);
-        check(pdr_bin_tiles(d_clip, views, V, d_idx, T, W, H, d_viewports, offsets.get(), list.get(), capacity,
-                            ws.get(), ws_bytes, status.get(), ctx.stream));
-        const auto st = status.download(ctx.stream);
-        if (st[PDR_STATUS_TILE_ENTRIES_HI] != 0) throw std::overflow_error("Tile triangle list exceeds backend limits");
-        if (!st[PDR_STATUS_TILE_OVERFLOW]) {
-            ctx.tile_capacity = std::max(ctx.tile_capacity, capacity);
-            check(pdr_rasterize_forward(d_clip, views, V, d_idx, T, W, H, d_viewports, cull, offsets.get(), list.get(),
-                                        capacity, d_raster, d_deriv, ctx.stream));
-            return;
-        }
-        capacity = st[PDR_STATUS_TILE_ENTRIES] + st[PDR_STATUS_TILE_ENTRIES] / 8 + 1024;
-    }
-    throw std::runtime_error("tile binning did not converge");
+    const std::size_t ws_bytes = pdr_render_direct_workspace_bytes(views, T, W, H);
+    DeviceArray<unsigned char> ws(std::max<std::size_t>(ws_bytes, 1));
+    pdr_render_args a{};
+    a.clip_positions = d_clip;
+    a.views = views;
+    a.vertex_count = V;
+    a.indices = d_idx;
+    a.triangle_count = T;
+    a.width = W;
+    a.height = H;
+    a.viewports = d_viewports;
+    a.cull_mode = cull;
+    a.workspace = ws.get();
+    a.workspace_bytes = ws_bytes;
+    a.raster = d_raster;
+    a.barycentric_derivatives = d_deriv;
+    check(pdr_render_direct(&a, ctx.stream));
 }
 
 }  // namespace
