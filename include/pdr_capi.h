@@ -251,6 +251,13 @@ typedef struct {
 PDR_API pdr_status pdr_refine_prepare_view(const float* image, uint32_t channel_count, const float* visibility_mask,
                                            const float* raster, uint64_t pixel_count, float* target, float* mask,
                                            void* stream);
+/* pdr_refine_prepare_view with the view's texture coordinates uv [P][2] (interpolate_forward of uv_attributes [V][2])
+ * and the sum of its mask, added in double to weight [PDR_REFINE_WEIGHT_PARTS], whose sum it is; all in one pass. */
+#define PDR_REFINE_WEIGHT_PARTS 64
+PDR_API pdr_status pdr_refine_prepare_view_uv(const float* image, uint32_t channel_count, const float* visibility_mask,
+                                              const float* raster, uint64_t pixel_count, const float* uv_attributes,
+                                              uint32_t vertex_count, const uint32_t* indices, uint32_t triangle_count,
+                                              float* target, float* mask, float* uv, double* weight, void* stream);
 /* One photometric dispatch set (all batch views of `step`) accumulating into gradient and loss[step]. */
 PDR_API pdr_status pdr_refine_photometric(const float* texture, uint32_t width, uint32_t height,
                                           const pdr_refine_view* views, uint32_t view_count,

@@ -91,6 +91,7 @@ _SIGNATURES = {
                                         _vp, _vp, _vp]),
     "pdr_interpolate_derivatives": (_i32, [_vp, _u32, _u32, _vp, _u32, _vp, _vp, _u32, _u64, _vp, _vp]),
     "pdr_refine_prepare_view": (_i32, [_vp, _u32, _vp, _vp, _u64, _vp, _vp, _vp]),
+    "pdr_refine_prepare_view_uv": (_i32, [_vp, _u32, _vp, _vp, _u64, _vp, _u32, _vp, _u32, _vp, _vp, _vp, _vp, _vp]),
     "pdr_refine_photometric": (_i32, [_vp, _u32, _u32, _vp, _u32, _u64, _u32, _u32, C.c_float, C.c_float, _vp, _vp,
                                       _vp]),
     "pdr_calibrate_reductions": (_i32, [_vp, _u64, _u64, _u32, _vp]),

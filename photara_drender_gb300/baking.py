@@ -451,19 +451,20 @@ class TextureBaker:
         clip = self._transform(pos, torch.from_numpy(mats).to(ctx.device))
         rasters = self._rasters(clip, idx, sizes, vps)
         table = (RefineViewC * n)()
-        keep, weights = [], []
+        keep = []
+        weights = torch.zeros((n, 64), dtype=torch.float64, device=ctx.device)  # PDR_REFINE_WEIGHT_PARTS
         for k in range(n):
             P = sizes[k][0] * sizes[k][1]
-            uvk = self.rasterizer.interpolate_forward(uvt, _CheckedIndices(idx, V), rasters[k])
+            uvk = torch.empty((P, 2), dtype=torch.float32, device=ctx.device)
             tgt = torch.empty((P, 3), dtype=torch.float32, device=ctx.device)
             msk = torch.empty((P,), dtype=torch.float32, device=ctx.device)
-            _native.call("pdr_refine_prepare_view", _ptr(imgs[k]), imgs[k].shape[2], _ptr(masks[k]), _ptr(rasters[k]),
-                         P, _ptr(tgt), _ptr(msk), ctx.stream())
+            _native.call("pdr_refine_prepare_view_uv", _ptr(imgs[k]), imgs[k].shape[2], _ptr(masks[k]), _ptr(rasters[k]),
+                         P, _ptr(uvt), V, _ptr(idx), idx.shape[0], _ptr(tgt), _ptr(msk), _ptr(uvk), _ptr(weights[k]),
+                         ctx.stream())
             keep += [uvk, tgt, msk]
-            weights.append(msk.sum(dtype=torch.float64))
             table[k].uv, table[k].target, table[k].mask, table[k].pixel_count = (uvk.data_ptr(), tgt.data_ptr(),
                                                                                  msk.data_ptr(), P)
-        weights = torch.stack(weights).tolist()  # one wait for all views
+        weights = weights.cpu().numpy().sum(1).tolist()  # one wait for all views
         table_dev = torch.frombuffer(bytearray(bytes(table)), dtype=torch.uint8).to(ctx.device)
         max_pixels = max(s[0] * s[1] for s in sizes)
         torch.cuda.synchronize(ctx.device)

@@ -263,6 +263,20 @@ pdr_status pdr_refine_prepare_view(const float* image, uint32_t C, const float* 
                        "refine_prepare_view");
 }
 
+pdr_status pdr_refine_prepare_view_uv(const float* image, uint32_t C, const float* mask, const float* raster, uint64_t P,
+                                      const float* uv_attributes, uint32_t V, const uint32_t* idx, uint32_t T,
+                                      float* target, float* out_mask, float* uv, double* weight, void* stream) {
+    if (!image || !raster || !target || !out_mask || P == 0 || (C != 3 && C != 4))
+        return fail(PDR_INVALID_ARGUMENT, "texture refinement images must contain RGB or RGBA data");
+    if (!uv_attributes || !idx || !uv || !weight || V == 0 || T == 0)
+        return fail(PDR_INVALID_ARGUMENT, "texture refinement needs uv, indices and outputs");
+    if (!aligned(raster, 16) || !aligned(uv, 8) || !aligned(weight, 8))
+        return fail(PDR_INVALID_ARGUMENT, "raster must be 16-byte aligned, uv and weights 8-byte");
+    return cuda_status(launch_prepare_view(image, C, mask, raster, P, target, out_mask, (cudaStream_t)stream,
+                                           uv_attributes, V, idx, T, uv, weight),
+                       "refine_prepare_view_uv");
+}
+
 pdr_status pdr_refine_photometric(const float* tex, uint32_t W, uint32_t H, const pdr_refine_view* views, uint32_t nviews,
                                   uint64_t max_pixels, uint32_t step, uint32_t batch, float eps, float norm, float* grad,
                                   float* loss, void* stream) {

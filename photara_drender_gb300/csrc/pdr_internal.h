@@ -110,7 +110,9 @@ cudaError_t launch_transform_positions(const float* pos3, uint32_t V, const floa
                                        cudaStream_t stream);
 cudaError_t launch_atlas_clip(const float* uv, uint32_t V, float* clip, cudaStream_t stream);
 cudaError_t launch_prepare_view(const float* image, uint32_t C, const float* ext_mask, const float* raster, size_t P,
-                                float* target, float* mask, cudaStream_t stream);
+                                float* target, float* mask, cudaStream_t stream,
+                                const float* uv_attributes = nullptr, uint32_t V = 0, const uint32_t* idx = nullptr,
+                                uint32_t T = 0, float* uv = nullptr, double* weight = nullptr);
 cudaError_t launch_photometric(const float* tex, uint32_t tw, uint32_t th, const pdr_refine_view* views,
                                uint32_t nviews, uint64_t max_pixels, uint32_t step, uint32_t batch, float eps,
                                float norm, float* grad, float* loss, cudaStream_t stream);

@@ -24,24 +24,67 @@ namespace {
 
 constexpr int kPhotoThreads = 256;
 
-// texture_refiner.cpp:228-242: target RGB, mask = clamp(external mask) on covered pixels.
-__global__ void prepare_view_kernel(const float* __restrict__ image, uint32_t C, const float* __restrict__ ext_mask,
-                                    const float4* __restrict__ raster, size_t P, float* __restrict__ target,
-                                    float* __restrict__ mask) {
+// What a view's coordinates and weight come from.
+struct ViewUv {
+    const float* attributes;  // [V][2], at any address
+    const uint3* idx;
+    uint32_t V, T;
+    float2* uv;      // [P]
+    double* weight;  // [PDR_REFINE_WEIGHT_PARTS]: their sum is the sum of the mask
+};
+
+// texture_refiner.cpp:228-242: target RGB, mask = clamp(external mask) on covered pixels; with kUv also the texture
+// coordinates (interpolate_forward_kernel's arithmetic) and the mask's sum, for which the raster and the mask were read
+// twice more: a view of 320 x 240 in one launch of 3 us instead of four of 33, most of it a reduction on one SM.
+template <bool kUv>
+__global__ void __launch_bounds__(256)
+prepare_view_kernel(const float* __restrict__ image, uint32_t C, const float* __restrict__ ext_mask,
+                    const float4* __restrict__ raster, size_t P, float* __restrict__ target, float* __restrict__ mask,
+                    ViewUv u) {
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    target[p * 3] = image[p * C];
-    target[p * 3 + 1] = image[p * C + 1];
-    target[p * 3 + 2] = image[p * C + 2];
     float m = 0.0f;
-    if (raster[p].w != 0.0f) {
-        m = 1.0f;
-        if (ext_mask) {
-            const float e = ext_mask[p];
-            m = e < 0.0f ? 0.0f : (1.0f < e ? 1.0f : e);  // std::clamp
+    if (p < P) {
+        const float4 r = raster[p];
+        target[p * 3] = image[p * C];
+        target[p * 3 + 1] = image[p * C + 1];
+        target[p * 3 + 2] = image[p * C + 2];
+        if (r.w != 0.0f) {
+            m = 1.0f;
+            if (ext_mask) {
+                const float e = ext_mask[p];
+                m = e < 0.0f ? 0.0f : (1.0f < e ? 1.0f : e);  // std::clamp
+            }
+        }
+        mask[p] = m;
+        if (kUv) {
+            float2 o = make_float2(0.0f, 0.0f);
+            const uint32_t id = raster_id(r.w);
+            if (id != 0 && id <= u.T) {
+                const uint3 v = u.idx[id - 1];
+                if (v.x < u.V && v.y < u.V && v.z < u.V) {
+                    const float* a = u.attributes + (size_t)v.x * 2;
+                    const float* b = u.attributes + (size_t)v.y * 2;
+                    const float* c = u.attributes + (size_t)v.z * 2;
+                    const float w = 1.0f - r.x - r.y;
+                    o.x = r.x * __ldg(a) + r.y * __ldg(b) + w * __ldg(c);
+                    o.y = r.x * __ldg(a + 1) + r.y * __ldg(b + 1) + w * __ldg(c + 1);
+                }
+            }
+            u.uv[p] = o;
         }
     }
-    mask[p] = m;
+    if (kUv) {
+        __shared__ double sums[8];
+        double s = m;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31u) == 0) sums[threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < 8; ++k) s += sums[k];
+            if (s != 0.0) atomicAdd(u.weight + blockIdx.x % PDR_REFINE_WEIGHT_PARTS, s);
+        }
+    }
 }
 
 struct ClampTaps {
@@ -436,10 +479,13 @@ cudaError_t launch_adam_tv(const float* tex_in, float* tex_out, float* grad, flo
 }
 
 cudaError_t launch_prepare_view(const float* image, uint32_t C, const float* ext_mask, const float* raster, size_t P,
-                                float* target, float* mask, cudaStream_t stream) {
-    prepare_view_kernel<<<(unsigned)((P + 255) / 256), 256, 0, stream>>>(image, C, ext_mask,
-                                                                         reinterpret_cast<const float4*>(raster), P,
-                                                                         target, mask);
+                                float* target, float* mask, cudaStream_t stream, const float* uv_attributes, uint32_t V,
+                                const uint32_t* idx, uint32_t T, float* uv, double* weight) {
+    const ViewUv u{uv_attributes, reinterpret_cast<const uint3*>(idx), V, T,
+                   reinterpret_cast<float2*>(uv), weight};
+    const auto kernel = uv ? prepare_view_kernel<true> : prepare_view_kernel<false>;
+    kernel<<<(unsigned)((P + 255) / 256), 256, 0, stream>>>(image, C, ext_mask, reinterpret_cast<const float4*>(raster), P,
+                                                            target, mask, u);
     return cudaGetLastError();
 }
 

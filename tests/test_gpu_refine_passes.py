@@ -132,3 +132,33 @@ def test_photometric_rounds(pixels, batch):
     bound = size * (5e-6 + (count[:, None] + 16) * 2.0 ** -24)
     assert (np.abs(got[:, :3] - grad) <= bound).all() and not got[:, 3].any()
     assert abs(t_loss[0].item() - loss) <= 1e-5 * loss and not t_loss[1:].any()
+
+
+@pytest.mark.parametrize("pixels", [1, 255, 257, 70001])
+@pytest.mark.parametrize("channels,external", [(3, True), (4, False)])
+def test_prepare_view_in_one_pass(pixels, channels, external):
+    """Target, mask, coordinates and weight of a view against the separate calls, bit for bit (the weight: sums of
+    2^-10 steps, exact in any order), for coordinates at an address that is no multiple of 8."""
+    baker = TextureBaker(0)
+    dev, s = baker.context.device, baker.context.stream()
+    rng = np.random.default_rng(pixels)
+    V, T = 50, 30
+    image = torch.tensor(rng.uniform(size=(pixels, channels)).astype(np.float32), device=dev)
+    ext = torch.tensor((rng.integers(-200, 1400, pixels) / 1024).astype(np.float32), device=dev) if external else None
+    raster = rng.uniform(size=(pixels, 4)).astype(np.float32)
+    raster[:, 3] = rng.integers(0, T + 3, pixels)  # some ids past the last triangle
+    raster = torch.tensor(raster, device=dev)
+    idx = torch.tensor(rng.integers(0, V, (T, 3)).astype(np.int32), device=dev)
+    uv = torch.rand(2 * V + 1, device=dev)[1:].view(V, 2)
+    new = lambda *shape: torch.full(shape, 7.0, device=dev)  # noqa: E731
+    t0, m0, u0 = new(pixels, 3), new(pixels), new(pixels, 2)
+    t1, m1, u1 = new(pixels, 3), new(pixels), new(pixels, 2)
+    weight = torch.zeros(64, dtype=torch.float64, device=dev)
+    e = None if ext is None else _ptr(ext)
+    _native.call("pdr_refine_prepare_view", _ptr(image), channels, e, _ptr(raster), pixels, _ptr(t0), _ptr(m0), s)
+    _native.call("pdr_interpolate_forward", _ptr(uv), 0, V, 2, _ptr(idx), T, _ptr(raster), 1, pixels, _ptr(u0), s)
+    _native.call("pdr_refine_prepare_view_uv", _ptr(image), channels, e, _ptr(raster), pixels, _ptr(uv), V, _ptr(idx), T,
+                 _ptr(t1), _ptr(m1), _ptr(u1), _ptr(weight), s)
+    for a, b in ((t0, t1), (m0, m1), (u0, u1)):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert float(weight.sum()) == float(m0.double().sum())
