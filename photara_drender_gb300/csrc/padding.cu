@@ -314,10 +314,11 @@ __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restric
 //    value by its four earlier neighbours' values (induction in raster order). So tiles may be swept in any
 //    order, with whatever their neighbours hold, and swept again, as long as in the end every texel
 //    satisfies its relaxation. Sweeping a tile satisfies all texels inside it; afterwards only the texels on
-//    its first row, first and last column look at other tiles, and a tile whose neighbours changed checks
-//    just those (tile_settled) before it is swept again. A nearest source is mostly close, so most tiles
-//    are final after one or two sweeps; the loop ends after a pass in which none changed. A value crosses at
-//    most two tile borders per row and one per 64 columns on its way, which bounds the passes.
+//    its first row, first and last column look at other tiles, and the next pass checks just those
+//    (tile_settled), where a tile they look at changed, before it sweeps a tile again. A nearest source is
+//    mostly close, so most tiles are final after one or two sweeps; the loop ends after a pass in which none
+//    changed. Some passes shift the tiling by half a tile: a source's region that follows a border, changing
+//    sides every few rows, takes a pass per change in one tiling and lies inside a tile of the other.
 // 2. With sides <= 4384 a real offset (squared length <= 2 * 4384^2) is always shorter than one inherited from
 //    a texel without source (components >= 12000 - 4384), no candidate reaches the +-16384 clamp, and the
 //    sequential relaxations equal "the first of [own, left, up, up-left, up-right] with the smallest squared
@@ -329,16 +330,24 @@ __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restric
 // candidate's squared length is (sx - x)^2 + (sy - y)^2 with the second term fixed along a row.
 //
 // What bounds it: the latency of a tile's wavefront (64 + 3 * 31 steps of about 50 instructions, 10 us) times
-// the passes: a hole of 300 texels takes about 25 passes a sweep, gutters and small holes 5 to 8. One
-// warp-wide wavefront per 32 rows of the whole atlas, each band waiting for the one above, was a chain of
-// W + 2H dependent steps whatever the atlas held. Whole padding call, 4096 x 4096 with 300-texel holes:
-// 6.91 -> 1.93 ms; 1400 x 1000, 8-texel gutters: 1.91 -> 0.42 ms. Tiles of 64 columns: 32 would save a third
-// of a pass and need up to twice the passes. Above kTileMaxSide fact 2 does not hold: pad_sweep_kernel.
+// the passes: 300-texel holes take about 7 and 20, gutters and small holes 5. One warp-wide wavefront per 32 rows
+// of the whole atlas, each band waiting for the one above, was a chain of W + 2H dependent steps whatever the
+// atlas held: 6.3 ms at 4096 x 4096, 1.6 at 1400 x 1000. Both sweeps now, in us (in parentheses without shifted
+// passes): 4096 x 4096 with 300-texel holes 698 (1421), rectangular charts over 38% of it 1752 (1489), round ones
+// 3098 (15792), one source in 50000 2362 (3831), all sources in the first or last corner 2924 or 4922; 1400 x 1000
+// with 8-texel gutters 115 (185). Tiles of 64 columns: 32 would save a third of a pass and need up to twice the
+// passes; strips of 2 to 8 tiles swept one after the other by a warp were slower (1421 -> 1972 to 2874 us). Above
+// kTileMaxSide fact 2 does not hold: pad_sweep_kernel.
 constexpr int32_t kTileMaxSide = 4384;
 constexpr int kPadTileW = 64;
 constexpr int kPadPitch = kPadTileW + 1;  // (row r, column t - 2r): odd pitch - 2, no bank conflicts
 constexpr int kPadRows = 8;               // rows of a tile loaded together: 16 loads of a lane in flight
 constexpr int kPadWarps = 4;              // 34 KB of shared memory: six CTAs per SM
+// Every how many passes the tiling is shifted. A value crosses a tile a pass in one tiling, half a tile in a shifted pass,
+// so not every second one: the forward sweep mostly carries values into empty texels, the reverse sweep mostly corrects
+// them (every 4 and 2 passes 695 us for the holes, but 6453 with all sources in the last corner; 3 and 3: 737, 4916).
+template <bool kBack>
+constexpr uint32_t kShiftEvery = kBack ? 3 : 8;
 constexpr uint32_t kPadMaxPasses = 1u << 16;
 constexpr uint32_t kNoSource = 0x75307530u;  // (30000, 30000): farther from any texel than a real source
 static_assert(kPadTileW == 64, "a lane moves two columns of a tile row");
@@ -347,11 +356,11 @@ struct TileSweeps {
     const uint32_t* src_bits;
     uint32_t* forward;   // [H][W] source positions after the forward sweep
     uint32_t* field;     // [H][W] after the reverse sweep
-    uint8_t* changed;    // [2][tiles]: tile changed in the pass before / in this pass
+    uint8_t* changed;    // [2][(tiles_x + 1) * (tiles_y + 1)]: tile changed in the last even / odd pass
     uint32_t* control;   // [2] failure flag, [8] barrier arrivals, [12..15] "a tile changed" per pass & 3
     uint32_t* status;
     uint32_t words_per_row;
-    int32_t W, H, tiles_x, tiles;
+    int32_t W, H, tiles_x, tiles_y;  // of the even passes
 };
 
 // All CTAs of the (cooperative) grid meet; false when the wait gave up or another CTA failed.
@@ -434,14 +443,15 @@ struct SweepSpace {
     }
 };
 
-// Whether the texels of a swept tile that look at other tiles still satisfy their relaxation.
+// Whether the texels of a tile on the other tiling's tile borders still satisfy their relaxation: its row `row` and the
+// columns `column - 1` and `column`, clamped to the tile.
 template <bool kBack>
 __device__ __forceinline__ bool tile_settled(const SweepSpace<kBack>& sp, int32_t X0, int32_t Y0, int32_t tw,
-                                             int32_t rows) {
-    // the first row (two texels a lane), the first and the last column: all loads in flight together
-    const int32_t lane = threadIdx.x & 31, r = min(lane, rows - 1);
-    const bool a = sp.settled(X0 + min(lane, tw - 1), Y0), b = sp.settled(X0 + min(lane + 32, tw - 1), Y0);
-    const bool c = sp.settled(X0, Y0 + r), e = sp.settled(X0 + tw - 1, Y0 + r);
+                                             int32_t rows, int32_t row, int32_t column0, int32_t column1) {
+    // two texels a lane of the row, one of each column: all loads in flight together
+    const int32_t lane = threadIdx.x & 31, r = Y0 + min(lane, rows - 1), y = min(max(row, Y0), Y0 + rows - 1);
+    const bool a = sp.settled(X0 + min(lane, tw - 1), y), b = sp.settled(X0 + min(lane + 32, tw - 1), y);
+    const bool c = sp.settled(min(max(column0, X0), X0 + tw - 1), r), e = sp.settled(min(max(column1, X0), X0 + tw - 1), r);
     return __all_sync(0xFFFFFFFFu, a & b & c & e);
 }
 
@@ -548,23 +558,43 @@ __device__ bool sweep_tiles(const TileSweeps& s, uint32_t& phase, uint32_t* buf,
     const SweepSpace<kBack> sp(s);
     const int32_t lane = threadIdx.x & 31;
     const int32_t warp = blockIdx.x * kPadWarps + (threadIdx.x >> 5), warps = gridDim.x * kPadWarps;
-    const int32_t tiles_y = s.tiles / s.tiles_x;
+    const size_t slot = (size_t)(s.tiles_x + 1) * (s.tiles_y + 1);
     for (uint32_t pass = 0; pass < kPadMaxPasses; ++pass) {
-        const uint8_t* before = s.changed + (size_t)((pass & 1u) ^ 1u) * s.tiles;
-        uint8_t* now = s.changed + (size_t)(pass & 1u) * s.tiles;
+        // tiles start at multiples of 64 x 32, in shifted passes half a tile earlier (clipped to the atlas)
+        const int32_t shifted = pass % kShiftEvery<kBack> == kShiftEvery<kBack> - 1u;
+        const int32_t was_shifted = pass % kShiftEvery<kBack> == 0u && pass > 0;  // the pass before
+        const int32_t shift_x = shifted * (kPadTileW / 2), shift_y = shifted * 16;
+        const int32_t nx = (s.W + shift_x + kPadTileW - 1) / kPadTileW, ny = (s.H + shift_y + 31) / 32;
+        const int32_t other_x = (s.W + was_shifted * (kPadTileW / 2) + kPadTileW - 1) / kPadTileW;
+        const int32_t other_y = (s.H + was_shifted * 16 + 31) / 32;
+        const uint8_t* before = s.changed + slot * ((pass & 1u) ^ 1u);
+        uint8_t* now = s.changed + slot * (pass & 1u);
         uint32_t* any = s.control + 12 + (pass & 3u);
         // the slot of pass + 2 was last read two barriers ago
         if (blockIdx.x == 0 && threadIdx.x == 0) s.control[12 + ((pass + 2u) & 3u)] = 0u;
-        for (int32_t tile = warp; tile < s.tiles; tile += warps) {
-            const int32_t ty = tile / s.tiles_x, tx = tile - ty * s.tiles_x;
-            const int32_t X0 = tx * kPadTileW, Y0 = ty * 32;
-            const int32_t tw = min(kPadTileW, s.W - X0), rows = min(32, s.H - Y0);
+        for (int32_t tile = warp; tile < nx * ny; tile += warps) {
+            const int32_t ty = tile / nx, tx = tile - ty * nx;
+            const int32_t left = tx * kPadTileW - shift_x, upper = ty * 32 - shift_y;
+            const int32_t X0 = max(left, 0), Y0 = max(upper, 0);
+            const int32_t tw = min(left + kPadTileW, s.W) - X0, rows = min(upper + 32, s.H) - Y0;
             bool todo = pass == 0;
-            if (pass > 0) {  // a neighbour this tile looks at changed: left, right, and the three above
-                const int32_t nx = tx + (lane == 0 || lane == 2 ? -1 : lane == 3 ? 0 : 1), ny = ty - (lane >= 2 ? 1 : 0);
-                const bool dirty = lane < 5 && nx >= 0 && nx < s.tiles_x && ny >= 0 && ny < tiles_y &&
-                                   __ldcg(before + ny * s.tiles_x + nx) != 0;
-                todo = __any_sync(0xFFFFFFFFu, dirty) && !tile_settled(sp, X0, Y0, tw, rows);
+            if (pass > 0) {
+                // a tile of the pass before changed: of the four that this one lies over, or, in the same tiling, of
+                // those it looks at, left, right and the three above
+                int32_t ox = tx - shifted + (lane & 1), oy = ty - shifted + (lane >> 1), count = 4;
+                if (shifted == was_shifted) {
+                    ox = tx + (lane == 0 || lane == 2 ? -1 : lane == 3 ? 0 : 1);
+                    oy = ty - (lane >= 2 ? 1 : 0);
+                    count = 5;
+                }
+                const bool dirty = lane < count && ox >= 0 && ox < other_x && oy >= 0 && oy < other_y &&
+                                   __ldcg(before + oy * other_x + ox) != 0;
+                todo = __any_sync(0xFFFFFFFFu, dirty);
+                if (todo) {
+                    const bool same = shifted == was_shifted;
+                    todo = !tile_settled(sp, X0, Y0, tw, rows, same ? Y0 : upper + 16,
+                                         same ? X0 + tw - 1 : left + kPadTileW / 2 - 1, same ? X0 : left + kPadTileW / 2);
+                }
             }
             const bool changed = todo && sweep_tile(sp, X0, Y0, tw, rows, pass == 0, buf, top);
             if (lane == 0) {
@@ -1040,12 +1070,12 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
         T.W = (int32_t)width;
         T.H = (int32_t)height;
         T.tiles_x = (int32_t)((width + kPadTileW - 1) / kPadTileW);
-        T.tiles = T.tiles_x * (int32_t)bands;
+        T.tiles_y = (int32_t)bands;
         // every CTA resident (they meet at barriers): a cooperative launch of at most what the device holds
         int per_sm = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pad_tiles_kernel, 32 * kPadWarps, 0);
         if (e) return set_cuda_error(e, "pdr_pad_texture_atlas");
-        const int32_t want = (T.tiles + kPadWarps - 1) / kPadWarps, most = per_sm * num_sms();
+        const int32_t want = (T.tiles_x * T.tiles_y + kPadWarps - 1) / kPadWarps, most = per_sm * num_sms();
         void* args[] = {&T};
         e = most > 0 ? cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(pad_tiles_kernel),
                                                    dim3((unsigned)(want < most ? want : most)), dim3(32 * kPadWarps), args,

@@ -202,3 +202,22 @@ def test_padding_tiles_sparse_sources_across_tiles(h, w):
         c, f, st = gpu_pad(color, valid, 50, cov, True)
         oc, of, ost = api.pad_texture_atlas(color, valid, 50, coverage_mask=cov, fill_unobserved=True)
         assert tuple(st) == ost and same_bits(c, oc) and same_bits(f, of), (h, w, sources)
+
+
+@pytest.mark.parametrize("h,w,charts", [(257, 300, 1), (330, 517, 2), (1024, 700, 3)])
+@pytest.mark.parametrize("flip", [False, True])
+def test_padding_round_charts(h, w, charts, flip):
+    """Curved outlines and sources in one corner: values that change tiles every few rows, and values that cross the
+    whole atlas, through even and shifted tilings."""
+    y, x = np.meshgrid(np.arange(h), np.arange(w), indexing="ij")
+    u, v = (x / w * charts) % 1 - 0.5, (y / h * charts) % 1 - 0.5
+    valid = (u * u + v * v < 0.13) if charts > 1 else (x < 20) & (y < 9 + x // 3)
+    if flip:
+        valid = valid[::-1, ::-1]
+    rng = np.random.default_rng(h + w)
+    color = rng.uniform(size=(h, w, 4)).astype(np.float32)
+    valid = np.ascontiguousarray(valid).astype(np.float32)
+    cov = (rng.random((h, w)) < 0.9).astype(np.float32)
+    c, f, st = gpu_pad(color, valid, 3, cov, True)
+    oc, of, ost = api.pad_texture_atlas(color, valid, 3, coverage_mask=cov, fill_unobserved=True)
+    assert tuple(st) == ost and same_bits(c, oc) and same_bits(f, of)
