@@ -878,6 +878,8 @@ KERNEL_SOURCES = {
 }
 # stage -> (sha256 of its sources, bytes)
 KERNEL_TRAFFIC = {
+    "visibility+shade": ("2b43e45df0e74c7b", 7327700000),
+    "render_backward": ("8200dc38ef29c163", 4745600000),
 }
 
 

@@ -2,12 +2,10 @@
 // many views (the chain python/photara_drender/atlas.py:36-62 render_textured_mesh runs as three
 // autograd functions, each a separate synchronous call in the reference).
 //
-// Forward: tile binning + one raster launch whose epilogue interpolates and samples for the winner.
-// Backward: one thread per pixel runs, in the reference's order and arithmetic, texture_grad_texture
-// (double-exact weights, vector atomics), texture_grad_uv, interpolate_grad_attributes /
-// interpolate_grad_raster for both attribute sets, and rasterize_backward for the summed raster
-// gradient. Per-vertex gradients are summed over each run of adjacent pixels of a warp that hit the
-// same triangle (warp shuffles), then the run's last lane adds them to global memory with vector
+// Forward: a visibility buffer and one shading pass (pdr_render_direct), or tile binning and one raster launch whose
+// epilogue interpolates and samples for the winner (pdr_render_forward).
+// Backward: one thread per pixel (render_bwd_tile.cuh), vertex gradients summed per warp and triangle in shared
+// memory before they are added to global memory with 16-byte
 // reductions. Intermediate grad_uv / grad_raster never leave registers. With sample_differences the
 // forward keeps the texel differences of each covered pixel's sample, so the backward reads 32 bytes
 // per pixel instead of gathering four texels again.
