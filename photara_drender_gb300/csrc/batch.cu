@@ -1,11 +1,11 @@
 // Uneven multi-mesh batches: every (mesh, view) of a batch is one job, and a batch runs as one
-// binning pass, one raster launch over the tiles of all jobs and one adjoint launch, however the
-// meshes differ in triangle count, view count, resolution and texture size. No counterpart in the
+// visibility pass, one shading launch over the tiles of all jobs (from tile lists: one binning pass and one raster
+// launch) and one adjoint launch, however the meshes differ in triangle count, view count, resolution and texture size. No counterpart in the
 // reference (it renders one mesh per call).
 //
 // The host writes a job table into the workspace: per job the view's clip positions, viewport and
 // image pointers, and three prefix sums (triangles, forward tiles, backward 16x8 tiles). A CTA or
-// thread finds its job by binary search over the matching prefix. Forward tiles have the batch's tile
+// thread finds its job by binary search over the matching prefix. Tiles of the tile lists have the batch's tile
 // shape (TW x TH pixels) and stage CHUNK triangles per pass; both come from the autotuner and change
 // only the work distribution: outputs are bit-identical for every shape (the tile routine does not
 // depend on the order or grouping of a tile's triangles).
