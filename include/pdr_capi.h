@@ -283,8 +283,8 @@ PDR_API pdr_status pdr_refine_schedule(const pdr_refine_options* options, uint32
  * + Adam steps with the cosine learning rate, then (when pair_count > 0) the seam polish with reset
  * moments. view_valid_weights is a host array of the views' valid weights (double, as the reference
  * keeps them); texture is updated in place; gradient/moment buffers are overwritten;
- * loss_history has steps + seam steps floats. With use_graph != 0 the sequence is recorded once
- * into a CUDA graph and launched as a single unit. */
+ * loss_history has steps + seam steps floats. With use_graph != 0 a sequence of more than 512
+ * launches is recorded once into a CUDA graph and launched as a single unit. */
 PDR_API pdr_status pdr_refine_run(const pdr_refine_options* options, const pdr_refine_view* views, uint32_t view_count,
                                   const double* view_valid_weights, uint64_t max_view_pixels,
                                   const float* seam_uv_pairs, uint32_t pair_count, const uint8_t* tv_valid,

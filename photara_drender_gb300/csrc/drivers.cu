@@ -192,6 +192,19 @@ pdr_status capture_graph(pdr_refine_graph* out, Enqueue&& enqueue) {
     return PDR_OK;
 }
 
+// A run that is launched once gains nothing from being recorded first: its launches overlap (launch_step in refine.cu),
+// a graph's kernels did not. 60 steps on a 512 x 512 atlas 1787 us recorded, 1515 launched. Up to 512 launches, half of
+// what a stream takes before a launch waits for the device, so the call returns as early as with a graph.
+bool launches_suffice(const pdr_refine_options* o, uint32_t npairs, cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const uint64_t launches = 3ull * o->steps + (npairs ? 2ull * o->seam_polish_steps : 0ull);
+    return capture == cudaStreamCaptureStatusNone && launches <= 512;
+}
+
 bool precond_params_ok(const float* params, const uint16_t* wbf) {
     return params && wbf && aligned(wbf, 16) && aligned(params, 4);
 }
@@ -328,7 +341,7 @@ pdr_status pdr_refine_run(const pdr_refine_options* o, const pdr_refine_view* vi
                           float* loss, int32_t use_graph, void* stream) {
     pdr_status st = check_refine_run(o, views, nviews, valid_weights, max_pixels, pairs, npairs, tex, grad, m1, m2, loss);
     if (st) return st;
-    if (!use_graph)
+    if (!use_graph || launches_suffice(o, npairs, (cudaStream_t)stream))
         return enqueue_refine(o, views, nviews, valid_weights, max_pixels, pairs, npairs, tv_valid, tv_chart, tex, grad,
                               m1, m2, loss, (cudaStream_t)stream);
     pdr_refine_graph g = nullptr;

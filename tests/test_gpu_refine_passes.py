@@ -162,3 +162,51 @@ def test_prepare_view_in_one_pass(pixels, channels, external):
     for a, b in ((t0, t1), (m0, m1), (u0, u1)):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
     assert float(weight.sum()) == float(m0.double().sum())
+
+
+@pytest.mark.parametrize("shape,steps,tv", [((256, 512), 120, False), ((256, 512), 120, True), ((32, 64), 160, True),
+                                            ((1024, 512), 40, False)])
+def test_overlapped_launches_read_final_values(shape, steps, tv):
+    """Refinement steps launched while their predecessors run, against the same steps recorded in a graph, bit for bit.
+    Every pixel samples one texel's centre (exact: sides are powers of two), and no two of a step the same one, so each
+    gradient value is one term and zeros, whatever the order; its texels lie on lines that other CTAs have just written."""
+    baker = TextureBaker(0)
+    dev, s = baker.context.device, baker.context.stream()
+    h, w = shape
+    N = h * w
+    rng = np.random.default_rng(h + steps)
+    views, keep = (RefineViewC * 2)(), []
+    for k in range(2):
+        pick = rng.permutation(N)
+        uv = np.stack([(pick % w + 0.5) / w, (pick // w + 0.5) / h], 1)
+        t = [torch.tensor(x.astype(np.float32), device=dev) for x in (uv, rng.uniform(size=(N, 3)), rng.uniform(size=N))]
+        keep.append(t)
+        views[k].uv, views[k].target, views[k].mask = (x.data_ptr() for x in t)
+        views[k].pixel_count = N
+    vd = torch.frombuffer(bytearray(bytes(views)), dtype=torch.uint8).to(dev)
+    valid = torch.tensor((rng.random((h, w)) < 0.8).astype(np.uint8), device=dev)
+    weight = (C.c_double * 2)(N, N)
+    o = RefineOptionsC(width=w, height=h, steps=steps, batch_size=1, learning_rate=0.02, minimum_learning_rate=0.01,
+                       photometric_epsilon=1e-3, adam_beta1=0.9, adam_beta2=0.999, adam_epsilon=1e-8, clamp_min=0.0,
+                       clamp_max=1.0, seam_polish_steps=0, seam_learning_rate=1e-3, seam_epsilon=1e-4,
+                       tv_scale=1e-6 if tv else 0.0, tv_epsilon=1e-4)
+    outs = []
+    for mode in ("launches", "graph", "launches"):
+        tex, scratch = torch.full((h, w, 3), 0.5, device=dev), torch.empty((h, w, 3), device=dev)
+        grad, m, v = torch.empty((h, w, 4), device=dev), torch.empty_like(tex), torch.empty_like(tex)
+        loss = torch.empty(steps, device=dev)
+        o.texture_scratch = scratch.data_ptr() if tv else None
+        args = (C.byref(o), _ptr(vd), 2, C.cast(weight, C.c_void_p), N, None, 0, _ptr(valid), None, _ptr(tex), _ptr(grad),
+                _ptr(m), _ptr(v), _ptr(loss))
+        if mode == "graph":
+            g = C.c_void_p()
+            _native.call("pdr_refine_graph_create", C.byref(g), *args, s)
+            _native.call("pdr_refine_graph_launch", g, s)
+            torch.cuda.synchronize()
+            _native.call("pdr_refine_graph_destroy", g)
+        else:
+            _native.call("pdr_refine_run", *args, 1, s)
+        outs.append([t.cpu().numpy() for t in (tex, m, v)])
+    for other in outs[1:]:
+        for a, b in zip(outs[0], other):
+            assert same_bits(a, b)
