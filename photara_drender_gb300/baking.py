@@ -4,7 +4,7 @@ GB300 C ABI.
 
 bake(): atlas G-buffer raster, shadow rasters of every view in batched launches, and one projection
 launch over all views (src/texture_baker.cpp:156-361). refine_texture(): per-view raster + uv caches,
-then the whole Adam loop recorded as one CUDA graph (src/texture_refiner.cpp:174-454).
+then the whole Adam loop recorded as one CUDA graph when it is long (src/texture_refiner.cpp:174-454).
 """
 from __future__ import annotations
 

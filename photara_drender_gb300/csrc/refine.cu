@@ -1,6 +1,6 @@
 // Texture-atlas refinement: view preparation, masked Charbonnier photometric gradient, seam
 // gradient, chart-aware total variation and the dense Adam update, plus the native driver that
-// records the whole optimisation as one CUDA graph.
+// launches the whole optimisation or records it as one CUDA graph.
 //
 // Reference path: src/texture_refiner.cpp:174-454, shaders/atlas_photometric_gradient.hlsl,
 // atlas_seam_gradient.hlsl, atlas_adam_update.hlsl; total variation from
