@@ -521,12 +521,29 @@ BatchWorkspace layout(void* base, const BatchPlan& p) {
     return w;
 }
 
-// The tables in one copy. The source is pageable: the call returns once it has been read.
+// A piece of the tables in a launch's arguments. A launch copies its arguments before it returns, so nothing of the
+// host's is read later, nothing waits for the stream, and a recorded call carries its own tables. An asynchronous copy
+// from pageable memory promises none of that: it may read the source after it returned, and recorded into a graph it
+// reads it at every replay. 16 KB (arguments may take 32,764 bytes) hold the tables of about 70 views. Six meshes of up
+// to 12 views, forward and adjoint: 2.98 ms, with the copy 2.97.
+constexpr uint32_t kPlanWords = 2048;
+struct PlanPiece {
+    unsigned long long words[kPlanWords];
+};
+
+__global__ void __launch_bounds__(256)
+upload_plan_kernel(const __grid_constant__ PlanPiece piece, uint32_t words, unsigned long long* __restrict__ out) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i < words) out[i] = piece.words[i];
+}
+
+// The tables of a batch into its workspace.
 cudaError_t upload_plan(const BatchWorkspace& w, const BatchPlan& p, cudaStream_t s) {
-    std::vector<char> host(w.plan_bytes);
+    std::vector<unsigned long long> host((w.plan_bytes + 7) / 8 + kPlanWords);  // the last piece is read whole
+    char* const bytes = reinterpret_cast<char*>(host.data());
     const char* base = reinterpret_cast<const char*>(w.jobs);
     auto put = [&](const void* at, const auto& v) {
-        std::memcpy(host.data() + (static_cast<const char*>(at) - base), v.data(), v.size() * sizeof(v[0]));
+        std::memcpy(bytes + (static_cast<const char*>(at) - base), v.data(), v.size() * sizeof(v[0]));
     };
     put(w.jobs, p.jobs);
     put(w.tri_base, p.tri_base);
@@ -535,7 +552,15 @@ cudaError_t upload_plan(const BatchWorkspace& w, const BatchPlan& p, cudaStream_
     put(w.warp_base, p.warp_base);
     put(w.meshes, p.meshes);
     put(w.vertex_base, p.vertex_base);
-    return cudaMemcpyAsync(w.jobs, host.data(), w.plan_bytes, cudaMemcpyHostToDevice, s);
+    unsigned long long* out = reinterpret_cast<unsigned long long*>(w.jobs);
+    const size_t words = w.plan_bytes / 8;
+    static_assert(alignof(BatchJob) == 8 && sizeof(BatchJob) % 8 == 0, "tables are moved in 8-byte words");
+    for (size_t at = 0; at < words; at += kPlanWords) {
+        const uint32_t n = (uint32_t)std::min<size_t>(kPlanWords, words - at);
+        upload_plan_kernel<<<(n + 255) / 256, 256, 0, s>>>(*reinterpret_cast<const PlanPiece*>(host.data() + at), n,
+                                                           out + at);
+    }
+    return cudaGetLastError();
 }
 
 template <int TW, int TH, int CHUNK>
