@@ -505,7 +505,9 @@ BatchWorkspace layout(void* base, const BatchPlan& p) {
     w.block_sums = reinterpret_cast<unsigned long long*>(take(scan_block_count(p.segs) * 8));
     const size_t binning_end = off;
     off = w.plan_bytes;
-    w.records = reinterpret_cast<float*>(take(p.record_floats * sizeof(float)));
+    // records are added to 16 bytes at a time; a caller's workspace may start at any multiple of 8
+    const uintptr_t records = reinterpret_cast<uintptr_t>(take(p.record_floats * sizeof(float) + 16));
+    w.records = reinterpret_cast<float*>((records + 15) & ~(uintptr_t)15);
     w.bytes = std::max(off, binning_end);
     off = w.plan_bytes;
     unsigned long long tris = 0, keys = 0;

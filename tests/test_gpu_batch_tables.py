@@ -1,5 +1,7 @@
 """A batch call's tables belong to the call: a recorded forward and adjoint of a MeshBatch replays after the host memory
-of the call is gone and reused, and batches whose tables take several pieces equal their meshes rendered alone."""
+of the call is gone and reused, and batches whose tables take several pieces equal their meshes rendered alone. The
+adjoint's workspace may start at any multiple of 8 bytes."""
+import ctypes as C
 import gc
 
 import numpy as np
@@ -7,8 +9,10 @@ import pytest
 import torch
 
 import photara_drender_gb300 as pdr
+from photara_drender_gb300 import _native
 from photara_drender_gb300 import synthetic as S
 from photara_drender_gb300.batch import BatchMesh, MeshBatch
+from photara_drender_gb300.rasterizer import _ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -77,4 +81,17 @@ def test_recorded_batch_replays_with_its_own_tables():
     g.replay()
     torch.cuda.synchronize(DEV)
     assert junk
+    check(r, meshes)
+
+
+def test_adjoint_workspace_at_a_multiple_of_8():
+    rng = np.random.default_rng(2)
+    meshes = [mesh(rng, 2, 2, 31, 29), mesh(rng, 1, 1, 16, 16)]
+    r = pdr.Rasterizer(0)
+    b = MeshBatch(r, meshes)
+    b.forward()
+    b.allocate_gradients()
+    ws = torch.empty(b.workspace.numel() + 8, dtype=torch.uint8, device=DEV)
+    _native.call("pdr_render_batch_backward", b._table(), len(meshes), b.A, b.mode, C.byref(b.config), _ptr(ws[8:]),
+                 b.workspace.numel(), _ptr(b.status), r.context.stream())
     check(r, meshes)
