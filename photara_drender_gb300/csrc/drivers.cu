@@ -56,6 +56,7 @@ pdr_status enqueue_refine(const pdr_refine_options* o, const pdr_refine_view* vi
     if (pc) chk(cudaMemsetAsync(pc->fallback, 0, sizeof(uint32_t), stream));
     // plain refinement with TV and a second atlas buffer: TV + Adam in one pass, the texture alternating
     // between the two buffers (the one read this step, the one written)
+    bool overlap = false;  // launch_step's: the first kernel begins when everything before the run has completed
     const bool fused_tv = !pc && o->tv_scale > 0.0f && tv_valid && o->texture_scratch;
     float* cur = tex;
     float* other = fused_tv ? o->texture_scratch : nullptr;
@@ -64,12 +65,13 @@ pdr_status enqueue_refine(const pdr_refine_options* o, const pdr_refine_view* vi
         for (uint32_t b = 0; b < o->batch_size; ++b) bvw += valid_weights[((size_t)step * o->batch_size + b) % nviews];
         const float norm = bvw > 0.0 ? static_cast<float>(1.0 / (bvw * 3.0)) : 0.0f;
         chk(launch_photometric(cur, o->width, o->height, views, nviews, max_pixels, step, o->batch_size,
-                               o->photometric_epsilon, norm, grad, loss, stream));
+                               o->photometric_epsilon, norm, grad, loss, stream, overlap));
+        overlap = true;
         float lr, bc1, bc2;
         refine_schedule(o, step, &lr, &bc1, &bc2);
         chk(launch_adam_tv(cur, other, grad, m1, m2, o->width, o->height, tv_valid, tv_chart, o->tv_epsilon,
                            o->tv_scale, lr, o->adam_beta1, o->adam_beta2, o->adam_epsilon, bc1, bc2, o->clamp_min,
-                           o->clamp_max, stream));
+                           o->clamp_max, stream, overlap));
         float* t = cur;
         cur = other;
         other = t;
@@ -92,7 +94,8 @@ pdr_status enqueue_refine(const pdr_refine_options* o, const pdr_refine_view* vi
         for (uint32_t b = 0; b < o->batch_size; ++b) bvw += valid_weights[((size_t)step * o->batch_size + b) % nviews];
         const float norm = bvw > 0.0 ? static_cast<float>(1.0 / (bvw * 3.0)) : 0.0f;
         chk(launch_photometric(tex, o->width, o->height, views, nviews, max_pixels, step, o->batch_size,
-                               o->photometric_epsilon, norm, grad, loss, stream));
+                               o->photometric_epsilon, norm, grad, loss, stream, overlap));
+        overlap = true;
         if (o->tv_scale > 0.0f && tv_valid)
             chk(launch_tv(tex, o->width, o->height, tv_valid, tv_chart, o->tv_epsilon, o->tv_scale, grad, stream));
         float lr, bc1, bc2;
@@ -102,7 +105,7 @@ pdr_status enqueue_refine(const pdr_refine_options* o, const pdr_refine_view* vi
                                    o->adam_beta2, o->adam_epsilon, bc1, bc2, o->clamp_min, o->clamp_max, stream));
         else
             chk(launch_adam(tex, grad, m1, m2, n, lr, o->adam_beta1, o->adam_beta2, o->adam_epsilon, bc1, bc2,
-                            o->clamp_min, o->clamp_max, stream));
+                            o->clamp_min, o->clamp_max, stream, overlap));
     }
     if (seam_steps) {
         // texture_refiner.cpp:371-415: reset gradient and moments, then seam + Adam steps
@@ -112,11 +115,11 @@ pdr_status enqueue_refine(const pdr_refine_options* o, const pdr_refine_view* vi
         const float norm = 1.0F / static_cast<float>(npairs * 3u);
         for (uint32_t s = 0; s < seam_steps && err == cudaSuccess; ++s) {
             chk(launch_seam(tex, o->width, o->height, pairs, npairs, o->seam_epsilon, norm, grad, loss, o->steps + s,
-                            stream));
+                            stream, overlap));
             const float bc1 = 1.0F - std::pow(o->adam_beta1, static_cast<float>(s + 1));
             const float bc2 = 1.0F - std::pow(o->adam_beta2, static_cast<float>(s + 1));
             chk(launch_adam(tex, grad, m1, m2, n, o->seam_learning_rate, o->adam_beta1, o->adam_beta2, o->adam_epsilon,
-                            bc1, bc2, o->clamp_min, o->clamp_max, stream));
+                            bc1, bc2, o->clamp_min, o->clamp_max, stream, overlap));
         }
     }
     return cuda_status(err, "refine");
@@ -297,7 +300,7 @@ pdr_status pdr_refine_photometric(const float* tex, uint32_t W, uint32_t H, cons
         return fail(PDR_INVALID_ARGUMENT, "texture refinement options are invalid");
     if (!aligned(grad, 16)) return fail(PDR_INVALID_ARGUMENT, "texture refinement buffers must be 16-byte aligned");
     return cuda_status(launch_photometric(tex, W, H, views, nviews, max_pixels, step, batch, eps, norm, grad, loss,
-                                          (cudaStream_t)stream),
+                                          (cudaStream_t)stream, false),
                        "refine_photometric");
 }
 
@@ -307,7 +310,8 @@ pdr_status pdr_refine_seam(const float* tex, uint32_t W, uint32_t H, const float
         return fail(PDR_INVALID_ARGUMENT, "seam_uv_pairs must have shape [pair_count, 2, 2]");
     if (!aligned(grad, 16)) return fail(PDR_INVALID_ARGUMENT, "texture refinement buffers must be 16-byte aligned");
     if (npairs == 0) return PDR_OK;
-    return cuda_status(launch_seam(tex, W, H, pairs, npairs, eps, norm, grad, loss, loss_index, (cudaStream_t)stream),
+    return cuda_status(launch_seam(tex, W, H, pairs, npairs, eps, norm, grad, loss, loss_index, (cudaStream_t)stream,
+                                   false),
                        "refine_seam");
 }
 
@@ -325,7 +329,8 @@ pdr_status pdr_refine_adam(float* tex, float* grad, float* m1, float* m2, uint64
         return fail(PDR_INVALID_ARGUMENT, "texture refinement buffers must be 16-byte aligned");
     if (n % 3) return fail(PDR_INVALID_ARGUMENT, "texture refinement values must be RGB texels (a multiple of 3)");
     if (n == 0) return PDR_OK;
-    return cuda_status(launch_adam(tex, grad, m1, m2, n, lr, b1, b2, eps, bc1, bc2, cmin, cmax, (cudaStream_t)stream),
+    return cuda_status(launch_adam(tex, grad, m1, m2, n, lr, b1, b2, eps, bc1, bc2, cmin, cmax, (cudaStream_t)stream,
+                                   false),
                        "refine_adam");
 }
 

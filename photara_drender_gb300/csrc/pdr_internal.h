@@ -113,20 +113,22 @@ cudaError_t launch_prepare_view(const float* image, uint32_t C, const float* ext
                                 float* target, float* mask, cudaStream_t stream,
                                 const float* uv_attributes = nullptr, uint32_t V = 0, const uint32_t* idx = nullptr,
                                 uint32_t T = 0, float* uv = nullptr, double* weight = nullptr);
+// The steps of a refinement. overlap: the stream's last work is a kernel of the same run, and the views, masks, pairs and
+// charts were complete before that run's first kernel, so that this one may begin before that one ends.
 cudaError_t launch_photometric(const float* tex, uint32_t tw, uint32_t th, const pdr_refine_view* views,
                                uint32_t nviews, uint64_t max_pixels, uint32_t step, uint32_t batch, float eps,
-                               float norm, float* grad, float* loss, cudaStream_t stream);
+                               float norm, float* grad, float* loss, cudaStream_t stream, bool overlap);
 cudaError_t launch_seam(const float* tex, uint32_t tw, uint32_t th, const float* pairs, uint32_t npairs, float eps,
-                        float norm, float* grad, float* loss, uint32_t loss_index, cudaStream_t stream);
+                        float norm, float* grad, float* loss, uint32_t loss_index, cudaStream_t stream, bool overlap);
 cudaError_t launch_tv(const float* tex, uint32_t tw, uint32_t th, const uint8_t* valid, const int32_t* chart, float eps,
                       float scale, float* grad, cudaStream_t stream);
 cudaError_t launch_adam(float* tex, float* grad, float* m, float* v, size_t n, float lr, float b1, float b2, float eps,
-                        float bc1, float bc2, float cmin, float cmax, cudaStream_t stream);
+                        float bc1, float bc2, float cmin, float cmax, cudaStream_t stream, bool overlap);
 // launch_tv followed by launch_adam in one pass, reading tex_in and writing tex_out (different buffers)
 cudaError_t launch_adam_tv(const float* tex_in, float* tex_out, float* grad, float* m, float* v, uint32_t tw,
                            uint32_t th, const uint8_t* valid, const int32_t* chart, float tv_eps, float tv_scale,
                            float lr, float b1, float b2, float eps, float bc1, float bc2, float cmin, float cmax,
-                           cudaStream_t stream);
+                           cudaStream_t stream, bool overlap);
 cudaError_t precond_prepare();  // sets the kernels' shared-memory limits (once; before any capture)
 cudaError_t launch_precond_forward(const float* params, const uint16_t* wbf, const uint16_t* feat, uint64_t n,
                                    float* out, uint32_t* status, cudaStream_t stream);

@@ -24,21 +24,33 @@ namespace {
 
 constexpr int kPhotoThreads = 256;
 
-// The kernels of a refinement follow one another directly, most of them a few microseconds long. Outside of a capture
-// each is launched while its predecessor still runs (programmatic stream serialization: its CTAs take the places that
-// come free) and waits here until the predecessor has completed and its writes are visible: 60 steps on a 512 x 512
-// atlas 1787 -> 1515 us, 1000 on 64 x 64 10.9 -> 6.3 ms. Recorded into a graph the same edges gained nothing (9.5 and
-// 9.9 ms), so captures get ordinary launches. What a predecessor writes is never read by a non-coherent load (__ldg): the
-// kernel has begun before it is final. texel_load is the coherent one.
-__device__ __forceinline__ void wait_predecessor() {
+// The kernels of a refinement follow one another directly, most of them a few microseconds long. Within a run and outside
+// of a capture each but the first is launched while its predecessor still runs (programmatic stream serialization: its CTAs
+// take the places that come free) and waits here until the predecessor has completed and its writes are visible: 60 steps
+// on a 512 x 512 atlas 1787 -> 1515 us, 1000 on 64 x 64 10.9 -> 6.3 ms. Recorded into a graph the same edges gained nothing
+// (9.5 and 9.9 ms), so captures get ordinary launches.
+// A kernel has begun before its predecessors' writes are final, so what a kernel of the run writes (texture, gradient,
+// moments) is read after the wait alone: through pointers that the wait hands on, which no load can be moved ahead of, and
+// by coherent loads (texel_load). Views, masks, coordinates, targets, pairs and charts may be read any way: the run's first
+// kernel is launched ordinarily, so they were complete before any kernel of the run began. A caller's single step
+// (pdr_refine_photometric and the like) follows kernels that may have written them, and is launched ordinarily as well.
+template <class P>
+__device__ __forceinline__ void hand_on(P& pointer) {
+    asm volatile("" : "+l"(pointer)::"memory");
+}
+
+template <class... P>
+__device__ __forceinline__ void wait_predecessor(P&... written) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    (hand_on(written), ...);
 }
 
 __device__ __forceinline__ float texel_load(const float* p) { return __ldca(p); }
 
+// overlap: the stream's last work is a kernel of this run.
 template <class... Params, class... Args>
-cudaError_t launch_step(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t stream, Args... args) {
+cudaError_t launch_step(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t stream, bool overlap, Args... args) {
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute.val.programmaticStreamSerializationAllowed = 1;
@@ -46,11 +58,13 @@ cudaError_t launch_step(void (*kernel)(Params...), dim3 grid, int threads, cudaS
     config.gridDim = grid;
     config.blockDim = dim3(threads);
     config.stream = stream;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const bool known = cudaStreamIsCapturing(stream, &capture) == cudaSuccess;
-    if (!known) cudaGetLastError();
     config.attrs = &attribute;
-    config.numAttrs = known && capture == cudaStreamCaptureStatusNone ? 1 : 0;
+    if (overlap) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const bool known = cudaStreamIsCapturing(stream, &capture) == cudaSuccess;
+        if (!known) cudaGetLastError();
+        config.numAttrs = known && capture == cudaStreamCaptureStatusNone ? 1 : 0;
+    }
     return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
@@ -175,7 +189,7 @@ __global__ void __launch_bounds__(kPhotoThreads, 5)
 photometric_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, const pdr_refine_view* __restrict__ views,
                    uint32_t nviews, uint32_t step, uint32_t batch, float eps, float norm, uint32_t rounds,
                    float* __restrict__ grad, float* __restrict__ loss) {
-    wait_predecessor();
+    wait_predecessor(tex, grad, loss);
     const pdr_refine_view v = views[((size_t)step * batch + blockIdx.y) % nviews];
     const float2* const uvs = reinterpret_cast<const float2*>(v.uv);
     float local = 0.0f;
@@ -217,7 +231,7 @@ photometric_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, cons
 __global__ void seam_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, const float4* __restrict__ pairs,
                             uint32_t npairs, float eps, float norm, float* __restrict__ grad, float* __restrict__ loss,
                             uint32_t loss_index) {
-    wait_predecessor();
+    wait_predecessor(tex, grad, loss);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float local = 0.0f;
     if (i < npairs) {
@@ -356,7 +370,7 @@ __device__ __forceinline__ void clear_gradient(float4* g, const float4& was) {
 
 __global__ void adam_kernel(float* __restrict__ tex, float* __restrict__ grad, float* __restrict__ m1,
                             float* __restrict__ m2, size_t texels, AdamStep s) {
-    wait_predecessor();
+    wait_predecessor(tex, grad, m1, m2);
     // one texel per thread: texture and moments [texels][3], gradient [texels][4] read and cleared as one
     // float4 (four texels per thread, or four values with the gradient gathered, were slower). 16.8 M texels of which
     // few have moments, a seam polish step: 330 us writing every value and dividing nine times; with the quotients and
@@ -435,7 +449,7 @@ adam_tv_kernel(const float* __restrict__ tex_in, float* __restrict__ tex_out, fl
                float* __restrict__ m1, float* __restrict__ m2, uint32_t tw, uint32_t th,
                const uint8_t* __restrict__ valid, const int32_t* __restrict__ chart, float tv_eps, float tv_scale,
                uint32_t rows, AdamStep s) {
-    wait_predecessor();
+    wait_predecessor(tex_in, tex_out, grad, m1, m2);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t x = blockIdx.x * 256u + threadIdx.x;
     const uint32_t y0 = blockIdx.y * rows, y1 = min(y0 + rows, th);
@@ -500,14 +514,14 @@ adam_tv_kernel(const float* __restrict__ tex_in, float* __restrict__ tex_out, fl
 cudaError_t launch_adam_tv(const float* tex_in, float* tex_out, float* grad, float* m, float* v, uint32_t tw,
                            uint32_t th, const uint8_t* valid, const int32_t* chart, float tv_eps, float tv_scale,
                            float lr, float b1, float b2, float eps, float bc1, float bc2, float cmin, float cmax,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, bool overlap) {
     // rows per warp: eight where the atlas still fills the chip several times, fewer below
     uint32_t rows = 8;
     const uint64_t strips = (uint64_t)((tw + 255) / 256) * th;  // CTAs at one row each
     while (rows > 1 && strips / rows < 152u * 16u) rows >>= 1;
     if ((th + rows - 1) / rows > 65535u) rows = (th + 65534u) / 65535u;
     const dim3 grid((tw + 255) / 256, (th + rows - 1) / rows);
-    return launch_step(adam_tv_kernel, grid, 256, stream, tex_in, tex_out, grad, m, v, tw, th, valid, chart, tv_eps, tv_scale,
+    return launch_step(adam_tv_kernel, grid, 256, stream, overlap, tex_in, tex_out, grad, m, v, tw, th, valid, chart, tv_eps, tv_scale,
                        rows, adam_step(lr, b1, b2, eps, bc1, bc2, cmin, cmax));
 }
 
@@ -524,20 +538,20 @@ cudaError_t launch_prepare_view(const float* image, uint32_t C, const float* ext
 
 cudaError_t launch_photometric(const float* tex, uint32_t tw, uint32_t th, const pdr_refine_view* views,
                                uint32_t nviews, uint64_t max_pixels, uint32_t step, uint32_t batch, float eps,
-                               float norm, float* grad, float* loss, cudaStream_t stream) {
+                               float norm, float* grad, float* loss, cudaStream_t stream, bool overlap) {
     // pixels per thread: eight where the step still fills the chip, fewer below (4 views of 320 x 240: two 6.2 us, one
     // 7.5, four 6.9)
     uint32_t rounds = 8;
     while (rounds > 1 && max_pixels * batch / (kPhotoThreads * rounds) < 152u * 3u) rounds >>= 1;
     const uint64_t per = (uint64_t)kPhotoThreads * rounds;
     const dim3 grid((unsigned)((max_pixels + per - 1) / per), batch);
-    return launch_step(photometric_kernel, grid, kPhotoThreads, stream, tex, tw, th, views, nviews, step, batch, eps, norm,
+    return launch_step(photometric_kernel, grid, kPhotoThreads, stream, overlap, tex, tw, th, views, nviews, step, batch, eps, norm,
                        rounds, grad, loss);
 }
 
 cudaError_t launch_seam(const float* tex, uint32_t tw, uint32_t th, const float* pairs, uint32_t npairs, float eps,
-                        float norm, float* grad, float* loss, uint32_t loss_index, cudaStream_t stream) {
-    return launch_step(seam_kernel, (npairs + 255) / 256, 256, stream, tex, tw, th, reinterpret_cast<const float4*>(pairs),
+                        float norm, float* grad, float* loss, uint32_t loss_index, cudaStream_t stream, bool overlap) {
+    return launch_step(seam_kernel, (npairs + 255) / 256, 256, stream, overlap, tex, tw, th, reinterpret_cast<const float4*>(pairs),
                        npairs, eps, norm, grad, loss, loss_index);
 }
 
@@ -548,14 +562,14 @@ cudaError_t launch_tv(const float* tex, uint32_t tw, uint32_t th, const uint8_t*
 }
 
 cudaError_t launch_adam(float* tex, float* grad, float* m, float* v, size_t n, float lr, float b1, float b2, float eps,
-                        float bc1, float bc2, float cmin, float cmax, cudaStream_t stream) {
+                        float bc1, float bc2, float cmin, float cmax, cudaStream_t stream, bool overlap) {
     // n = texels * 3 values. One texel per thread (the loop strides only past 2^31 blocks): a grid capped at
     // eight CTAs per SM that looped over the arrays kept fewer loads in flight
     const size_t texels = n / 3;
     size_t blocks = (texels + 255) / 256;
     if (blocks > 0x7FFFFFFFu) blocks = 0x7FFFFFFFu;
     if (blocks == 0) blocks = 1;
-    return launch_step(adam_kernel, (unsigned)blocks, 256, stream, tex, grad, m, v, texels,
+    return launch_step(adam_kernel, (unsigned)blocks, 256, stream, overlap, tex, grad, m, v, texels,
                        adam_step(lr, b1, b2, eps, bc1, bc2, cmin, cmax));
 }
 
