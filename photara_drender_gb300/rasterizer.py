@@ -272,7 +272,9 @@ class Rasterizer:
     def __init__(self, device_index: int = 0, enable_validation: bool = False):
         self.context = Context(device_index, enable_validation)
         self._capacity = 0
-        self._viewport_cache = {}  # (viewport, views, width, height) -> device rows, at most _VIEWPORT_CACHE of them
+        # (viewport, views, width, height) -> device rows, at most _VIEWPORT_CACHE of them, the last used ones
+        self._viewport_cache = {}
+        self._captured_viewports = {}  # id -> rows that a recorded graph reads by their address: kept for good
 
     @property
     def device_info(self) -> DeviceInfo:
@@ -281,7 +283,8 @@ class Rasterizer:
     def _device_viewports(self, viewport, views: int, width: int, height: int) -> torch.Tensor:
         """The device rows of one viewport for all views, kept on the rasterizer: they are constants, their upload
         waits for the host, and it is not allowed inside a CUDA graph capture. Rows given per view are kept too,
-        for the captures."""
+        for the captures. The least recently used are dropped, but never rows handed out while a capture records: the
+        graph reads them by their address for as long as it is replayed, and nothing else need hold them."""
         try:
             key = (views, width, height, None if viewport is None else tuple(
                 tuple(float(x) for x in v) if isinstance(v, (list, tuple)) else v if v is None else float(v)
@@ -296,7 +299,14 @@ class Rasterizer:
             self._viewport_cache[key] = rows
         else:  # possibly made on another stream: its memory may not be reused under this one's work
             rows.record_stream(torch.cuda.current_stream(self.context.device))
+            self._viewport_cache[key] = self._viewport_cache.pop(key)  # the last used one
+        self._keep_if_captured(rows)
         return rows
+
+    def _keep_if_captured(self, rows: torch.Tensor) -> None:
+        """Keeps viewport rows for the rasterizer's life when a capture on the current stream records their address."""
+        if torch.cuda.is_current_stream_capturing():
+            self._captured_viewports[id(rows)] = rows
 
     # -- tile binning -------------------------------------------------------------------------
     def _bin(self, clip: torch.Tensor, idx: torch.Tensor, width: int, height: int, vps: torch.Tensor):

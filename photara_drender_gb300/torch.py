@@ -295,6 +295,7 @@ class _RenderFunction(torch.autograd.Function):
             a.indices, a.triangle_count = idx.data_ptr(), idx.shape[0]
             a.width, a.height = raster.shape[2], raster.shape[1]
             a.viewports, a.raster = ctx.vps.data_ptr(), raster.data_ptr()
+            r._keep_if_captured(ctx.vps)
             keep = []
             if attrs is not None:
                 gi = g_interp.contiguous() if g_interp is not None else torch.zeros(
