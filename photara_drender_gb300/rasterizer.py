@@ -285,12 +285,14 @@ class Rasterizer:
         waits for the host, and it is not allowed inside a CUDA graph capture. Rows given per view are kept too,
         for the captures. The least recently used are dropped, but never rows handed out while a capture records: the
         graph reads them by their address for as long as it is replayed, and nothing else need hold them."""
+        if viewport is not None and not hasattr(viewport, "__len__"):
+            viewport = list(viewport)  # an iterator can be read once
         try:
             key = (views, width, height, None if viewport is None else tuple(
                 tuple(float(x) for x in v) if isinstance(v, (list, tuple)) else v if v is None else float(v)
                 for v in viewport))
             rows = self._viewport_cache.get(key)
-        except TypeError:
+        except (TypeError, ValueError, RuntimeError):  # rows that are arrays or tensors
             return _viewports(viewport, views, width, height, self.context.device)[0]
         if rows is None:
             rows, _ = _viewports(viewport, views, width, height, self.context.device)
