@@ -554,7 +554,8 @@ PDR_API pdr_status pdr_render_batch_direct_workspace_bytes(const pdr_render_mesh
 PDR_API pdr_status pdr_render_batch_direct(const pdr_render_mesh* meshes, uint32_t mesh_count, uint32_t attribute_count,
                                            uint32_t cull_mode, uint32_t address_mode, void* workspace,
                                            size_t workspace_bytes, void* stream);
-/* The adjoints of the forward for every mesh (gradient outputs are overwritten). */
+/* The adjoints of the forward for every mesh (gradient outputs are overwritten). Meshes whose gradient outputs are the
+ * same or overlap receive the sum. */
 PDR_API pdr_status pdr_render_batch_backward(const pdr_render_mesh* meshes, uint32_t mesh_count,
                                              uint32_t attribute_count, uint32_t address_mode,
                                              const pdr_batch_config* config, void* workspace,

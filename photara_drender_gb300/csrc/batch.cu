@@ -59,6 +59,7 @@ struct BatchMeshSum {
     unsigned long long first_record;
     uint32_t V, views;
     float *g_clip, *g_attr, *g_uv;
+    unsigned long long add;  // the gradients lie in buffers that others add into as well: added, not stored
 };
 
 // The last job j with base[j] <= x (base[0] == 0, non-decreasing).
@@ -336,7 +337,7 @@ batch_vertex_sum_kernel(const BatchMeshSum* __restrict__ meshes, const unsigned 
     const uint32_t m = find_job(vertex_base, nmeshes, at);
     const BatchMeshSum& s = meshes[m];
     sum_vertex_records<kA>(records + s.first_record, s.views, s.V, (uint32_t)(at - vertex_base[m]), s.g_clip, s.g_attr,
-                           s.g_uv);
+                           s.g_uv, s.add != 0);
 }
 
 struct BatchPlan {
@@ -346,6 +347,33 @@ struct BatchPlan {
     std::vector<unsigned long long> vertex_base;  // nmeshes + 1
     unsigned long long total_tris = 0, segs = 0, btiles = 0, keys = 0, record_floats = 0;
 };
+
+// Marks the meshes whose gradient buffers overlap another's, or one another (one mesh at two resolutions, say): their
+// gradients are sums over all of them.
+void mark_shared_gradients(const pdr_render_mesh* meshes, uint32_t n, uint32_t A, BatchPlan* plan) {
+    struct Range {
+        uintptr_t begin, end;
+        uint32_t mesh;
+    };
+    std::vector<Range> ranges;
+    for (uint32_t m = 0; m < n; ++m) {
+        const pdr_render_mesh& M = meshes[m];
+        const auto add = [&](const float* p, uint64_t floats) {
+            const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+            if (p && floats) ranges.push_back({b, b + floats * sizeof(float), m});
+        };
+        add(M.grad_clip_positions, (uint64_t)M.views * M.vertex_count * 4);
+        add(M.grad_attributes, (uint64_t)M.vertex_count * A);
+        add(M.grad_uv_attributes, (uint64_t)M.vertex_count * 2);
+        add(M.grad_texture, (uint64_t)M.texture_width * M.texture_height * 4);
+    }
+    std::sort(ranges.begin(), ranges.end(), [](const Range& a, const Range& b) { return a.begin < b.begin; });
+    size_t last = 0;  // the range so far that ends last
+    for (size_t k = 1; k < ranges.size(); ++k) {
+        if (ranges[k].begin < ranges[last].end) plan->meshes[ranges[k].mesh].add = plan->meshes[ranges[last].mesh].add = 1;
+        if (ranges[k].end > ranges[last].end) last = k;
+    }
+}
 
 bool config_supported(const pdr_batch_config* c) {
     if (!c) return false;
@@ -429,10 +457,11 @@ pdr_status plan_batch(const pdr_render_mesh* meshes, uint32_t n, const pdr_batch
             plan->btile_base.push_back(plan->btile_base.back() + (unsigned long long)btcx * btcy);
         }
         plan->meshes.push_back({plan->record_floats, M.vertex_count, M.views, M.grad_clip_positions, M.grad_attributes,
-                                M.grad_uv_attributes});
+                                M.grad_uv_attributes, 0});
         plan->vertex_base.push_back(plan->vertex_base.back() + M.vertex_count);
         plan->record_floats += record * M.views * M.vertex_count;
     }
+    if (need_grads) mark_shared_gradients(meshes, n, A, plan);
     plan->total_tris = plan->tri_base.back();
     plan->segs = plan->tile_base.back();
     plan->btiles = plan->btile_base.back();
@@ -703,6 +732,13 @@ pdr_status pdr_render_batch_backward(const pdr_render_mesh* meshes, uint32_t mes
         const pdr_render_mesh& M = meshes[m];
         if (M.grad_texture)
             e = cudaMemsetAsync(M.grad_texture, 0, (size_t)M.texture_width * M.texture_height * 4 * sizeof(float), s);
+        if (!plan.meshes[m].add) continue;
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(M.grad_clip_positions, 0, (size_t)M.views * M.vertex_count * 4 * sizeof(float), s);
+        if (e == cudaSuccess && M.grad_attributes)
+            e = cudaMemsetAsync(M.grad_attributes, 0, (size_t)M.vertex_count * attribute_count * sizeof(float), s);
+        if (e == cudaSuccess && M.grad_uv_attributes)
+            e = cudaMemsetAsync(M.grad_uv_attributes, 0, (size_t)M.vertex_count * 2 * sizeof(float), s);
     }
     if (e != cudaSuccess) return set_cuda_error(e, "render_batch_backward(set-up)");
     const uint32_t nj = (uint32_t)plan.jobs.size(), total = (uint32_t)plan.btiles;

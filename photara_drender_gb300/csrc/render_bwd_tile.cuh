@@ -374,11 +374,12 @@ __device__ __forceinline__ void render_backward_pixel(const BackwardView& v, uin
 
 // The vertex-gradient records of one vertex in all views into the outputs: each view's clip gradient (x, y, 0, w),
 // and the uv and attribute gradients summed over the views in view order. Every output element is written, so
-// none needs clearing first.
+// none needs clearing first; with `add` they are added to outputs that were cleared and that others add to.
 template <int kA>
 __device__ __forceinline__ void sum_vertex_records(const float* __restrict__ rec_all, uint32_t views, uint32_t V,
                                                    uint32_t vtx, float* __restrict__ g_clip_all,
-                                                   float* __restrict__ g_attr, float* __restrict__ g_uv) {
+                                                   float* __restrict__ g_attr, float* __restrict__ g_uv,
+                                                   bool add = false) {
     constexpr uint32_t kR = vertex_record_floats(kA);
     constexpr uint32_t kNV = 2 + kA + 3;
     float acc[2 + kA];
@@ -397,8 +398,22 @@ __device__ __forceinline__ void sum_vertex_records(const float* __restrict__ rec
         }
 #pragma unroll
         for (int j = 0; j < 2 + kA; ++j) acc[j] += r[j];
-        reinterpret_cast<float4*>(g_clip_all)[(size_t)view * V + vtx] =
-            make_float4(r[kNV - 3], r[kNV - 2], 0.0f, r[kNV - 1]);
+        const float4 clip = make_float4(r[kNV - 3], r[kNV - 2], 0.0f, r[kNV - 1]);
+        if (add)
+            red_v4(g_clip_all + ((size_t)view * V + vtx) * 4, clip);
+        else
+            reinterpret_cast<float4*>(g_clip_all)[(size_t)view * V + vtx] = clip;
+    }
+    if (add) {
+        if (g_uv) {
+            atomicAdd(g_uv + (size_t)vtx * 2, acc[0]);
+            atomicAdd(g_uv + (size_t)vtx * 2 + 1, acc[1]);
+        }
+        if (g_attr) {
+#pragma unroll
+            for (int a = 0; a < kA; ++a) atomicAdd(g_attr + (size_t)vtx * kA + a, acc[2 + a]);
+        }
+        return;
     }
     if (g_uv) {
         g_uv[(size_t)vtx * 2] = acc[0];
