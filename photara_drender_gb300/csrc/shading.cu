@@ -79,19 +79,19 @@ interpolate_backward_kernel(const float* __restrict__ attr_all, size_t attr_stri
     const float* attr = attr_all + (size_t)view * attr_stride;
     const bool inside = valid && vi.x < V && vi.y < V && vi.z < V;
     VertexSums<kC + 3>& s = sums[threadIdx.x >> 5];
+    uint3 once = vi;  // each distinct vertex once: a repeated corner is no vertex, its weight is with the first
+    if (vi.y == vi.x) once.y = 0xffffffffu;
+    if (vi.z == vi.x || vi.z == vi.y) once.z = 0xffffffffu;
     if (valid && grad_attr_all) {
         const uint32_t vs[3] = {vi.x, vi.y, vi.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const uint32_t vx = vs[k];
-            bool first = true;
-#pragma unroll
-            for (int j = 0; j < k; ++j) first = first && vs[j] != vx;
             float wgt = 0.0f;
             if (vi.x == vx) wgt += r.x;
             if (vi.y == vx) wgt += r.y;
             if (vi.z == vx) wgt += 1.0f - r.x - r.y;
-            s.vals[lane][k] = first ? wgt : 0.0f;
+            s.vals[lane][k] = wgt;
         }
     }
     float gx = 0.0f, gy = 0.0f;
@@ -114,7 +114,7 @@ interpolate_backward_kernel(const float* __restrict__ attr_all, size_t attr_stri
         if (grad_attr_all) {
             float* grad_attr = grad_attr_all + (size_t)view * attr_stride;
             add_vertex_sums(
-                s, valid, id, vi, n,
+                s, valid, id, once, n,
                 [](const VertexSums<kC + 3>& q, uint32_t l, uint32_t corner, uint32_t c) {
                     return q.vals[l][corner] * q.vals[l][3 + c];
                 },
