@@ -9,6 +9,7 @@ everywhere: positions [B, V, 4] rasterize B views in one launch.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import math
 import threading
@@ -77,22 +78,23 @@ def _ptr(t: Optional[torch.Tensor]):
 
 class _HostWords:
     """Status blocks in pinned host memory, one per context, cut from pages of 128 (pinning one takes 0.2 ms). A
-    context gives its block back when it goes; it waits for the device on every use, so nothing writes to it then."""
+    context gives its block back when it goes; it waits for the device on every use, so nothing writes to it then.
+    give() runs as a finalizer, at any allocation of any thread, take()'s own included: no lock that it could wait for,
+    the deque's operations are atomic."""
 
     def __init__(self):
-        self._lock = threading.Lock()
-        self._free = []
+        self._free = collections.deque()
 
     def take(self) -> torch.Tensor:
-        with self._lock:
-            if not self._free:
+        while True:
+            try:
+                return self._free.pop()
+            except IndexError:
                 page = torch.zeros((128, _native.STATUS_WORDS), dtype=torch.int32, pin_memory=True)
-                self._free = list(page.unbind(0))
-            return self._free.pop()
+                self._free.extend(page.unbind(0))
 
     def give(self, block: torch.Tensor) -> None:
-        with self._lock:
-            self._free.append(block)
+        self._free.append(block)
 
 
 _host_words = _HostWords()
