@@ -48,6 +48,7 @@ constexpr int kLead = 8;             // columns a waiting band lets the previous
 constexpr int kL2Ahead = 64;         // steps the reverse sweep prefetches the forward field into L2
 constexpr long long kWaitCycles = 1ll << 32;  // about two seconds at GB300 clocks
 constexpr int kStatThreads = 256;
+constexpr uint32_t kPadControlWords = 32;  // TileSweeps::control
 
 enum : uint32_t { kErrTimeout = 1, kErrFaceRange = 2, kErrDegenerate = 4, kErrManifold = 8 };
 
@@ -941,7 +942,7 @@ PadLayout pad_layout(uint32_t W, uint32_t H, uint32_t C) {
     const size_t words = (size_t)((W + 31) / 32) * H, bands = (H + 31) / 32;
     size_t o = 0;
     L.control = o;
-    o += align_up(4 * sizeof(uint32_t));
+    o += align_up(kPadControlWords * sizeof(uint32_t));
     L.counters = o;
     o += align_up(4 * sizeof(unsigned long long));
     L.bits = o;
