@@ -624,6 +624,15 @@ PDR_API pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const 
                                          uint32_t height, uint32_t margin, uint32_t fill_unobserved,
                                          uint32_t maximum_fill_distance, float valid_threshold, void* workspace,
                                          size_t workspace_bytes, uint64_t* stats, uint32_t* status, void* stream);
+/* pdr_pad_texture_atlas, which sweeps atlases of up to 4384 texels a side in tiles until no tile changes, with the
+ * number of passes a direction may take before band sweeps, whose time depends on the size alone, take over (0: at
+ * once). The results are the same. */
+PDR_API pdr_status pdr_pad_texture_atlas_passes(float* color, uint32_t channels, const float* valid_mask,
+                                                const float* coverage_mask, float* filled_mask, uint32_t width,
+                                                uint32_t height, uint32_t margin, uint32_t fill_unobserved,
+                                                uint32_t maximum_fill_distance, float valid_threshold,
+                                                uint32_t max_passes, void* workspace, size_t workspace_bytes,
+                                                uint64_t* stats, uint32_t* status, void* stream);
 /* Workspace of pdr_fill_texture_on_surface. */
 PDR_API pdr_status pdr_surface_fill_workspace_bytes(uint32_t width, uint32_t height, uint32_t triangle_count,
                                                     size_t* bytes);

@@ -82,6 +82,8 @@ _SIGNATURES = {
     "pdr_pad_workspace_bytes": (_i32, [_u32, _u32, _u32, _vp]),
     "pdr_pad_texture_atlas": (_i32, [_vp, _u32, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, C.c_float, _vp, _sz, _vp,
                                      _vp, _vp]),
+    "pdr_pad_texture_atlas_passes": (_i32, [_vp, _u32, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, C.c_float, _u32, _vp,
+                                            _sz, _vp, _vp, _vp]),
     "pdr_surface_fill_workspace_bytes": (_i32, [_u32, _u32, _u32, _vp]),
     "pdr_fill_texture_on_surface": (_i32, [_vp, _u32, _vp, _vp, _vp, _u32, _u32, _vp, _u32, _vp, _sz, _vp, _vp, _vp]),
     "pdr_mip_pyramid_size": (_i32, [_u32, _u32, _u32, _vp, _vp]),

@@ -164,14 +164,15 @@ __device__ __forceinline__ uint32_t final_index(uint32_t x, uint32_t y, uint32_t
 
 // One 8SSEDT sweep (texture_padding.cpp:80-94): the forward sweep writes `out` from the source bits, the
 // reverse sweep (kBack) reads the forward field `in` and writes the final field `out`. control: [0]
-// forward ticket, [1] reverse ticket, [2] failure flag. The relaxations run one by one, with the
-// reference's clamp of offsets to +-16384. For atlases above kTileMaxSide, and where the device cannot
-// hold pad_tiles_kernel's grid at once.
+// forward ticket, [1] reverse ticket, [2] failure flag, [3] pad_tiles_kernel gave up. The relaxations run one by
+// one, with the reference's clamp of offsets to +-16384. For atlases above kTileMaxSide, where the device cannot
+// hold pad_tiles_kernel's grid at once, and (after_tiles) behind that kernel, where it gave up.
 template <bool kBack>
 __global__ void __launch_bounds__(32) pad_sweep_kernel(const uint32_t* __restrict__ src_bits, uint32_t words_per_row,
                                                        const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                        uint32_t* __restrict__ boundary, uint32_t* control,
-                                                       uint32_t* status, int32_t W, int32_t H) {
+                                                       uint32_t* status, int32_t W, int32_t H, bool after_tiles) {
+    if (after_tiles && (control[3] == 0u || control[2] != 0u)) return;
     const int lane = threadIdx.x;
     uint32_t band = 0;
     if (lane == 0) band = atomicAdd(&control[kBack ? 1 : 0], 1u);
@@ -349,7 +350,14 @@ constexpr int kPadWarps = 4;              // 34 KB of shared memory: six CTAs pe
 // them (every 4 and 2 passes 695 us for the holes, but 6453 with all sources in the last corner; 3 and 3: 737, 4916).
 template <bool kBack>
 constexpr uint32_t kShiftEvery = kBack ? 3 : 8;
-constexpr uint32_t kPadMaxPasses = 1u << 16;
+// Passes a direction may take before the band sweeps take over. A pass settles at least the texels whose four earlier
+// neighbours were final, so W + 2H always suffice, but at 13 us or more each that could be 30 times the bands' time. Of
+// 140 atlases of 64 to 4096 texels a side with charts, holes, dots, curves and single sources, none took more than
+// (W + 2H) / 43 (all sources at the far end of a long side): the line leaves a third more, and so many short passes in
+// both directions take twice as long as the bands' sweeps. No line on the passes tells the few apart that bands sweep
+// faster: sources along the last column alone (4096 x 4096 13.0 ms, bands 6.9; every pass improves half of the tiles a
+// little) and long curves across an atlas 30 times as wide as high (4000 x 130 2.0 ms, bands 1.8).
+inline uint32_t pad_max_passes(uint32_t W, uint32_t H) { return (W + 2 * H) / 32 + 8; }
 constexpr uint32_t kNoSource = 0x75307530u;  // (30000, 30000): farther from any texel than a real source
 static_assert(kPadTileW == 64, "a lane moves two columns of a tile row");
 
@@ -358,9 +366,10 @@ struct TileSweeps {
     uint32_t* forward;   // [H][W] source positions after the forward sweep
     uint32_t* field;     // [H][W] after the reverse sweep
     uint8_t* changed;    // [2][(tiles_x + 1) * (tiles_y + 1)]: tile changed in the last even / odd pass
-    uint32_t* control;   // [2] failure flag, [8] barrier arrivals, [12..15] "a tile changed" per pass & 3
+    uint32_t* control;   // [2] failure flag, [3] gave up, [8] barrier arrivals, [12..15] "a tile changed" per pass & 3
     uint32_t* status;
-    uint32_t words_per_row;
+    uint32_t* boundary;  // the band sweeps', in the place of `changed`
+    uint32_t boundary_words, words_per_row, max_passes;
     int32_t W, H, tiles_x, tiles_y;  // of the even passes
 };
 
@@ -554,13 +563,15 @@ __device__ __forceinline__ bool sweep_tile(const SweepSpace<kBack>& sp, int32_t 
     return __any_sync(0xFFFFFFFFu, changed);
 }
 
+enum class Sweep { kDone, kTooLong, kFailed };
+
 template <bool kBack>
-__device__ bool sweep_tiles(const TileSweeps& s, uint32_t& phase, uint32_t* buf, uint32_t* top) {
+__device__ Sweep sweep_tiles(const TileSweeps& s, uint32_t& phase, uint32_t* buf, uint32_t* top) {
     const SweepSpace<kBack> sp(s);
     const int32_t lane = threadIdx.x & 31;
     const int32_t warp = blockIdx.x * kPadWarps + (threadIdx.x >> 5), warps = gridDim.x * kPadWarps;
     const size_t slot = (size_t)(s.tiles_x + 1) * (s.tiles_y + 1);
-    for (uint32_t pass = 0; pass < kPadMaxPasses; ++pass) {
+    for (uint32_t pass = 0; pass < s.max_passes; ++pass) {
         // tiles start at multiples of 64 x 32, in shifted passes half a tile earlier (clipped to the atlas)
         const int32_t shifted = pass % kShiftEvery<kBack> == kShiftEvery<kBack> - 1u;
         const int32_t was_shifted = pass % kShiftEvery<kBack> == 0u && pass > 0;  // the pass before
@@ -603,10 +614,10 @@ __device__ bool sweep_tiles(const TileSweeps& s, uint32_t& phase, uint32_t* buf,
                 if (changed) atomicOr(any, 1u);
             }
         }
-        if (!pad_grid_barrier(s.control, phase)) return false;
-        if (ld_relaxed(any) == 0) return true;
+        if (!pad_grid_barrier(s.control, phase)) return Sweep::kFailed;
+        if (ld_relaxed(any) == 0) return Sweep::kDone;
     }
-    return false;
+    return Sweep::kTooLong;  // in every CTA alike
 }
 
 __global__ void __launch_bounds__(32 * kPadWarps, 6) pad_tiles_kernel(TileSweeps s) {
@@ -614,12 +625,18 @@ __global__ void __launch_bounds__(32 * kPadWarps, 6) pad_tiles_kernel(TileSweeps
     __shared__ uint32_t top[kPadWarps][kPadTileW + 2];
     const int warp = threadIdx.x >> 5;
     uint32_t phase = 0;
-    bool ok = sweep_tiles<false>(s, phase, buf[warp], top[warp]);
-    // the reverse sweep starts its passes at slot 0: clear the slots behind a barrier of their own
-    if (ok && blockIdx.x == 0 && threadIdx.x < 4) s.control[12 + threadIdx.x] = 0u;
-    ok = ok && pad_grid_barrier(s.control, phase);
-    ok = ok && sweep_tiles<true>(s, phase, buf[warp], top[warp]);
-    if (!ok && threadIdx.x == 0) {
+    Sweep r = sweep_tiles<false>(s, phase, buf[warp], top[warp]);
+    if (r == Sweep::kDone) {
+        // the reverse sweep starts its passes at slot 0: clear the slots behind a barrier of their own
+        if (blockIdx.x == 0 && threadIdx.x < 4) s.control[12 + threadIdx.x] = 0u;
+        r = pad_grid_barrier(s.control, phase) ? sweep_tiles<true>(s, phase, buf[warp], top[warp]) : Sweep::kFailed;
+    }
+    if (r == Sweep::kTooLong) {  // the band sweeps behind this kernel start over, with their boundaries marked
+        if (blockIdx.x == 0 && threadIdx.x == 0) s.control[3] = 1u;
+        for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < s.boundary_words; k += gridDim.x * blockDim.x)
+            s.boundary[k] = kMarker;
+    }
+    if (r == Sweep::kFailed && threadIdx.x == 0) {
         atomicExch(s.control + 2, 1u);
         atomicOr(s.status + PDR_STATUS_PAD_ERROR, kErrTimeout);
     }
@@ -631,8 +648,9 @@ struct FillParams {
     const float* coverage;
     float* filled;
     const uint32_t* src_bits;
-    const uint32_t* field;  // [H][W] source positions (bands == 0, pad_tiles_kernel) or band-major offsets (final_index)
+    const uint32_t* field;  // [H][W] source positions (pad_tiles_kernel) or band-major offsets (final_index)
     uint32_t channels, words_per_row, margin, fill_unobserved, bands;
+    bool tiled;             // positions, unless pad_tiles_kernel gave up
     bool color4;            // four channels at a 16-byte aligned base: texels move as float4
     int32_t W, H;
     unsigned long long margin2, limit2;
@@ -643,18 +661,18 @@ __device__ __forceinline__ bool is_source(const FillParams& P, uint32_t x, uint3
 }
 
 // texture_padding.cpp:292-330 for one non-source texel: 0 skip, 1 fill, 2 covered but left unfilled.
-__device__ __forceinline__ int fill_decision(const FillParams& P, uint32_t x, uint32_t y, uint64_t& src,
-                                             bool& covered) {
+__device__ __forceinline__ int fill_decision(const FillParams& P, bool positions, uint32_t x, uint32_t y,
+                                             uint64_t& src, bool& covered) {
     const uint64_t p = (uint64_t)y * (uint32_t)P.W + x;
     int32_t ox, oy;
-    if (P.bands) {
-        const uint32_t f = P.field[final_index(x, y, (uint32_t)P.W, P.bands)];
-        ox = unpack_x(f);
-        oy = unpack_y(f);
-    } else {
+    if (positions) {
         const uint32_t f = P.field[p];
         ox = (int32_t)(f & 0xFFFFu) - (int32_t)x;
         oy = (int32_t)(f >> 16) - (int32_t)y;
+    } else {
+        const uint32_t f = P.field[final_index(x, y, (uint32_t)P.W, P.bands)];
+        ox = unpack_x(f);
+        oy = unpack_y(f);
     }
     const int32_t d2 = ox * ox + oy * oy;
     if (d2 >= 2 * kFar * kFar) return 0;
@@ -674,6 +692,7 @@ __global__ void __launch_bounds__(kStatThreads) pad_fill_kernel(FillParams P, co
                                                                 unsigned long long* counters) {
     __shared__ unsigned long long red[kStatThreads / 32];
     if (control[2] != 0 || (stats[0] == 0 && stats[4] == 0)) return;
+    const bool positions = P.tiled && control[3] == 0u;
     const uint32_t n = (uint32_t)P.W * (uint32_t)P.H;  // at most 2^28
     unsigned long long gutter = 0, unobserved = 0, remaining = 0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -681,7 +700,7 @@ __global__ void __launch_bounds__(kStatThreads) pad_fill_kernel(FillParams P, co
         if (is_source(P, x, y)) continue;
         uint64_t s = 0;
         bool covered = false;
-        const int d = fill_decision(P, x, y, s, covered);
+        const int d = fill_decision(P, positions, x, y, s, covered);
         if (d == 0) continue;
         if (d == 2) {
             ++remaining;
@@ -697,7 +716,7 @@ __global__ void __launch_bounds__(kStatThreads) pad_fill_kernel(FillParams P, co
                 if (is_source(P, sx, sy) || s >= limit) break;
                 uint64_t next = 0;
                 bool cov2 = false;
-                if (fill_decision(P, sx, sy, next, cov2) != 1) break;
+                if (fill_decision(P, positions, sx, sy, next, cov2) != 1) break;
                 limit = s;
                 s = next;
                 sx = (uint32_t)(s % (uint32_t)P.W);
@@ -1035,6 +1054,16 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
                                  uint32_t fill_unobserved, uint32_t maximum_fill_distance, float valid_threshold,
                                  void* workspace, size_t workspace_bytes, uint64_t* stats, uint32_t* status,
                                  void* stream) {
+    return pdr_pad_texture_atlas_passes(color, channels, valid_mask, coverage_mask, filled_mask, width, height, margin,
+                                        fill_unobserved, maximum_fill_distance, valid_threshold,
+                                        pad_max_passes(width, height), workspace, workspace_bytes, stats, status, stream);
+}
+
+pdr_status pdr_pad_texture_atlas_passes(float* color, uint32_t channels, const float* valid_mask,
+                                        const float* coverage_mask, float* filled_mask, uint32_t width, uint32_t height,
+                                        uint32_t margin, uint32_t fill_unobserved, uint32_t maximum_fill_distance,
+                                        float valid_threshold, uint32_t max_passes, void* workspace,
+                                        size_t workspace_bytes, uint64_t* stats, uint32_t* status, void* stream) {
     pdr_status st = check_pad_args(width, height, channels, valid_threshold);
     if (st) return st;
     if (!color || !valid_mask || !filled_mask || !workspace || !stats || !status)
@@ -1058,7 +1087,7 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
     pad_classify_kernel<<<stat_blocks(words * 32), kStatThreads, 0, s>>>(valid_mask, coverage_mask, filled_mask, bits,
                                                                          wpr, width, height, valid_threshold, st64);
     uint32_t* field2 = reinterpret_cast<uint32_t*>(ws + L.field2);
-    bool tiled = width <= (uint32_t)kTileMaxSide && height <= (uint32_t)kTileMaxSide;
+    bool tiled = max_passes > 0 && width <= (uint32_t)kTileMaxSide && height <= (uint32_t)kTileMaxSide;
     if (tiled) {
         TileSweeps T{};
         T.src_bits = bits;
@@ -1067,7 +1096,10 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
         T.changed = reinterpret_cast<uint8_t*>(boundary);
         T.control = control;
         T.status = status;
+        T.boundary = boundary;
+        T.boundary_words = 2 * bands * width;
         T.words_per_row = wpr;
+        T.max_passes = max_passes;
         T.W = (int32_t)width;
         T.H = (int32_t)height;
         T.tiles_x = (int32_t)((width + kPadTileW - 1) / kPadTileW);
@@ -1092,11 +1124,12 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
     if (!tiled) {
         e = cudaMemsetAsync(boundary, 0x80, 2ull * bands * width * sizeof(uint32_t), s);
         if (e) return set_cuda_error(e, "pdr_pad_texture_atlas");
-        pad_sweep_kernel<false><<<bands, 32, 0, s>>>(bits, wpr, nullptr, field, boundary, control, status,
-                                                     (int32_t)width, (int32_t)height);
-        pad_sweep_kernel<true><<<bands, 32, 0, s>>>(bits, wpr, field, field2, boundary + (size_t)bands * width,
-                                                    control, status, (int32_t)width, (int32_t)height);
     }
+    // behind the tiles they return at once unless those gave up
+    pad_sweep_kernel<false><<<bands, 32, 0, s>>>(bits, wpr, nullptr, field, boundary, control, status, (int32_t)width,
+                                                 (int32_t)height, tiled);
+    pad_sweep_kernel<true><<<bands, 32, 0, s>>>(bits, wpr, field, field2, boundary + (size_t)bands * width, control,
+                                                status, (int32_t)width, (int32_t)height, tiled);
     if (snapshot) {
         e = cudaMemcpyAsync(ws + L.snapshot, color, (size_t)width * height * channels * sizeof(float),
                             cudaMemcpyDeviceToDevice, s);
@@ -1109,7 +1142,8 @@ pdr_status pdr_pad_texture_atlas(float* color, uint32_t channels, const float* v
     P.filled = filled_mask;
     P.src_bits = bits;
     P.field = field2;
-    P.bands = tiled ? 0u : bands;
+    P.bands = bands;
+    P.tiled = tiled;
     P.channels = channels;
     P.color4 = channels == 4 && ((uintptr_t)color & 15u) == 0;
     P.words_per_row = wpr;
