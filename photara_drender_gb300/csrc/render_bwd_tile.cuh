@@ -43,7 +43,8 @@ __device__ __forceinline__ void load_v8_cs(const float4* addr, float4& a, float4
 // rasterize_backward.hlsl:78-90: whether pixel (px, py) lies in the triangle's clamped pixel bounds,
 // floor(lo) <= px < ceil(hi), which is lo < px + 1 and hi > px. The bounds are first formed with approximate
 // quotients: with `m` pixels to spare, far more than their error (2 ulp of each quotient scaled to pixels, and a
-// few roundings), they decide; otherwise, next to the bounds, the reference's divisions do.
+// few roundings; divisors from 2^126 on give 0 and are left out), they decide; otherwise, next to the bounds, the
+// reference's divisions do.
 __device__ __forceinline__ bool visited(float4 p0, float4 p1, float4 p2, float4 vp, uint32_t px, uint32_t py, uint32_t W,
                                         uint32_t H) {
     {
@@ -55,7 +56,8 @@ __device__ __forceinline__ bool visited(float4 p0, float4 p1, float4 p2, float4 
         const float mx = 0.05f + 2e-6f * (vp.z * (1.0f + fmaxf(fabsf(lx), fabsf(hx))) + fabsf(vp.x));
         const float my = 0.05f + 2e-6f * (vp.w * (1.0f + fmaxf(fabsf(ly), fabsf(hy))) + fabsf(vp.y));
         const float x = (float)px, y = (float)py;
-        if ((lx * 0.5f + 0.5f) * vp.z + vp.x < x + 1.0f - mx && (hx * 0.5f + 0.5f) * vp.z + vp.x > x + mx &&
+        if (fmaxf(p0.w, fmaxf(p1.w, p2.w)) < 8e37f &&
+            (lx * 0.5f + 0.5f) * vp.z + vp.x < x + 1.0f - mx && (hx * 0.5f + 0.5f) * vp.z + vp.x > x + mx &&
             (ly * 0.5f + 0.5f) * vp.w + vp.y < y + 1.0f - my && (hy * 0.5f + 0.5f) * vp.w + vp.y > y + my)
             return true;
     }
