@@ -114,6 +114,7 @@ class MeshBatch:
         return arr
 
     def set_config(self, config: Tuple[int, int, int]) -> None:
+        """The tile configuration of pdr_render_batch_forward; the passes here do not depend on it."""
         if tuple(config) not in CONFIGS:
             raise ValueError(f"batch configuration must be one of {CONFIGS}")
         self.config = BatchConfigC(*config)
@@ -150,27 +151,24 @@ class MeshBatch:
 
     def autotune(self, configs: Sequence[Tuple[int, int, int]] = CONFIGS, reps: int = 3,
                  backward: bool = True) -> Dict[Tuple[int, int, int], float]:
-        """Times forward (+ backward) of this batch for every configuration and keeps the fastest.
-        Returns {config: median milliseconds}."""
+        """Times forward (+ backward) of this batch. Neither depends on the tile configuration (that of
+        pdr_render_batch_forward), so they are timed once and every configuration gets that time; the first is
+        kept. Returns {config: median milliseconds}."""
         dev = self.r.context.device
-        times = {}
         for cfg in configs:
             self.set_config(cfg)
+        samples = []
+        for timed in range(reps + 1):  # the first untimed
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize(dev)
+            e0.record()
             self.forward()
             if backward:
                 self.backward()
-            samples = []
-            for _ in range(reps):
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                torch.cuda.synchronize(dev)
-                e0.record()
-                self.forward()
-                if backward:
-                    self.backward()
-                e1.record()
-                torch.cuda.synchronize(dev)
+            e1.record()
+            torch.cuda.synchronize(dev)
+            if timed:
                 samples.append(e0.elapsed_time(e1))
-            times[tuple(cfg)] = sorted(samples)[len(samples) // 2]
-        best = min(times, key=times.get)
-        self.set_config(best)
+        times = {tuple(cfg): sorted(samples)[len(samples) // 2] for cfg in configs}
+        self.set_config(min(times, key=times.get))
         return times
