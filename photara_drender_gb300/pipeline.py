@@ -211,18 +211,25 @@ class RenderFwdBwd:
         self.forward(clip, attrs, uv_attrs, texture, stream)
         self.backward(clip, attrs, uv_attrs, texture, grad_attr_out, grad_sampled, stream)
 
+    def _ordered(self, views: int) -> bool:
+        """Whether the shading of this many views together, or their adjoint, sorts its tiles by the texture's part they
+        sample (csrc/tile_order.cuh: order_pays), with three kernels more."""
+        texels = self.tw * self.th
+        return 16 * texels >= 128 << 20 and views > 1 and 2 * views * self.P >= texels
+
     def kernels_per_step(self) -> int:
-        """Kernels one step launches. Direct: two visibility kernels and the shading for each group of views that
-        shares the key buffer (512 MB), the adjoint and the pass that sums its per-view vertex records (the shading
-        and the adjoint each order their tiles by three more where the texture exceeds L2, not counted). Otherwise:
-        binning (count, three scan phases, fill; the unfused path also sorts each tile, two passes), the raster (the
-        main launch and the pass over tiles whose lists were cut), then fused: the shading is the raster's epilogue
-        and the backward as above; unfused: three forwards, texture backward, two interpolate backwards, raster
-        backward."""
+        """Kernels one step launches. Direct: two visibility kernels, the shading and, where it pays, the order of its
+        tiles for each group of views that shares the key buffer (512 MB). Otherwise: binning (count, three scan phases,
+        fill; the unfused path also sorts each tile, two passes) and the raster (the main launch and the pass over tiles
+        whose lists were cut). Then fused: the shading is the raster's epilogue, and the backward is the adjoint, the order
+        of its tiles where it pays, and the pass that sums its per-view vertex records; unfused: three forwards, texture
+        backward, two interpolate backwards, raster backward."""
+        backward = 2 + 3 * self._ordered(self.views)
         if self.direct:
-            per_group = max(1, min(self.views, (512 << 20) // (8 * self.P)))
-            return 3 * ((self.views + per_group - 1) // per_group) + 2
-        return 5 + 2 + 2 if self.fused else 5 + 2 + 2 + 3 + 1 + 2 + 1
+            per_group = max(1, min(self.views, 65535, (512 << 20) // (8 * self.P)))
+            groups = [min(per_group, self.views - k) for k in range(0, self.views, per_group)]
+            return sum(3 + 3 * self._ordered(n) for n in groups) + backward
+        return 5 + 2 + backward if self.fused else 5 + 2 + 2 + 3 + 1 + 2 + 1
 
     def capture(self, clip, attrs, uv_attrs, texture, grad_attr_out, grad_sampled) -> "torch.cuda.CUDAGraph":
         """Records one step into a CUDA graph (replay with .replay()); for small, launch-bound batches.
