@@ -866,20 +866,22 @@ def c5_leg(dev, hbm):
 # ---- GPU arm ------------------------------------------------------------------------------------------
 
 STAGES = ["visibility+shade", "render_backward"]
-# Source files each timed stage is compiled from, and its DRAM bytes (dram__bytes_read.sum +
+# Source files each timed stage is compiled from (its launches' files and what they include; render_backward's order of
+# tiles is launched from visibility.cu), and its DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum over its kernels) on this 64-view workload from an ncu capture of the
 # full-size run, recorded with the SHA-256 of those sources at capture time. A capture cannot run
 # inside the timed region; when the sources no longer hash to the recorded value the figure belongs to
 # other code and the line reports traffic as null.
 KERNEL_SOURCES = {
-    "visibility+shade": ["visibility.cu", "visibility.cuh", "raster_tile.cuh", "ndc_axis.cuh", "tile_order.cuh",
-                         "pdr_common.cuh"],
-    "render_backward": ["fused.cu", "render_bwd_tile.cuh", "vertex_sums.cuh", "tile_order.cuh", "pdr_common.cuh"],
+    "visibility+shade": ["visibility.cu", "visibility.cuh", "raster_tile.cuh", "bin_rect.cuh", "ndc_axis.cuh",
+                         "tile_order.cuh", "pdr_common.cuh", "pdr_internal.h"],
+    "render_backward": ["fused.cu", "visibility.cu", "render_bwd_tile.cuh", "ndc_axis.cuh", "tile_order.cuh",
+                        "pdr_common.cuh", "pdr_internal.h"],
 }
 # stage -> (sha256 of its sources, bytes)
 KERNEL_TRAFFIC = {
-    "visibility+shade": ("2b43e45df0e74c7b", 7327700000),
-    "render_backward": ("8200dc38ef29c163", 4745600000),
+    "visibility+shade": ("e8b231d59d198ff3", 7327000000),
+    "render_backward": ("72fb25e21c5dec5b", 4748200000),
 }
 
 
