@@ -518,7 +518,7 @@ cudaError_t launch_adam_tv(const float* tex_in, float* tex_out, float* grad, flo
     // rows per warp: eight where the atlas still fills the chip several times, fewer below
     uint32_t rows = 8;
     const uint64_t strips = (uint64_t)((tw + 255) / 256) * th;  // CTAs at one row each
-    while (rows > 1 && strips / rows < 152u * 16u) rows >>= 1;
+    while (rows > 1 && strips / rows < (uint32_t)num_sms() * 16u) rows >>= 1;
     if ((th + rows - 1) / rows > 65535u) rows = (th + 65534u) / 65535u;
     const dim3 grid((tw + 255) / 256, (th + rows - 1) / rows);
     return launch_step(adam_tv_kernel, grid, 256, stream, overlap, tex_in, tex_out, grad, m, v, tw, th, valid, chart, tv_eps, tv_scale,
@@ -542,7 +542,7 @@ cudaError_t launch_photometric(const float* tex, uint32_t tw, uint32_t th, const
     // pixels per thread: eight where the step still fills the chip, fewer below (4 views of 320 x 240: two 6.2 us, one
     // 7.5, four 6.9)
     uint32_t rounds = 8;
-    while (rounds > 1 && max_pixels * batch / (kPhotoThreads * rounds) < 152u * 3u) rounds >>= 1;
+    while (rounds > 1 && max_pixels * batch / (kPhotoThreads * rounds) < (uint32_t)num_sms() * 3u) rounds >>= 1;
     const uint64_t per = (uint64_t)kPhotoThreads * rounds;
     const dim3 grid((unsigned)((max_pixels + per - 1) / per), batch);
     return launch_step(photometric_kernel, grid, kPhotoThreads, stream, overlap, tex, tw, th, views, nviews, step, batch, eps, norm,
