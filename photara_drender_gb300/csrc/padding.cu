@@ -14,7 +14,7 @@
 //   reference's order with its strict comparison and clamp, so every texel takes the same value.
 // * atlases up to 4384 texels a side: 64 x 32 tiles, swept in parallel and repeated until every tile was
 //   swept with the values its neighbours end with (pad_tiles_kernel).
-// * larger atlases (pad_sweep_kernel): bands are warps ordered by a ticket; a band's first row reads the row
+// * larger atlases, and those whose tiles take too many passes (pad_sweep_kernel): bands are warps ordered by a ticket; a band's first row reads the row
 //   above from the previous band's boundary buffer. Entries start as a marker that no offset can equal
 //   (|offset| <= 16384), so a value is ready exactly when it differs from the marker: no fences. Every wait
 //   is bounded.
