@@ -14,12 +14,12 @@ pytestmark = pytest.mark.gpu
 
 # a small texture; one larger than L2 that the views sample densely enough to sort their tiles, and one that they do not;
 # two groups of views, of which the second has a view too few to sort
-@pytest.mark.parametrize("views,side,texture", [(3, 96, (64, 48, 4)), (4, 1024, (2048, 4096, 4)), (3, 96, (2048, 4096, 4)),
-                                                (17, 2048, (2048, 4096, 4))])
-@pytest.mark.parametrize("kind", ["direct", "tile lists", "unfused"])
-def test_count_matches_a_profile(views, side, texture, kind):
-    if views == 17 and kind != "direct":
-        pytest.skip("groups of views are the direct forward's")
+CASES = [(3, 96, (64, 48, 4)), (4, 1024, (2048, 4096, 4)), (3, 96, (2048, 4096, 4))]
+
+
+@pytest.mark.parametrize("views,side,texture,kind", [(*c, k) for c in CASES for k in ("direct", "tile lists", "unfused")]
+                         + [(17, 2048, (2048, 4096, 4), "direct")])
+def test_count_matches_a_recorded_step(views, side, texture, kind):
     pos3, idx = S.icosphere(2)
     mats, _ = S.orbit_cameras(views)
     dev = torch.device("cuda", 0)
