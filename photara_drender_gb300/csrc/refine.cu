@@ -30,23 +30,28 @@ constexpr int kPhotoThreads = 256;
 // on a 512 x 512 atlas 1787 -> 1515 us, 1000 on 64 x 64 10.9 -> 6.3 ms. Recorded into a graph the same edges gained nothing
 // (9.5 and 9.9 ms), so captures get ordinary launches.
 // A kernel has begun before its predecessors' writes are final, so what a kernel of the run writes (texture, gradient,
-// moments) is read after the wait alone: through pointers that the wait hands on, which no load can be moved ahead of, and
-// by coherent loads (texel_load). Views, masks, coordinates, targets, pairs and charts may be read any way: the run's first
-// kernel is launched ordinarily, so they were complete before any kernel of the run began. A caller's single step
-// (pdr_refine_photometric and the like) follows kernels that may have written them, and is launched ordinarily as well.
-template <class P>
-__device__ __forceinline__ void hand_on(P& pointer) {
-    asm volatile("" : "+l"(pointer)::"memory");
-}
-
-template <class... P>
-__device__ __forceinline__ void wait_predecessor(P&... written) {
+// moments) is read by coherent_load alone, after the wait: no load of it by a non-coherent path, and none that the compiler
+// may move ahead of the wait, as it may a plain load through a restrict pointer (volatile assembly keeps its order).
+// Everything written depends on such a load. Plain loads through pointers that the wait hands on were slower by 1 to 2% on
+// 60 steps of a 512 x 512 atlas (1549 us, so 1521, in turn). Views, masks, coordinates, targets, pairs and charts may be read any way: the
+// run's first kernel is launched ordinarily, so they were complete before any kernel of the run began. A caller's single
+// step (pdr_refine_photometric and the like) follows kernels that may have written them, and is launched ordinarily as well.
+__device__ __forceinline__ void wait_predecessor() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    (hand_on(written), ...);
 }
 
-__device__ __forceinline__ float texel_load(const float* p) { return __ldca(p); }
+__device__ __forceinline__ float coherent_load(const float* p) {
+    float v;
+    asm volatile("ld.global.ca.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ float4 coherent_load(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 
 // overlap: the stream's last work is a kernel of this run.
 template <class... Params, class... Args>
@@ -189,7 +194,7 @@ __global__ void __launch_bounds__(kPhotoThreads, 5)
 photometric_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, const pdr_refine_view* __restrict__ views,
                    uint32_t nviews, uint32_t step, uint32_t batch, float eps, float norm, uint32_t rounds,
                    float* __restrict__ grad, float* __restrict__ loss) {
-    wait_predecessor(tex, grad, loss);
+    wait_predecessor();
     const pdr_refine_view v = views[((size_t)step * batch + blockIdx.y) % nviews];
     const float2* const uvs = reinterpret_cast<const float2*>(v.uv);
     float local = 0.0f;
@@ -213,7 +218,7 @@ photometric_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, cons
             for (uint32_t c = 0; c < 3; ++c) {
                 float rendered = 0.0f;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) rendered += texel_load(tex + (size_t)t.o[k] * 3 + c) * t.w[k];
+                for (int k = 0; k < 4; ++k) rendered += coherent_load(tex + (size_t)t.o[k] * 3 + c) * t.w[k];
                 const float d = rendered - v.target[p * 3 + c];
                 const float robust = sqrtf(d * d + eps * eps);
                 og[c] = d / robust * m * norm;
@@ -231,7 +236,7 @@ photometric_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, cons
 __global__ void seam_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t th, const float4* __restrict__ pairs,
                             uint32_t npairs, float eps, float norm, float* __restrict__ grad, float* __restrict__ loss,
                             uint32_t loss_index) {
-    wait_predecessor(tex, grad, loss);
+    wait_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float local = 0.0f;
     if (i < npairs) {
@@ -244,8 +249,8 @@ __global__ void seam_kernel(const float* __restrict__ tex, uint32_t tw, uint32_t
             float c0 = 0.0f, c1 = 0.0f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                c0 += texel_load(tex + (size_t)a.o[k] * 3 + c) * a.w[k];
-                c1 += texel_load(tex + (size_t)b.o[k] * 3 + c) * b.w[k];
+                c0 += coherent_load(tex + (size_t)a.o[k] * 3 + c) * a.w[k];
+                c1 += coherent_load(tex + (size_t)b.o[k] * 3 + c) * b.w[k];
             }
             const float d = c0 - c1;
             const float robust = sqrtf(d * d + eps * eps);
@@ -370,21 +375,21 @@ __device__ __forceinline__ void clear_gradient(float4* g, const float4& was) {
 
 __global__ void adam_kernel(float* __restrict__ tex, float* __restrict__ grad, float* __restrict__ m1,
                             float* __restrict__ m2, size_t texels, AdamStep s) {
-    wait_predecessor(tex, grad, m1, m2);
+    wait_predecessor();
     // one texel per thread: texture and moments [texels][3], gradient [texels][4] read and cleared as one
     // float4 (four texels per thread, or four values with the gradient gathered, were slower). 16.8 M texels of which
     // few have moments, a seam polish step: 330 us writing every value and dividing nine times; with the quotients and
     // without rewriting zero gradients 291, without rewriting unchanged texels 199, without their arithmetic 132.
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < texels; t += stride) {
-        const float4 d = __ldca(reinterpret_cast<const float4*>(grad) + t);
+        const float4 d = coherent_load(reinterpret_cast<const float4*>(grad) + t);
         const float g[3] = {d.x, d.y, d.z};
         float x[3], m[3], v[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            x[c] = tex[t * 3 + c];
-            m[c] = m1[t * 3 + c];
-            v[c] = m2[t * 3 + c];
+            x[c] = coherent_load(tex + t * 3 + c);
+            m[c] = coherent_load(m1 + t * 3 + c);
+            v[c] = coherent_load(m2 + t * 3 + c);
         }
         const float was[9] = {x[0], x[1], x[2], m[0], m[1], m[2], v[0], v[1], v[2]};
         adam_texel(x, g, m, v, s);
@@ -418,7 +423,7 @@ __device__ __forceinline__ TvTexel load_tv(const float* __restrict__ tex, const 
     TvTexel o = {{0.0f, 0.0f, 0.0f}, 0, false};
     if (inside) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) o.c[c] = texel_load(tex + t * 3 + c);
+        for (int c = 0; c < 3; ++c) o.c[c] = coherent_load(tex + t * 3 + c);
         o.valid = __ldg(valid + t) != 0;
         if (chart) o.chart = __ldg(chart + t);
     }
@@ -449,7 +454,7 @@ adam_tv_kernel(const float* __restrict__ tex_in, float* __restrict__ tex_out, fl
                float* __restrict__ m1, float* __restrict__ m2, uint32_t tw, uint32_t th,
                const uint8_t* __restrict__ valid, const int32_t* __restrict__ chart, float tv_eps, float tv_scale,
                uint32_t rows, AdamStep s) {
-    wait_predecessor(tex_in, tex_out, grad, m1, m2);
+    wait_predecessor();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t x = blockIdx.x * 256u + threadIdx.x;
     const uint32_t y0 = blockIdx.y * rows, y1 = min(y0 + rows, th);
@@ -468,11 +473,11 @@ adam_tv_kernel(const float* __restrict__ tex_in, float* __restrict__ tex_out, fl
         float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float m[3] = {0.0f, 0.0f, 0.0f}, v[3] = {0.0f, 0.0f, 0.0f};
         if (in) {
-            d = reinterpret_cast<const float4*>(grad)[t];
+            d = coherent_load(reinterpret_cast<const float4*>(grad) + t);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                m[c] = m1[t * 3 + c];
-                v[c] = m2[t * 3 + c];
+                m[c] = coherent_load(m1 + t * 3 + c);
+                v[c] = coherent_load(m2 + t * 3 + c);
             }
         }
         TvTexel next;
