@@ -33,9 +33,10 @@ constexpr int kPhotoThreads = 256;
 // moments) is read by coherent_load alone, after the wait: no load of it by a non-coherent path, and none that the compiler
 // may move ahead of the wait, as it may a plain load through a restrict pointer (volatile assembly keeps its order).
 // Everything written depends on such a load. Plain loads through pointers that the wait hands on were slower by 1 to 2% on
-// 60 steps of a 512 x 512 atlas (1549 us, so 1521, in turn). Views, masks, coordinates, targets, pairs and charts may be read any way: the
-// run's first kernel is launched ordinarily, so they were complete before any kernel of the run began. A caller's single
-// step (pdr_refine_photometric and the like) follows kernels that may have written them, and is launched ordinarily as well.
+// 60 steps of a 512 x 512 atlas (1549 us, so 1521, in turn).
+// Views, masks, coordinates, targets, pairs and charts may be read any way: the run's first kernel is launched
+// ordinarily, so they were complete before any kernel of the run began. A caller's single step (pdr_refine_photometric and
+// the like) follows kernels that may have written them, and is launched ordinarily as well.
 __device__ __forceinline__ void wait_predecessor() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
